@@ -5,6 +5,7 @@
 // primitive each kept pixel shows.  The work is split by what it depends on,
 // so each part runs once per pixel, per face or per vertex:
 //
+//   begin_kernel         flags cleared, block maps, per-job light units
 //   mark_kernel          pixels -> faces they show (visibility flags)
 //   face_prep_kernel     per visible face: clip positions, 3x3 inverse m of
 //                        [x, y, w] (same operations as the forward set-up);
@@ -281,7 +282,7 @@ __device__ __forceinline__ void reduce_params(const ParamGrad& pg, float* job_pa
 }
 
 // The scene's light directions normalised (the same operations as the
-// fragment shaders'), with their norms: once per job by light_kernel, read by
+// fragment shaders'), with their norms: once per job by begin_kernel, read by
 // every pixel block of the job.
 struct LightUnit {
   float dir[3], dir_n;  // light_direction (phong, phong_darboux)
@@ -318,9 +319,8 @@ struct Work {
                         // phong_darboux NDC triangle (9) when that shader is in the batch
   int vstride;
   int vacc_stride;      // 3, or 12 with phong_darboux
-  const int2* fmap;     // face block map (kRows faces per block)
-  const int2* vmap;     // vertex block map
-  unsigned* starts;     // per-job block starts of both maps (2 x (n_jobs + 1))
+  int2* fmap;           // face block map (kRows faces per block)
+  int2* vmap;           // vertex block map
   LightUnit* light;     // per job: normalised light directions
 };
 
@@ -366,18 +366,26 @@ __global__ void __launch_bounds__(kThreads) mark_kernel(RastBatch B, Work w) {
   }
 }
 
-// One thread per job: its LightUnit, so that the pixel kernel's blocks load
-// it with the job instead of computing it on one thread between two barriers.
-__global__ void __launch_bounds__(kThreads) light_kernel(RastBatch B, Work w) {
-  const int j = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x);
-  if (j >= B.n_jobs) return;
-  const RastJob& J = B.jobs[j];
-  LightUnit u;
-  u.dir_n = norm3(J.light_direction);
-  normalise3(J.light_direction, u.dir);
-  u.eye_n = norm3(J.light_dir_eye);
-  normalise3(J.light_dir_eye, u.eye);
-  w.light[j] = u;
+// First launch of the backward: visibility flags cleared, both block maps,
+// and each job's LightUnit (one thread per job), so that the pixel kernel's
+// blocks load it with the job instead of computing it on one thread between
+// two barriers.  One launch where two memsets, four block-map kernels and a
+// light kernel ran one after the other.
+__global__ void __launch_bounds__(kThreads) begin_kernel(RastBatch B, Work w, unsigned fblocks, unsigned vblocks) {
+  fill_words(w.fvis, static_cast<size_t>(B.total_setup), 0u);
+  fill_words(w.vvis, static_cast<size_t>(B.total_vout), 0u);
+  fill_block_map<kMapFaces>(B.jobs, B.n_jobs, kRows, w.fmap, fblocks);
+  fill_block_map<kMapVertices>(B.jobs, B.n_jobs, kRows, w.vmap, vblocks);
+  for (int j = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); j < B.n_jobs;
+       j += static_cast<int>(gridDim.x * blockDim.x)) {
+    const RastJob& J = B.jobs[j];
+    LightUnit u;
+    u.dir_n = norm3(J.light_direction);
+    normalise3(J.light_direction, u.dir);
+    u.eye_n = norm3(J.light_dir_eye);
+    normalise3(J.light_dir_eye, u.eye);
+    w.light[j] = u;
+  }
 }
 
 // Per visible face: clip rows of its corners, their 3x3 inverse (the forward
@@ -1228,7 +1236,7 @@ __global__ void __launch_bounds__(kThreads, 4) post_kernel(RastBatch B, Work w, 
 // ------------------------------------------------------------------ layout
 
 struct Layout {
-  size_t fvis_off, frec_off, facc_off, vvis_off, vvar_off, vacc_off, fmap_off, vmap_off, start_off, light_off, total;
+  size_t fvis_off, frec_off, facc_off, vvis_off, vvar_off, vacc_off, fmap_off, vmap_off, light_off, total;
   int vacc_stride;
   int vstride;
   unsigned fblocks, vblocks;
@@ -1258,7 +1266,6 @@ static Layout layout(const RastBatch& b) {
   L.vblocks = block_map_capacity(b.total_vout, b.n_jobs, kRows);
   L.fmap_off = take(static_cast<size_t>(L.fblocks) * sizeof(int2));
   L.vmap_off = take(static_cast<size_t>(L.vblocks) * sizeof(int2));
-  L.start_off = take(2 * block_start_bytes(b.n_jobs));
   L.light_off = take(static_cast<size_t>(b.n_jobs) * sizeof(LightUnit));
   L.total = off;
   return L;
@@ -1270,12 +1277,11 @@ static void launch_all(const RastBatch& b, const Work& w, const Layout& L, const
   const int64_t max_px = static_cast<int64_t>(b.max_width) * b.max_height;
   const dim3 pgrid(static_cast<unsigned>((max_px + kThreads - 1) / kThreads), static_cast<unsigned>(b.n_jobs));
   const unsigned fgrid = L.fblocks, vgrid = L.vblocks;
-  build_block_map(b, kMapFaces, kRows, const_cast<int2*>(w.fmap), w.starts, s);
-  build_block_map(b, kMapVertices, kRows, const_cast<int2*>(w.vmap), w.starts + b.n_jobs + 1, s);
+  begin_kernel<<<begin_blocks(static_cast<size_t>(b.total_setup) + static_cast<size_t>(b.total_vout), b.n_jobs, sm_count()),
+                 kThreads, 0, s>>>(b, w, fgrid, vgrid);
   const int64_t mark_px = static_cast<int64_t>(kThreads) * kMarkPixels;
   mark_kernel<<<dim3(static_cast<unsigned>((max_px + mark_px - 1) / mark_px), static_cast<unsigned>(b.n_jobs)),
                 kThreads, 0, s>>>(b, w);
-  light_kernel<<<static_cast<unsigned>((b.n_jobs + kThreads - 1) / kThreads), kThreads, 0, s>>>(b, w);
   prof.mark("backward_mark_kernels");
   face_prep_kernel<<<fgrid, kThreads, 0, s>>>(b, w);
   prof.mark("backward_face_prep_kernel");
@@ -1311,11 +1317,9 @@ static int run(const RastBatch* batch, const CanvasGrad& grad_canvas, const floa
          reinterpret_cast<float*>(ws + L.facc_off), reinterpret_cast<unsigned char*>(ws + L.vvis_off),
          reinterpret_cast<float*>(ws + L.vvar_off), reinterpret_cast<float*>(ws + L.vacc_off), L.vstride,
          L.vacc_stride,
-         reinterpret_cast<const int2*>(ws + L.fmap_off), reinterpret_cast<const int2*>(ws + L.vmap_off),
-         reinterpret_cast<unsigned*>(ws + L.start_off), reinterpret_cast<LightUnit*>(ws + L.light_off)};
+         reinterpret_cast<int2*>(ws + L.fmap_off), reinterpret_cast<int2*>(ws + L.vmap_off),
+         reinterpret_cast<LightUnit*>(ws + L.light_off)};
   Profiler prof(profile, s, "rast_backward");
-  if (cudaMemsetAsync(w.fvis, 0, static_cast<size_t>(b.total_setup), s) != cudaSuccess) return RAST_ERR_CUDA;
-  if (cudaMemsetAsync(w.vvis, 0, static_cast<size_t>(b.total_vout), s) != cudaSuccess) return RAST_ERR_CUDA;
   const int mask = b.shader_mask;
   auto only = [&](int sh) { return mask == (1 << sh); };
   if (only(RAST_SHADER_DEPTH)) launch_all<RAST_SHADER_DEPTH>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);

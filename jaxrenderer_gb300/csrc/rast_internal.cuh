@@ -132,9 +132,13 @@ __device__ __forceinline__ int block_queue_rows(Flag flag, int* s_q, int* s_n) {
 }
 
 // ---- block maps: grids over the faces (or vertices) of every job with no
-// empty blocks.  Entry b of the map is (job, first item of the block) for
-// the b-th block of the concatenated per-job block ranges, (-1, 0) past the
-// end.  A batch needs at most floor(total / per_block) + n_jobs blocks.
+// more than one empty block per job.  Job j's blocks of `per_block` items
+// start at entry begin_j / per_block + j, begin_j its first row (setup_begin
+// or vout_begin, the running sum of n_faces / n_verts): the entries up to the
+// next job's first one hold every block of the job, since floor((a + n) / p) -
+// floor(a / p) + 1 >= ceil(n / p), and no prefix sum over the jobs is needed.
+// Entry b is (job, first item of the block), or (-1, 0) for an empty block.
+// A batch needs floor(total / per_block) + n_jobs entries.
 constexpr int kMapFaces = 0, kMapVertices = 1;
 
 __host__ __device__ inline unsigned block_map_capacity(int64_t total, int n_jobs, int per_block) {
@@ -142,74 +146,62 @@ __host__ __device__ inline unsigned block_map_capacity(int64_t total, int n_jobs
 }
 
 template <int kField>
-__device__ __forceinline__ unsigned blocks_of_job(const RastJob* jobs, int j, int per_block) {
-  const int n = kField == kMapFaces ? __ldg(&jobs[j].n_faces) : __ldg(&jobs[j].n_verts);
-  return n > 0 ? static_cast<unsigned>((n + per_block - 1) / per_block) : 0u;
+__device__ __forceinline__ unsigned map_entry_of_job(const RastJob* jobs, int n_jobs, int j, int per_block,
+                                                     unsigned capacity) {
+  if (j >= n_jobs) return capacity;
+  const int64_t begin = kField == kMapFaces ? __ldg(&jobs[j].setup_begin) : __ldg(&jobs[j].vout_begin);
+  return min(static_cast<unsigned>(begin / per_block) + static_cast<unsigned>(j), capacity);
 }
 
-// Exclusive prefix of per-job block counts -> start[0..n_jobs] (start[n_jobs]
-// = total).  One block of 1024 threads; thread t owns a contiguous run of jobs.
+// Fills the map; every block of the grid calls it.  Few jobs take a block
+// each (one job of 389,120 faces has 3,040 entries, 9.7 us when one thread
+// wrote them), many jobs a warp each.
+constexpr int kMapBlockJobs = 2048;  // up to this many jobs: a block per job
 template <int kField>
-__global__ void __launch_bounds__(1024)
-block_prefix_kernel(const RastJob* __restrict__ jobs, int n_jobs, int per_block, unsigned* __restrict__ start) {
-  __shared__ unsigned s_sum[1024];
-  const int t = threadIdx.x;
-  const int per_thread = (n_jobs + 1023) / 1024;
-  const int j0 = min(n_jobs, t * per_thread), j1 = min(n_jobs, j0 + per_thread);
-  unsigned mine = 0;
-  for (int j = j0; j < j1; ++j) mine += blocks_of_job<kField>(jobs, j, per_block);
-  s_sum[t] = mine;
-  __syncthreads();
-  for (int off = 1; off < 1024; off <<= 1) {
-    const unsigned add = t >= off ? s_sum[t - off] : 0u;
-    __syncthreads();
-    s_sum[t] += add;
-    __syncthreads();
+__device__ __forceinline__ void fill_block_map(const RastJob* __restrict__ jobs, int n_jobs, int per_block,
+                                               int2* __restrict__ map, unsigned capacity) {
+  const bool wide = n_jobs <= kMapBlockJobs;
+  const unsigned team = wide ? blockDim.x : 32u;
+  const unsigned t = threadIdx.x % team, teams = blockDim.x / team;
+  for (int j = static_cast<int>(blockIdx.x * teams + threadIdx.x / team); j < n_jobs;
+       j += static_cast<int>(gridDim.x * teams)) {
+    const int n = kField == kMapFaces ? __ldg(&jobs[j].n_faces) : __ldg(&jobs[j].n_verts);
+    const unsigned a = map_entry_of_job<kField>(jobs, n_jobs, j, per_block, capacity);
+    const unsigned b = map_entry_of_job<kField>(jobs, n_jobs, j + 1, per_block, capacity);
+    for (unsigned e = a + t; e < b; e += team) {
+      const int64_t first = static_cast<int64_t>(e - a) * per_block;
+      map[e] = first < n ? make_int2(j, static_cast<int>(first)) : make_int2(-1, 0);
+    }
   }
-  unsigned at = s_sum[t] - mine;
-  for (int j = j0; j < j1; ++j) {
-    start[j] = at;
-    at += blocks_of_job<kField>(jobs, j, per_block);
-  }
-  if (t == 1023) start[n_jobs] = s_sum[1023];
 }
 
-// One thread per job writes its blocks' entries; the threads past the jobs
-// fill the tail of the map (entries >= total) with (-1, 0).
-template <int kField>
-__global__ void __launch_bounds__(256)
-block_fill_kernel(const RastJob* __restrict__ jobs, int n_jobs, int per_block, const unsigned* __restrict__ start,
-                  int2* __restrict__ map, unsigned capacity) {
-  const int j = blockIdx.x * 256 + threadIdx.x;
-  if (j < n_jobs) {
-    const unsigned a = start[j], nb = start[j + 1] - a;
-    for (unsigned b = 0; b < nb && a + b < capacity; ++b) map[a + b] = make_int2(j, static_cast<int>(b) * per_block);
-  }
-  const unsigned total = start[n_jobs];
-  const unsigned stride = gridDim.x * 256u;
-  for (unsigned k = total + static_cast<unsigned>(j); k < capacity; k += stride) map[k] = make_int2(-1, 0);
+// Sets `bytes` bytes at p (16-byte aligned; the last 16-byte word may run
+// past `bytes`, inside the workspace's 256-byte granules), the whole grid
+// striding over them.
+__device__ __forceinline__ void fill_words(void* p, size_t bytes, unsigned value) {
+  uint4* w = static_cast<uint4*>(p);
+  const size_t n = (bytes + 15) / 16;
+  for (size_t k = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n;
+       k += static_cast<size_t>(gridDim.x) * blockDim.x)
+    w[k] = make_uint4(value, value, value, value);
 }
 
-// Builds the map of `field` for batch b on stream s.  `start` holds
-// n_jobs + 1 unsigned.
-inline cudaError_t build_block_map(const RastBatch& b, int field, int per_block, int2* map, unsigned* start,
-                                   cudaStream_t s) {
-  const int64_t total = field == kMapFaces ? b.total_setup : b.total_vout;
-  const unsigned cap = block_map_capacity(total, b.n_jobs, per_block);
-  if (cap == 0 || b.n_jobs <= 0) return cudaSuccess;
-  const unsigned grid = static_cast<unsigned>((b.n_jobs + 255) / 256);
-  if (field == kMapFaces) {
-    block_prefix_kernel<kMapFaces><<<1, 1024, 0, s>>>(b.jobs, b.n_jobs, per_block, start);
-    block_fill_kernel<kMapFaces><<<grid, 256, 0, s>>>(b.jobs, b.n_jobs, per_block, start, map, cap);
-  } else {
-    block_prefix_kernel<kMapVertices><<<1, 1024, 0, s>>>(b.jobs, b.n_jobs, per_block, start);
-    block_fill_kernel<kMapVertices><<<grid, 256, 0, s>>>(b.jobs, b.n_jobs, per_block, start, map, cap);
-  }
-  return cudaGetLastError();
+// Blocks of 256 threads for a launch that fills `bytes` bytes and block maps
+// of n_jobs jobs: at most eight per SM.
+inline unsigned begin_blocks(size_t bytes, int n_jobs, int sms) {
+  const size_t maps = n_jobs <= kMapBlockJobs ? n_jobs : (n_jobs + 7) / 8;
+  const size_t fill = bytes / (256 * 16 * 2) + 1;
+  const size_t most = static_cast<size_t>(sms > 0 ? sms : 1) * 8;
+  const size_t want = maps > fill ? maps : fill;
+  return static_cast<unsigned>(want < most ? want : most);
 }
 
-// Bytes of the per-job block starts that build_block_map needs.
-inline size_t block_start_bytes(int n_jobs) { return (static_cast<size_t>(n_jobs) + 1) * sizeof(unsigned); }
+inline int sm_count() {
+  int sms = 0, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms > 0 ? sms : 1;
+}
 
 // Pixel (i, j) of a job from its x-major local index i * H + j; 32-bit
 // division when the job's pixel count fits (every job in practice).

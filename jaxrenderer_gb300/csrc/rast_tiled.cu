@@ -4,12 +4,12 @@
 // tested with the same operations; binning only removes pairs that cannot
 // pass.
 //
-//   job_tiles_kernel   per-job tile grid (fixed stride: tiles of the largest job)
 //   setup_bin_kernel   one thread per face: clip positions, det/keep/inverse;
 //                      then one thread per candidate (queued in shared memory):
 //                      conservative tile range of its coverage region, bin counts
-//   scan_local_kernel  \  exclusive prefix sum of bin counts -> bin offsets;
-//   scan_apply_kernel  /  tiles whose bins exceed the capacity are marked
+//   begin_kernel       block map of the faces, counters and flags cleared
+//   offsets_kernel     bin counts -> bin offsets; tiles whose bins exceed the
+//                      capacity are marked
 //   scatter_kernel     over the binned faces the set-up listed, one warp per 32:
 //                      face id into every bin its rectangle overlaps
 //   raster_kernel      persistent warps, one tile each: bin entries staged in
@@ -37,6 +37,9 @@ constexpr int kScanBlock = 1024;       // elements per scan block (256 threads x
 constexpr int kRasterWarps = 4;        // warps per CTA of the raster kernel
 constexpr int kStage = 32;             // bin entries staged per warp round
 constexpr uint32_t kOverflow = 0x80000000u;
+constexpr int kFaceThreads = 256;      // threads and faces per block of the face varyings
+constexpr int kVaryRowsPerThread = 16;
+constexpr int kVaryRows = kFaceThreads * kVaryRowsPerThread;
 
 // Tile shapes offered to the autotuner.  (tw, th): tw pixels along x
 // (axis 0 of the buffers), th along y (contiguous in memory).
@@ -547,11 +550,44 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
   }
 }
 
-// Block-local exclusive scan of counts -> offsets, block sums out.
+// First launch of a pass: the face block map, and everything that starts
+// from zero (tile counts and cursors, the counters, the visible-face flags)
+// or from the empty key (the small path's per-pixel keys).  One launch where
+// two block-map kernels and up to four memsets ran one after the other, each
+// 1-3 us of latency on the path of a small batch and 10-16 us for one
+// thread per job writing a large job's map entries.
+struct BeginWork {
+  int2* fmap;
+  unsigned fmap_blocks;
+  int map_rows;  // faces per block of the map
+  int2* vmap;    // the face varyings' map (kVaryRows faces per block)
+  unsigned vmap_blocks;
+  void* zero[3];
+  size_t zero_bytes[3];
+  void* keys;  // small path: every key starts as kEmptyKey
+  size_t key_bytes;
+};
+
+__global__ void __launch_bounds__(256) begin_kernel(RastBatch B, BeginWork w) {
+#pragma unroll
+  for (int k = 0; k < 3; ++k) fill_words(w.zero[k], w.zero_bytes[k], 0u);
+  fill_words(w.keys, w.key_bytes, 0xffffffffu);
+  fill_block_map<kMapFaces>(B.jobs, B.n_jobs, w.map_rows, w.fmap, w.fmap_blocks);
+  fill_block_map<kMapFaces>(B.jobs, B.n_jobs, kVaryRows, w.vmap, w.vmap_blocks);
+}
+
+// Bin offsets: a tile only needs a contiguous range of the bins, in no
+// particular order among tiles, so each block of kScanBlock tiles scans its
+// counts and takes its range with one addition to the entry cursor (one
+// launch; a prefix sum over all tiles took two).  Tiles whose bin does not
+// fit into `capacity` entries are marked (they are rasterised by a full scan
+// instead).  The cursor ends as the total of entries requested.
 __global__ void __launch_bounds__(256)
-scan_local_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets,
-                  uint32_t* __restrict__ block_sums, int64_t n) {
-  __shared__ uint32_t s[256];
+offsets_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets, int64_t n, uint64_t capacity,
+               unsigned int* __restrict__ status, unsigned long long* __restrict__ cursor) {
+  __shared__ uint32_t s_warp[8];
+  __shared__ unsigned long long s_base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanBlock + threadIdx.x * 4;
   uint32_t v[4], t = 0;
 #pragma unroll
@@ -559,64 +595,34 @@ scan_local_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ of
     v[k] = (base + k < n) ? counts[base + k] : 0u;
     t += v[k];
   }
-  s[threadIdx.x] = t;
-  __syncthreads();
-  for (int off = 1; off < 256; off <<= 1) {
-    const uint32_t add = threadIdx.x >= off ? s[threadIdx.x - off] : 0u;
-    __syncthreads();
-    s[threadIdx.x] += add;
-    __syncthreads();
-  }
-  uint32_t run = s[threadIdx.x] - t;  // exclusive prefix of this thread
+  uint32_t incl = t;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    if (base + k < n) offsets[base + k] = run;
-    run += v[k];
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += o;
   }
-  if (threadIdx.x == 255) block_sums[blockIdx.x] = s[255];
-}
-
-// Adds the prefix of all previous blocks; marks tiles whose bin does not fit
-// into `capacity` entries (they are rasterised by a full scan instead).
-__global__ void __launch_bounds__(256)
-scan_apply_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ offsets,
-                  const uint32_t* __restrict__ block_sums, int64_t n, uint64_t capacity,
-                  unsigned int* __restrict__ status) {
-  __shared__ unsigned long long s_prefix;
-  __shared__ unsigned long long s_part[256];
-  unsigned long long part = 0;
-  for (int b = threadIdx.x; b < static_cast<int>(blockIdx.x); b += 256) part += block_sums[b];
-  s_part[threadIdx.x] = part;
+  if (lane == 31) s_warp[warp] = incl;
   __syncthreads();
-  for (int off = 128; off > 0; off >>= 1) {
-    if (threadIdx.x < off) s_part[threadIdx.x] += s_part[threadIdx.x + off];
-    __syncthreads();
+  uint32_t before = 0, total = 0;
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    if (k < warp) before += s_warp[k];
+    total += s_warp[k];
   }
-  if (threadIdx.x == 0) s_prefix = s_part[0];
+  if (threadIdx.x == 0) s_base = atomicAdd(cursor, static_cast<unsigned long long>(total));
   __syncthreads();
-  const unsigned long long prefix = s_prefix;
-  const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanBlock + threadIdx.x * 4;
-  const unsigned long long local_last = (n > 0 && base <= n - 1 && n - 1 < base + 4) ? offsets[n - 1] : 0ull;
+  unsigned long long o = s_base + before + (incl - t);
   bool over = false;
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
-    const int64_t i = base + k;
-    if (i >= n) break;
-    const unsigned long long o = prefix + offsets[i];
-    const uint32_t c = counts[i];
-    if (o + c > capacity || o >= kOverflow) {
-      offsets[i] = kOverflow;
-      over = over || c > 0;
-    } else {
-      offsets[i] = static_cast<uint32_t>(o);
+    if (base + k < n) {
+      const bool fits = o + v[k] <= capacity && o < kOverflow;
+      offsets[base + k] = fits ? static_cast<uint32_t>(o) : kOverflow;
+      over = over || (!fits && v[k] > 0);
     }
+    o += v[k];
   }
   if (over) atomicOr(status, 1u);
-  // total bin entries requested (before capacity), for rast_tiled_stats
-  if (n > 0 && base <= n - 1 && n - 1 < base + 4) {
-    const unsigned long long total = prefix + local_last + counts[n - 1];
-    *reinterpret_cast<unsigned long long*>(status + 1) = total;
-  }
 }
 
 // Face ids into the bins of the tiles their rectangles cover, over the list
@@ -1078,9 +1084,6 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
 // in shared memory, then one thread per (visible face, corner) runs the
 // vertex shader, so faces nobody sees leave no idle lanes and the block's
 // job load and queue are paid once per kVaryRows faces.
-constexpr int kFaceThreads = 256;
-constexpr int kVaryRowsPerThread = 16;
-constexpr int kVaryRows = kFaceThreads * kVaryRowsPerThread;
 
 __global__ void __launch_bounds__(kFaceThreads)
 face_varyings_kernel(RastBatch B, const int2* __restrict__ vmap, const unsigned char* __restrict__ visible,
@@ -1185,8 +1188,8 @@ inline uint64_t default_bin_capacity(const RastBatch& b) {
 }
 
 struct Layout {
-  size_t setup_off, bbox_off, binned_off, counts_off, offsets_off, cursors_off, bsums_off, bins_off, winner_off,
-      vis_off, fvar_off, fmap_off, fstart_off, vmap_off, vstart_off, keys_off, misc_off, total;
+  size_t setup_off, bbox_off, binned_off, counts_off, offsets_off, cursors_off, bins_off, winner_off, vis_off, fvar_off,
+      fmap_off, vmap_off, keys_off, misc_off, total;
   unsigned fmap_blocks, vmap_blocks;  // face block maps: setup/scatter, face varyings
   bool small_path;  // setup kernel rasterises small faces (not when near ties are counted)
   int vstride;
@@ -1222,7 +1225,6 @@ static Layout layout(const RastBatch& b, TileShape ts, uint64_t bin_capacity, in
   L.counts_off = take(static_cast<size_t>(L.n_tiles) * 4);
   L.cursors_off = take(static_cast<size_t>(L.n_tiles) * 4);
   L.offsets_off = take(static_cast<size_t>(L.n_tiles) * 4);
-  L.bsums_off = take(static_cast<size_t>(L.n_scan_blocks) * 4);
   L.bins_off = take(static_cast<size_t>(bin_capacity) * 4);
   L.winner_layers = b.max_layers > 0 ? RAST_MAX_LAYERS : 1;  // the raster variant writes every slot
   L.winner_off = take(static_cast<size_t>(b.total_pixels) * 4 * L.winner_layers);
@@ -1235,10 +1237,8 @@ static Layout layout(const RastBatch& b, TileShape ts, uint64_t bin_capacity, in
   L.fvar_off = take(shading ? static_cast<size_t>(b.total_setup) * 3 * vstride * sizeof(float) : 0);
   L.fmap_blocks = block_map_capacity(b.total_setup, b.n_jobs, kSetupThreads);
   L.fmap_off = take(static_cast<size_t>(L.fmap_blocks) * sizeof(int2));
-  L.fstart_off = take(block_start_bytes(b.n_jobs));
   L.vmap_blocks = shading ? block_map_capacity(b.total_setup, b.n_jobs, kVaryRows) : 0;
   L.vmap_off = take(static_cast<size_t>(L.vmap_blocks) * sizeof(int2));
-  L.vstart_off = take(shading ? block_start_bytes(b.n_jobs) : 0);
   L.small_path = b.near_ties == nullptr && small_area > 0 && b.max_layers == 0;
   L.keys_off = take(L.small_path ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0);
   L.misc_off = take(256);
@@ -1357,7 +1357,6 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
   uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.counts_off);
   uint32_t* cursors = reinterpret_cast<uint32_t*>(ws + L.cursors_off);
   uint32_t* offsets = reinterpret_cast<uint32_t*>(ws + L.offsets_off);
-  uint32_t* bsums = reinterpret_cast<uint32_t*>(ws + L.bsums_off);
   int32_t* bins = reinterpret_cast<int32_t*>(ws + L.bins_off);
   int32_t* winner = reinterpret_cast<int32_t*>(ws + L.winner_off);
   // [0] raster tile counter, [1] overflow status, [2..3] bin entries, [4..5] raster pixel tests,
@@ -1372,26 +1371,29 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
   // shaded jobs resolve in the deferred shade (from the per-face varyings when there are faces)
   const bool shading = b.total_pixels > 0 && (b.shader_mask != (1 << RAST_SHADER_DEPTH) || b.total_setup == 0);
   const bool pre = shading && fvar != nullptr && b.total_setup > 0;
+  const int sms = sm_count();
   if (cover) {
-    // counts and cursors are adjacent: one memset clears both, plus the counters
-    if (cudaMemsetAsync(counts, 0, L.offsets_off - L.counts_off, s) != cudaSuccess) return RAST_ERR_CUDA;
-    if (cudaMemsetAsync(misc, 0, 256, s) != cudaSuccess) return RAST_ERR_CUDA;
     unsigned long long* keys = nullptr;
-    if (L.small_path && b.total_pixels > 0 && b.total_setup > 0) {
+    if (L.small_path && b.total_pixels > 0 && b.total_setup > 0)
       keys = reinterpret_cast<unsigned long long*>(ws + L.keys_off);
-      if (cudaMemsetAsync(keys, 0xff, static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long), s) !=
-          cudaSuccess)  // every key starts as kEmptyKey
-        return RAST_ERR_CUDA;
-    }
-    if (vis && b.total_setup > 0 && cudaMemsetAsync(vis, 0, static_cast<size_t>(b.total_setup), s) != cudaSuccess)
-      return RAST_ERR_CUDA;
-    prof.mark("memset");
     int2* fmap = reinterpret_cast<int2*>(ws + L.fmap_off);
+    BeginWork bw{};
+    bw.fmap = fmap;
+    bw.fmap_blocks = b.total_setup > 0 ? L.fmap_blocks : 0u;
+    bw.map_rows = kSetupThreads;
+    bw.vmap = reinterpret_cast<int2*>(ws + L.vmap_off);
+    bw.vmap_blocks = pre ? L.vmap_blocks : 0u;
+    bw.zero[0] = counts;  // counts and cursors are adjacent
+    bw.zero_bytes[0] = L.offsets_off - L.counts_off;
+    bw.zero[1] = misc;
+    bw.zero_bytes[1] = 256;
+    bw.zero[2] = vis;
+    bw.zero_bytes[2] = vis ? static_cast<size_t>(b.total_setup) : 0;
+    bw.keys = keys;
+    bw.key_bytes = keys ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0;
+    begin_kernel<<<begin_blocks(bw.zero_bytes[0] + bw.zero_bytes[2] + bw.key_bytes, b.n_jobs, sms), 256, 0, s>>>(b, bw);
+    prof.mark("begin_kernel");
     if (b.total_setup > 0) {
-      if (build_block_map(b, kMapFaces, kSetupThreads, fmap, reinterpret_cast<unsigned*>(ws + L.fstart_off), s) !=
-          cudaSuccess)
-        return RAST_ERR_CUDA;
-      prof.mark("block_map_kernel");
       const unsigned grid = L.fmap_blocks;
       if (keys)
         setup_bin_kernel<true><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, bbox, counts, keys, small_area,
@@ -1400,24 +1402,15 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
         setup_bin_kernel<false><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, bbox, counts, nullptr, 0,
                                                               binned, misc + 6);
       prof.mark("setup_bin_kernel");
-      scan_local_kernel<<<static_cast<unsigned>(L.n_scan_blocks), 256, 0, s>>>(counts, offsets, bsums, L.n_tiles);
-      scan_apply_kernel<<<static_cast<unsigned>(L.n_scan_blocks), 256, 0, s>>>(counts, offsets, bsums, L.n_tiles,
-                                                                                L.bin_capacity, misc + 1);
-      prof.mark("scan_kernels");
-      {
-        int sms = 0, dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        // the list's length is on the device: a full wave of blocks strides over it
-        const unsigned sgrid = static_cast<unsigned>(std::max(sms, 1) * (2048 / kSetupThreads));
-        scatter_kernel<<<std::min(sgrid, grid), kSetupThreads, 0, s>>>(L.G, binned, misc + 6, offsets, cursors, bins);
-      }
+      offsets_kernel<<<static_cast<unsigned>(L.n_scan_blocks), 256, 0, s>>>(
+          counts, offsets, L.n_tiles, L.bin_capacity, misc + 1, reinterpret_cast<unsigned long long*>(misc + 2));
+      prof.mark("offsets_kernel");
+      // the list's length is on the device: a full wave of blocks strides over it
+      const unsigned sgrid = static_cast<unsigned>(sms * (2048 / kSetupThreads));
+      scatter_kernel<<<std::min(sgrid, grid), kSetupThreads, 0, s>>>(L.G, binned, misc + 6, offsets, cursors, bins);
       prof.mark("scatter_kernel");
     }
     if (b.total_pixels > 0) {
-      int sms = 0, dev = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
       if (b.total_setup > 0) {
         // the key path exists only when ties are not counted and no job is
         // layered
@@ -1442,11 +1435,7 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
       }
       prof.mark("raster_kernel");
       if (pre) {
-        int2* vmap = reinterpret_cast<int2*>(ws + L.vmap_off);
-        if (build_block_map(b, kMapFaces, kVaryRows, vmap, reinterpret_cast<unsigned*>(ws + L.vstart_off), s) !=
-            cudaSuccess)
-          return RAST_ERR_CUDA;
-        face_varyings_kernel<<<L.vmap_blocks, kFaceThreads, 0, s>>>(b, vmap, vis, fvar, L.vstride);
+        face_varyings_kernel<<<L.vmap_blocks, kFaceThreads, 0, s>>>(b, bw.vmap, vis, fvar, L.vstride);
         prof.mark("face_varyings_kernel");
       }
     }
