@@ -61,7 +61,9 @@ __device__ __forceinline__ int block_uniform_job(const RastJob* jobs, int n, int
 }
 
 // PerPrimitive.create (pipeline.py:80-113) from the three clip positions.
-// Record: [inv0..3] [inv4..7] [inv8 z0 z1 z2] [det flags 0 0].
+// Record: [inv0..3] [inv4..7] [inv8 z0 z1 z2] [det flags 0 0]; the tiled
+// form keeps the face's pixel rectangle in [3].x and [3].z and writes records
+// of binned faces and face 0 only.
 __device__ __forceinline__ void setup_from_clip(const float4* c, float* inv, float* det_out,
                                                 int* flags_out) {
   const float m[9] = {c[0].x, c[0].y, c[0].w, c[1].x, c[1].y, c[1].w, c[2].x, c[2].y, c[2].w};
@@ -252,12 +254,15 @@ struct Fragment {
   float colour[3];
 };
 
-// Without xy_given, (x, y) is computed here from the pixel (i, j).
+// Without xy_given, (x, y) is computed here from the pixel (i, j).  Chosen
+// primitives are candidates (kept and front-facing) except the default
+// chooser's fallback to primitive 0, whose flags come from its record.
 __device__ __forceinline__ void shade_primitive(const RastJob& J, const RastPools& P, const float4* rec_base,
                                                 int i, int j, float x, float y, int p, const VaryingSource& src,
-                                                Fragment* f, bool xy_given) {
+                                                Fragment* f, bool xy_given, bool fallback = false) {
   const float4* rec = rec_base + static_cast<int64_t>(p) * 4;
-  const float4 a = rec[0], b = rec[1], cz = rec[2], d = rec[3];
+  const float4 a = rec[0], b = rec[1], cz = rec[2];
+  const int flags = fallback ? __float_as_int(rec[3].y) : kCandidate;
   if (!xy_given) {
     x = (static_cast<float>(i) - J.viewport[3]) / J.viewport[0];
     y = (static_cast<float>(j) - J.viewport[7]) / J.viewport[5];
@@ -265,7 +270,6 @@ __device__ __forceinline__ void shade_primitive(const RastJob& J, const RastPool
   const float c[3] = {(x * a.x + y * a.w) + b.z, (x * a.y + y * b.x) + b.w,
                       (x * a.z + y * b.y) + cz.x};
   const bool in_tri = c[0] >= 0.0f && c[1] >= 0.0f && c[2] >= 0.0f;
-  const int flags = __float_as_int(d.y);
   f->chooser_keep = (flags & kKeep) && in_tri;
   const bool front = (flags & kFront) != 0;
   const float w_rcp = (c[0] + c[1]) + c[2];
@@ -323,7 +327,7 @@ __device__ __forceinline__ void resolve_pixel(const RastJob& J, const RastPools&
   if (J.n_faces <= 0) return;
   const int p = w < 0 ? 0 : w;
   Fragment f;
-  shade_primitive(J, P, rec_base, i, j, 0.0f, 0.0f, p, src, &f, false);
+  shade_primitive(J, P, rec_base, i, j, 0.0f, 0.0f, p, src, &f, false, w < 0);
   r->keep = f.chooser_keep && f.keep;
   r->z = f.z;
   r->prim = r->keep ? p : -1;

@@ -32,7 +32,7 @@
 namespace rast {
 namespace tiled {
 
-constexpr int kSetupThreads = 128;    // faces per setup/scatter block (256: 1 % slower, 64: 7 %)
+constexpr int kSetupThreads = 128;    // threads per setup/scatter block (256: 1 % slower, 64: 7 %)
 constexpr int kScanBlock = 1024;       // elements per scan block (256 threads x 4)
 constexpr int kRasterWarps = 4;        // warps per CTA of the raster kernel
 constexpr int kStage = 32;             // bin entries staged per warp round
@@ -141,10 +141,11 @@ __device__ __forceinline__ void clip_push0(ClipStage& s, ClipStage& s1, ClipStag
 // the corners' error and the rounding of the pixel <-> NDC maps.  Returns
 // false when no pixel can be covered.
 // The job's screen rectangle one pixel wider on every side, in NDC (pixels
-// -1 and W), computed once per block.
+// -1 and W), computed once per job by begin_kernel.
 struct ScreenRect {
   float xl, xh, yl, yh, X, Y;
-  bool ok;  // finite, non-degenerate viewport
+  float gx, gy;  // half a pixel in NDC (0: rounding could reach it, see off_screen)
+  int ok;  // finite, non-degenerate viewport
 };
 
 __device__ __forceinline__ ScreenRect screen_rect(const RastJob& J) {
@@ -160,29 +161,90 @@ __device__ __forceinline__ ScreenRect screen_rect(const RastJob& J) {
   r.yh = fmaxf(ya, yb);
   r.X = fmaxf(fabsf(r.xl), fabsf(r.xh));
   r.Y = fmaxf(fabsf(r.yl), fabsf(r.yh));
+  r.gx = 0.5f / fabsf(sx);
+  r.gy = 0.5f / fabsf(sy);
+  if (!(r.X * 4.8e-7f < r.gx)) r.gx = 0.0f;  // 8 u X
+  if (!(r.Y * 4.8e-7f < r.gy)) r.gy = 0.0f;
   return r;
+}
+
+// True when no pixel of the job can pass the edge tests against the inverse
+// inv3 computes for the clip rows m = [x, y, w] of a face (and determinant
+// det > 1e-6): the face lies on the far side of one line of the screen
+// rectangle (or of w = 0), and the rounding of the inverse provably cannot
+// bring it back.  Decided before the inverse and the coverage rectangle, which
+// cost four times what the rest of the set-up does: on the brax-like batch
+// the light's view holds a fifth of its front faces.
+//
+// With u = 2^-24, M_k the largest |entry| of column k, D_k its spread over the
+// three rows: each column X_j of the computed inverse solves (A + dA_j) X_j =
+// e_j with |dA_j| <= 12 u |L||U| (Higham, Accuracy and Stability of Numerical
+// Algorithms, Theorem 9.4, plus the reciprocal pivot's rounding) <= e M_k per
+// entry, e = 85 u (|L| <= 1, rows of |U| <= M, 2 M, 4 M).  The cofactors of A
+// are at most C_x = M_y D_w + M_w D_y (and so on), so the residual A X - I is
+// at most r = 1.18 q, q = e S / det, S = M_x C_x + M_y C_y + M_w C_w, when
+// q <= 1/20.  A pixel p = [x, y, 1] whose three computed edge values c are >=
+// 0 satisfies p = c' A with |c' - c| <= 1.22 r |c|_1 plus the evaluation's own
+// 3.6 u T / det, T = X C_x + Y C_y + C_w.  For a functional l that is
+// positive on every row (smallest l0, largest l1) and negative on every
+// pixel (at most -g), l(p) = c' l(A) >= |c|_1 (l0 - 4.4 q l1) - 13.4 u T l1 /
+// det: a contradiction when l0 >= 5 q l1 and 16 u T l1 < g det.  Products
+// that could overflow or underflow are excluded by M <= 2^30 (with det > 1e-6
+// the smallest M is then above 2^-83); NaN fails every comparison.
+__device__ __forceinline__ bool off_screen(const float* m, float det, const ScreenRect& R) {
+  const float x0 = m[0], x1 = m[3], x2 = m[6], y0 = m[1], y1 = m[4], y2 = m[7], w0 = m[2], w1 = m[5], w2 = m[8];
+  const float wmin = fminf(w0, fminf(w1, w2)), wmax = fmaxf(w0, fmaxf(w1, w2));
+  // l0 > 0: the face is beyond that side; the side's margin g
+  float l0 = -wmax, l1 = -wmin, g = 1.0f;
+  auto side = [&](float s, float a0, float a1, float a2, float c, float margin) {  // l = s (a - c w), one rounding each
+    const float p = __fmaf_rn(-c, w0, a0), q = __fmaf_rn(-c, w1, a1), r = __fmaf_rn(-c, w2, a2);
+    const float lo = s > 0.0f ? fminf(p, fminf(q, r)) : -fmaxf(p, fmaxf(q, r));
+    if (lo > l0) {
+      l0 = lo;
+      l1 = s > 0.0f ? fmaxf(p, fmaxf(q, r)) : -fminf(p, fminf(q, r));
+      g = margin;
+    }
+  };
+  side(1.0f, x0, x1, x2, R.xh, R.gx);
+  side(-1.0f, x0, x1, x2, R.xl, R.gx);
+  side(1.0f, y0, y1, y2, R.yh, R.gy);
+  side(-1.0f, y0, y1, y2, R.yl, R.gy);
+  if (!(l0 > 0.0f) || !R.ok) return false;
+  const float xmin = fminf(x0, fminf(x1, x2)), xmax = fmaxf(x0, fmaxf(x1, x2));
+  const float ymin = fminf(y0, fminf(y1, y2)), ymax = fmaxf(y0, fmaxf(y1, y2));
+  const float Mx = fmaxf(xmax, -xmin), My = fmaxf(ymax, -ymin), Mw = fmaxf(wmax, -wmin);
+  const float Dx = xmax - xmin, Dy = ymax - ymin, Dw = wmax - wmin;
+  const float Cx = __fmaf_rn(My, Dw, Mw * Dy), Cy = __fmaf_rn(Mx, Dw, Mw * Dx), Cw = __fmaf_rn(Mx, Dy, My * Dx);
+  const float S = __fmaf_rn(Mx, Cx, __fmaf_rn(My, Cy, Mw * Cw));
+  const float T = __fmaf_rn(R.X, Cx, __fmaf_rn(R.Y, Cy, Cw));
+  const float d = det - 48.0f * 5.9604645e-08f * (Mx * My * Mw);  // the determinant's own rounding: 42 u MxMyMw
+  const float eS = 85.0f * 5.9604645e-08f * S;
+  return fmaxf(Mx, fmaxf(My, Mw)) <= 1073741824.0f && 20.0f * eS <= d && 5.0f * eS * l1 <= l0 * d &&
+         16.0f * 5.9604645e-08f * T * l1 < g * d;
 }
 
 // Corner of the widened half-planes i and j: the solution of
 // a_i x + b_i y + c_i = 0 = a_j x + b_j y + c_j by Cramer's rule, with a
 // bound on its rounding error: N and D each carry at most 2u times the sum
-// of their products' magnitudes, the quotient 2u relative (u = 2^-24); the
-// bound below doubles both.  False when the corner's error could exceed a
-// quarter pixel (scales psx, psy: pixels per NDC unit) or D's sign is not
-// certain.  *d returns D = cross((a_i, b_i), (a_j, b_j)).
+// of their products' magnitudes (the bound below doubles that), the product
+// with the approximate reciprocal (1 ulp) at most 3u relative (u = 2^-24; the
+// bound takes 4u).  False when the corner's error could exceed a quarter
+// pixel (scales psx, psy: pixels per NDC unit), D's sign is not certain or D
+// leaves the approximate reciprocal's range.  *d returns D = cross((a_i, b_i),
+// (a_j, b_j)).
 __device__ __forceinline__ bool widened_corner(float ai, float bi, float ci, float aj, float bj, float cj, float psx,
                                                float psy, float* x, float* y, float* d) {
   constexpr float u4 = 4.0f * 5.9604645e-08f;
   const float D = ai * bj - aj * bi;
   const float eD = fabsf(ai * bj) + fabsf(aj * bi);
-  const float r = 1.0f / D;
+  const float r = __fdividef(1.0f, D);
   *x = (bi * cj - bj * ci) * r;
   *y = (aj * ci - ai * cj) * r;
   *d = D;
   const float ex = u4 * ((fabsf(bi * cj) + fabsf(bj * ci) + fabsf(*x) * eD) * fabsf(r) + fabsf(*x));
   const float ey = u4 * ((fabsf(aj * ci) + fabsf(ai * cj) + fabsf(*y) * eD) * fabsf(r) + fabsf(*y));
   // written so that NaN or inf anywhere fails
-  return fabsf(D) > 2.0f * u4 * eD && ex * psx < 0.25f && ey * psy < 0.25f;
+  return fabsf(D) > 2.0f * u4 * eD && fabsf(D) < 1e37f && ex * psx < 0.25f && ey * psy < 0.25f;
 }
 
 // The region where all three widened edge functions are >= 0 is a bounded
@@ -203,20 +265,10 @@ __device__ __forceinline__ bool coverage_bbox(const float* inv, const RastJob& J
   const int W = J.width, H = J.height;
   const float sx = J.viewport[0], ox = J.viewport[3];
   const float sy = J.viewport[5], oy = J.viewport[7];
-  bool finite = true;
-#pragma unroll
-  for (int k = 0; k < 9; ++k) finite = finite && isfinite(inv[k]);
-  if (!finite || !R.ok) {
-    *i0 = 0;
-    *i1 = W - 1;
-    *j0 = 0;
-    *j1 = H - 1;
-    return true;  // cannot bound: every pixel of the job
-  }
   const float xl = R.xl, xh = R.xh, yl = R.yl, yh = R.yh, X = R.X, Y = R.Y;
   // edge k: a_k x + b_k y + (c_k + eps_k), kept in scalars (no arrays: the
   // clip stages below capture them)
-  bool small = true;  // |c_k| < 1e37 on the rectangle: no overflow below
+  bool small = R.ok;  // |c_k| < 1e37 on the rectangle: no overflow below (NaN and infinite entries fail)
   auto widened = [&](float a, float b, float c) {
     const float bound = X * fabsf(a) + Y * fabsf(b) + fabsf(c);
     small = small && bound < 1e37f;
@@ -230,7 +282,7 @@ __device__ __forceinline__ bool coverage_bbox(const float* inv, const RastJob& J
     *i1 = W - 1;
     *j0 = 0;
     *j1 = H - 1;
-    return true;  // edge functions too large to evaluate safely: every pixel
+    return true;  // cannot bound, or edge functions too large to evaluate safely: every pixel of the job
   }
   float mnx, mxx, mny, mxy;
   float tx[3], ty[3];
@@ -312,10 +364,9 @@ __device__ __forceinline__ unsigned fast_div(unsigned n, unsigned long long inv)
   return inv == 0ull ? n : static_cast<unsigned>(__umul64hi(static_cast<unsigned long long>(n), inv));
 }
 
-// Per-face coverage rectangle in pixels, [x, z] x [y, w] (ushort4: i0, j0,
-// i1, j1); empty (x > z) for faces that are not binned.
-constexpr unsigned short kNoRect = 0xffff;
-__device__ __forceinline__ ushort4 empty_rect() { return make_ushort4(kNoRect, kNoRect, 0, 0); }
+__device__ __forceinline__ unsigned pack_pixel(int i, int j) {
+  return static_cast<unsigned>(i) | (static_cast<unsigned>(j) << 16);
+}
 
 // Vertex positions of face f of job J -> clip space (same operations as the
 // vertex shader's gl_Position).
@@ -373,39 +424,52 @@ __device__ __forceinline__ void warp_tiles(int tx0, int ty0, int tx1, int ty1, i
   }
 }
 
-// Phase 1, one thread per face: clip positions, determinant and keep/front
-// flags (written for every face).  Candidates (kept, front-facing) and face
+// Phase 1, one thread per face and round: clip positions, determinant,
+// keep/front flags and the off-screen test.  The faces that remain
+// (candidates: kept, front-facing and not known to miss the screen) and face
 // 0 (the chooser's fallback, whose record is read even when it is not a
 // candidate) are queued in shared memory with their [x, y, w] clip rows and
-// depths.  Phase 2, one thread per queued face, so culled faces leave no idle
-// lanes: the LU inverse -> setup record, and for candidates a conservative
-// coverage rectangle.  Rectangles of at most kSmallArea pixels (when near
-// ties are not counted) go to a second queue; the others are binned: the
-// warp adds their tile counts with one atomic per distinct tile per round
-// (lanes hitting the same tile merged with __match_any_sync).  Phase 3, one
-// warp per queued small face, one lane per pixel of its rectangle: the
-// raster kernel's edge tests and depth, folded into the per-pixel minimum of
-// the packed (depth | id) keys with a 64-bit atomicMin.
-// Grid: one block per kSetupThreads faces of a job (face block map).
+// depths.  Phase 2, one thread per queued face, so dropped faces leave no idle
+// lanes: the LU inverse and a conservative coverage rectangle; faces with a
+// rectangle get their setup record (inverse, depths, rectangle) and their
+// byte in `binned_flag`, the others leave no record.  Rectangles of at most
+// kSmallArea pixels (when near ties are not counted) go to a second queue;
+// the others are binned: the warp adds their tile counts with one atomic per
+// distinct tile per round (lanes hitting the same tile merged with
+// __match_any_sync).  Phase 3, one warp per queued small face, one lane per
+// pixel of its rectangle: the raster kernel's edge tests and depth, folded
+// into the per-pixel minimum of the packed (depth | id) keys with a 64-bit
+// atomicMin.
+// Grid: one block per setup_rows() faces of a job (face block map).
 constexpr int kRecordOnly = static_cast<int>(0x80000000u);  // queued for its record, not binned
 constexpr int kSmallArea = 32;                               // largest small rectangle: one pixel per lane
 constexpr int kTableMax = 1024;                              // pixel -> NDC tables kept in shared memory
 
 // 1,536 resident threads per SM without the small path (40 registers): the
-// kernel is latency-bound, and more resident warps beat the spills (0.83 /
-// 0.90 ms -> 0.73 / 0.76 ms per pass on the 4096-scene brax-like batch at 6
-// blocks of 256; 1,280 and 2,048 threads measured slower; 12 blocks of 128,
-// 0.71 / 0.74 ms).  The small path's shared arrays allow fewer.
+// kernel is latency- and issue-bound (position gathers, then the inverse's
+// division chains), and more resident warps beat the spills: 4096 brax-like
+// scenes, both passes, 1,076 us at 12 blocks of 128, 1,109 at 10, 1,248 at 8,
+// 1,382 at 14.  The small path's shared arrays allow fewer.
 __host__ __device__ constexpr int setup_min_blocks(bool small) { return small ? 0 : 1536 / kSetupThreads; }
+// Faces per block: rounds of one face per thread.  Two rounds fill phase 2's
+// warps better and pay the job load once per 256 faces (the whole step 4,000
+// us; one round 4,106, four 4,201, whose queue costs resident blocks).  The
+// off-screen test ahead of the inverse and records for binned faces only took
+// both passes from 1,488 to 1,046 us (of 23.3 M faces each: 0.25 ms of
+// positions at the measured copy rate).
+__host__ __device__ constexpr int setup_rounds(bool small) { return small ? 1 : 2; }
+__host__ __device__ constexpr int setup_rows(bool small) { return setup_rounds(small) * kSetupThreads; }
 
 template <bool kSmall>
 __global__ void __launch_bounds__(kSetupThreads, setup_min_blocks(kSmall))
 setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4* __restrict__ setup,
-                 ushort4* __restrict__ bbox, uint32_t* __restrict__ counts, unsigned long long* __restrict__ keys,
-                 int small_area, int4* __restrict__ binned, unsigned int* __restrict__ n_binned) {
+                 unsigned char* __restrict__ binned_flag, uint32_t* __restrict__ counts,
+                 unsigned long long* __restrict__ keys, int small_area, int4* __restrict__ binned,
+                 unsigned int* __restrict__ n_binned, const ScreenRect* __restrict__ rects) {
+  constexpr int kRounds = setup_rounds(kSmall), kRows = setup_rows(kSmall);
   __shared__ RastJob sJ;
-  __shared__ float s_m[12][kSetupThreads];
-  __shared__ int s_face[kSetupThreads];
+  __shared__ float s_m[12][kRows];
+  __shared__ int s_face[kRows];
   constexpr int kQ = kSmall ? kSetupThreads : 1;  // small-path arrays only where used
   constexpr int kT = kSmall ? kTableMax : 1;
   __shared__ float s_small[12][kQ];  // inverse (9) and clip depths (3) of small faces
@@ -419,6 +483,8 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
   const int jid = blk.x;
   const int nf = __ldg(&B.jobs[jid].n_faces);
   load_job_to_shared(B.jobs + jid, &sJ);
+  if (threadIdx.x < sizeof(ScreenRect) / 4)
+    reinterpret_cast<int*>(&s_rect)[threadIdx.x] = __ldg(reinterpret_cast<const int*>(rects + jid) + threadIdx.x);
   if (threadIdx.x == 0) s_qn = s_sn = 0;
   __syncthreads();
   const RastJob& J = sJ;
@@ -428,44 +494,47 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
     for (int i = threadIdx.x; i < J.width; i += kSetupThreads) s_xs[i] = (static_cast<float>(i) - ox) / sx;
     for (int j = threadIdx.x; j < J.height; j += kSetupThreads) s_ys[j] = (static_cast<float>(j) - oy) / sy;
   }
-  if (threadIdx.x == 0) s_rect = screen_rect(J);  // read after the queue's barrier
-  const int f = blk.y + static_cast<int>(threadIdx.x);
-  bool queued = false, cand = false;
-  float m[12];
-  if (f < nf) {
-    const int64_t row = J.setup_begin + f;
-    float4 c[3];
-    face_clip(J, B.pools, f, c);
+#pragma unroll 1
+  for (int round = 0; round < kRounds; ++round) {
+    const int f = blk.y + round * kSetupThreads + static_cast<int>(threadIdx.x);
+    bool queued = false, cand = false;
+    float m[12];
+    if (f < nf) {
+      const int64_t row = J.setup_begin + f;
+      float4 c[3];
+      face_clip(J, B.pools, f, c);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      m[3 * k + 0] = c[k].x;
-      m[3 * k + 1] = c[k].y;
-      m[3 * k + 2] = c[k].w;
-      m[9 + k] = c[k].z;
+      for (int k = 0; k < 3; ++k) {
+        m[3 * k + 0] = c[k].x;
+        m[3 * k + 1] = c[k].y;
+        m[3 * k + 2] = c[k].w;
+        m[9 + k] = c[k].z;
+      }
+      const float det = det3(m);
+      int flags = 0;
+      if (fabsf(det) > 1e-6f) flags |= kKeep;
+      if (det >= 0.0f) flags |= kFront;
+      cand = (flags & kCandidate) == kCandidate && !off_screen(m, det, s_rect);
+      queued = cand || f == 0;
+      if (f == 0) setup[row * 4 + 3] = make_float4(0.0f, __int_as_float(flags), 0.0f, 0.0f);
+      binned_flag[row] = 0;
     }
-    const float det = det3(m);
-    int flags = 0;
-    if (fabsf(det) > 1e-6f) flags |= kKeep;
-    if (det >= 0.0f) flags |= kFront;
-    setup[row * 4 + 3] = make_float4(det, __int_as_float(flags), 0.0f, 0.0f);
-    cand = (flags & kCandidate) == kCandidate;
-    queued = cand || f == 0;
-    if (!cand) bbox[row] = empty_rect();
-  }
-  const unsigned qm = __ballot_sync(0xffffffffu, queued);
-  int base = 0;
-  if ((threadIdx.x & 31) == 0 && qm) base = atomicAdd(&s_qn, __popc(qm));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (queued) {
-    const int q = base + __popc(qm & lanemask_lt());
-    s_face[q] = cand ? f : (f | kRecordOnly);
+    const unsigned qm = __ballot_sync(0xffffffffu, queued);
+    int base = 0;
+    if ((threadIdx.x & 31) == 0 && qm) base = atomicAdd(&s_qn, __popc(qm));
+    base = __shfl_sync(0xffffffffu, base, 0);
+    if (queued) {
+      const int q = base + __popc(qm & lanemask_lt());
+      s_face[q] = cand ? f : (f | kRecordOnly);
 #pragma unroll
-    for (int k = 0; k < 12; ++k) s_m[k][q] = m[k];
+      for (int k = 0; k < 12; ++k) s_m[k][q] = m[k];
+    }
   }
   __syncthreads();
   const int qn = s_qn;
-  const int q = threadIdx.x;
-  if (static_cast<int>(threadIdx.x & ~31u) < qn) {  // warps holding queued faces
+#pragma unroll 1
+  for (int q0 = static_cast<int>(threadIdx.x & ~31u); q0 < qn; q0 += kSetupThreads) {  // warps holding queued faces
+    const int q = q0 + static_cast<int>(threadIdx.x & 31u);
     int tx0 = 1, ty0 = 1, tx1 = 0, ty1 = 0;
     bool small = false;
     int fq = 0, i0 = 0, i1 = 0, j0 = 0, j1 = 0;
@@ -478,23 +547,25 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
       for (int k = 0; k < 9; ++k) mq[k] = s_m[k][q];
       inv3(mq, iv);
       float4* out = setup + (J.setup_begin + fq) * 4;
-      out[0] = make_float4(iv[0], iv[1], iv[2], iv[3]);
-      out[1] = make_float4(iv[4], iv[5], iv[6], iv[7]);
-      out[2] = make_float4(iv[8], s_m[9][q], s_m[10][q], s_m[11][q]);
-      if (!(entry & kRecordOnly)) {
-        ushort4 bb = empty_rect();
-        if (coverage_bbox(iv, J, s_rect, &i0, &i1, &j0, &j1)) {
-          if (kSmall && (i1 - i0 + 1) * (j1 - j0 + 1) <= small_area) {
-            small = true;  // rasterised in phase 3, not binned
-          } else {
-            tx0 = i0 >> G.tws;
-            tx1 = i1 >> G.tws;
-            ty0 = j0 >> G.ths;
-            ty1 = j1 >> G.ths;
-            bb = make_ushort4(i0, j0, i1, j1);  // the raster kernel tests only these pixels of each tile
-          }
+      const bool covers = !(entry & kRecordOnly) && coverage_bbox(iv, J, s_rect, &i0, &i1, &j0, &j1);
+      if (covers || fq == 0) {
+        out[0] = make_float4(iv[0], iv[1], iv[2], iv[3]);
+        out[1] = make_float4(iv[4], iv[5], iv[6], iv[7]);
+        out[2] = make_float4(iv[8], s_m[9][q], s_m[10][q], s_m[11][q]);
+      }
+      if (covers) {
+        if (kSmall && (i1 - i0 + 1) * (j1 - j0 + 1) <= small_area) {
+          small = true;  // rasterised in phase 3, not binned
+        } else {
+          tx0 = i0 >> G.tws;
+          tx1 = i1 >> G.tws;
+          ty0 = j0 >> G.ths;
+          ty1 = j1 >> G.ths;
+          // the raster kernel tests only these pixels of each tile
+          out[3] = make_float4(__uint_as_float(pack_pixel(i0, j0)), __int_as_float(kCandidate),
+                               __uint_as_float(pack_pixel(i1, j1)), 0.0f);
+          binned_flag[J.setup_begin + fq] = 1;
         }
-        bbox[J.setup_begin + fq] = bb;
       }
     }
     const unsigned sm = kSmall ? __ballot_sync(0xffffffffu, small) : 0u;
@@ -519,8 +590,7 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
     bbase = __shfl_sync(0xffffffffu, bbase, 0);
     if (bin)
       binned[bbase + __popc(bm & lanemask_lt())] =
-          make_int4(jid, fq, static_cast<int>(static_cast<unsigned>(i0) | (static_cast<unsigned>(j0) << 16)),
-                    static_cast<int>(static_cast<unsigned>(i1) | (static_cast<unsigned>(j1) << 16)));
+          make_int4(jid, fq, static_cast<int>(pack_pixel(i0, j0)), static_cast<int>(pack_pixel(i1, j1)));
     uint32_t* cnt = counts + static_cast<int64_t>(jid) * G.tiles_per_job;
     warp_tiles(tx0, ty0, tx1, ty1, G.tiles_x, [&](int, int tile, bool valid) {
       const unsigned peers = __match_any_sync(0xffffffffu, valid ? tile : -1);
@@ -566,6 +636,7 @@ struct BeginWork {
   size_t zero_bytes[3];
   void* keys;  // small path: every key starts as kEmptyKey
   size_t key_bytes;
+  ScreenRect* rects;  // per job
 };
 
 __global__ void __launch_bounds__(256) begin_kernel(RastBatch B, BeginWork w) {
@@ -574,6 +645,9 @@ __global__ void __launch_bounds__(256) begin_kernel(RastBatch B, BeginWork w) {
   fill_words(w.keys, w.key_bytes, 0xffffffffu);
   fill_block_map<kMapFaces>(B.jobs, B.n_jobs, w.map_rows, w.fmap, w.fmap_blocks);
   fill_block_map<kMapFaces>(B.jobs, B.n_jobs, kVaryRows, w.vmap, w.vmap_blocks);
+  for (int j = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); j < B.n_jobs;
+       j += static_cast<int>(gridDim.x * blockDim.x))
+    w.rects[j] = screen_rect(B.jobs[j]);
 }
 
 // Bin offsets: a tile only needs a contiguous range of the bins, in no
@@ -736,7 +810,7 @@ __device__ __forceinline__ bool depth_of_order(uint32_t o, float* z) {
 // reads the tile's whole bin and drops the entries that miss its rows).
 template <int TW, int TH, bool kKeys, bool kTies, int kL, int kWPT>
 __global__ void __launch_bounds__(32 * kRasterWarps, raster_min_blocks<TW, TH, kL, kL == 1 && !kTies>())
-raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const ushort4* __restrict__ rects,
+raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const unsigned char* __restrict__ binned_flag,
               const uint32_t* __restrict__ counts, const uint32_t* __restrict__ offsets,
               const int32_t* __restrict__ bins, int32_t* __restrict__ winner,
               unsigned int* __restrict__ work, int64_t n_units, unsigned char* __restrict__ visible,
@@ -799,29 +873,30 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
       continue;
     }
     const float4* jrec = setup + J.setup_begin * 4;
-    const ushort4* jrect = rects + J.setup_begin;
     const bool overflow = (off & kOverflow) != 0;
     const int n = overflow ? J.n_faces : static_cast<int>(t_count);
-    // entry `e` of the tile's list -> (record, id, rectangle); ids of
-    // non-candidates (only met on the full-scan path) are -1 and their
-    // records unused
-    auto fetch = [&](int e, float4& r0, float4& r1, float4& r2, int& id, ushort4& rc) {
+    // entry `e` of the tile's list -> (record, id, rectangle: i0 | j0 << 16,
+    // i1 | j1 << 16); on the full-scan path faces that are not binned (no
+    // candidates, or off every pixel) have no record: their ids are -1
+    auto fetch = [&](int e, float4& r0, float4& r1, float4& r2, int& id, uint2& rc) {
       const int fid = overflow ? e : __ldg(bins + static_cast<int64_t>(off) + e);
       const float4* r = jrec + static_cast<int64_t>(fid) * 4;
       id = fid;
-      if (kPairs) rc = __ldg(jrect + fid);
-      if (overflow && (__float_as_int(__ldg(r + 3).y) & kCandidate) != kCandidate) {
+      if (overflow && !__ldg(binned_flag + J.setup_begin + fid)) {
         id = -1;
-        r0 = r1 = r2 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         return;
       }
       r0 = __ldg(r);
       r1 = __ldg(r + 1);
       r2 = __ldg(r + 2);
+      if (kPairs) {
+        const float4 r3 = __ldg(r + 3);
+        rc = make_uint2(__float_as_uint(r3.x), __float_as_uint(r3.z));
+      }
     };
     float4 n0, n1, n2;
     int nid = -1;
-    ushort4 nrc = empty_rect();
+    uint2 nrc = make_uint2(0u, 0u);
     if (lane < n) fetch(lane, n0, n1, n2, nid, nrc);  // first: its loads overlap the tile's set-up
     const float sx = J.viewport[0], ox = J.viewport[3], sy = J.viewport[5], oy = J.viewport[7];
     const float vp22 = J.viewport[10], vp23 = J.viewport[11];
@@ -886,11 +961,9 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
       int cnt = 0, pinfo = 0;
       float prcp = 0.0f;
       if (kPairs) {
-        // the entry's rectangle cut to the warp's pixels (tile-local); on
-        // the full-scan path faces without one (small faces of the set-up's
-        // own rasterisation, non-candidates) drop out here
-        const int lx0 = max(static_cast<int>(nrc.x) - x0, 0), lx1 = min(static_cast<int>(nrc.z) - x0, lxe);
-        const int ly0 = max(static_cast<int>(nrc.y) - y0, 0), ly1 = min(static_cast<int>(nrc.w) - y0, lye);
+        // the entry's rectangle cut to the warp's pixels (tile-local)
+        const int lx0 = max(static_cast<int>(nrc.x & 0xffffu) - x0, 0), lx1 = min(static_cast<int>(nrc.y & 0xffffu) - x0, lxe);
+        const int ly0 = max(static_cast<int>(nrc.x >> 16) - y0, 0), ly1 = min(static_cast<int>(nrc.y >> 16) - y0, lye);
         take = take && lx0 <= lx1 && ly0 <= ly1;
         if (take) {
           const float ra = tx_ndc[lx0], rb = tx_ndc[lx1], sa = ty_ndc[ly0], sb = ty_ndc[ly1];
@@ -1188,8 +1261,8 @@ inline uint64_t default_bin_capacity(const RastBatch& b) {
 }
 
 struct Layout {
-  size_t setup_off, bbox_off, binned_off, counts_off, offsets_off, cursors_off, bins_off, winner_off, vis_off, fvar_off,
-      fmap_off, vmap_off, keys_off, misc_off, total;
+  size_t setup_off, flag_off, binned_off, counts_off, offsets_off, cursors_off, bins_off, winner_off, vis_off, fvar_off,
+      fmap_off, vmap_off, rect_off, keys_off, misc_off, total;
   unsigned fmap_blocks, vmap_blocks;  // face block maps: setup/scatter, face varyings
   bool small_path;  // setup kernel rasterises small faces (not when near ties are counted)
   int vstride;
@@ -1220,7 +1293,7 @@ static Layout layout(const RastBatch& b, TileShape ts, uint64_t bin_capacity, in
     return o;
   };
   L.setup_off = take(static_cast<size_t>(b.total_setup) * 64);
-  L.bbox_off = take(static_cast<size_t>(b.total_setup) * sizeof(ushort4));
+  L.flag_off = take(static_cast<size_t>(b.total_setup));
   L.binned_off = take(static_cast<size_t>(b.total_setup) * sizeof(int4));
   L.counts_off = take(static_cast<size_t>(L.n_tiles) * 4);
   L.cursors_off = take(static_cast<size_t>(L.n_tiles) * 4);
@@ -1235,12 +1308,13 @@ static Layout layout(const RastBatch& b, TileShape ts, uint64_t bin_capacity, in
   const bool shading = vstride > 0;
   L.vis_off = take(shading ? static_cast<size_t>(b.total_setup) : 0);
   L.fvar_off = take(shading ? static_cast<size_t>(b.total_setup) * 3 * vstride * sizeof(float) : 0);
-  L.fmap_blocks = block_map_capacity(b.total_setup, b.n_jobs, kSetupThreads);
+  L.small_path = b.near_ties == nullptr && small_area > 0 && b.max_layers == 0;
+  L.fmap_blocks = block_map_capacity(b.total_setup, b.n_jobs, setup_rows(L.small_path));
   L.fmap_off = take(static_cast<size_t>(L.fmap_blocks) * sizeof(int2));
   L.vmap_blocks = shading ? block_map_capacity(b.total_setup, b.n_jobs, kVaryRows) : 0;
   L.vmap_off = take(static_cast<size_t>(L.vmap_blocks) * sizeof(int2));
-  L.small_path = b.near_ties == nullptr && small_area > 0 && b.max_layers == 0;
   L.keys_off = take(L.small_path ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0);
+  L.rect_off = take(static_cast<size_t>(b.n_jobs) * sizeof(ScreenRect));
   L.misc_off = take(256);
   L.total = off;
   return L;
@@ -1292,7 +1366,7 @@ template <bool kKeys, bool kTies, int kL>
 // blocks of this instance that fit on an SM) takes the work units (bin
 // tiles x warps per tile).
 static void launch_raster(TileShape ts, int wpt, int sms, cudaStream_t s, const RastBatch& b, const Layout& L,
-                          const float4* setup, const ushort4* rects, const uint32_t* counts, const uint32_t* offsets, const int32_t* bins,
+                          const float4* setup, const unsigned char* flag, const uint32_t* counts, const uint32_t* offsets, const int32_t* bins,
                           int32_t* winner, unsigned int* misc, unsigned char* vis,
                           const unsigned long long* keys) {
   const unsigned block = 32 * kRasterWarps;
@@ -1302,7 +1376,7 @@ static void launch_raster(TileShape ts, int wpt, int sms, cudaStream_t s, const 
         per_sm <= 0)
       per_sm = 8;
     const unsigned grid = static_cast<unsigned>(std::max(sms, 1) * per_sm);
-    kernel<<<grid, block, 0, s>>>(b, L.G, setup, rects, counts, offsets, bins, winner, misc, L.n_tiles * wpt, vis,
+    kernel<<<grid, block, 0, s>>>(b, L.G, setup, flag, counts, offsets, bins, winner, misc, L.n_tiles * wpt, vis,
                                   keys);
   };
   if (wpt == 2) {  // the warp's sub-tile is (tw, th / 2)
@@ -1353,7 +1427,7 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
   float4* setup = reinterpret_cast<float4*>(ws + L.setup_off);
-  ushort4* bbox = reinterpret_cast<ushort4*>(ws + L.bbox_off);
+  unsigned char* flag = reinterpret_cast<unsigned char*>(ws + L.flag_off);
   uint32_t* counts = reinterpret_cast<uint32_t*>(ws + L.counts_off);
   uint32_t* cursors = reinterpret_cast<uint32_t*>(ws + L.cursors_off);
   uint32_t* offsets = reinterpret_cast<uint32_t*>(ws + L.offsets_off);
@@ -1380,7 +1454,7 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
     BeginWork bw{};
     bw.fmap = fmap;
     bw.fmap_blocks = b.total_setup > 0 ? L.fmap_blocks : 0u;
-    bw.map_rows = kSetupThreads;
+    bw.map_rows = setup_rows(L.small_path);
     bw.vmap = reinterpret_cast<int2*>(ws + L.vmap_off);
     bw.vmap_blocks = pre ? L.vmap_blocks : 0u;
     bw.zero[0] = counts;  // counts and cursors are adjacent
@@ -1390,17 +1464,18 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
     bw.zero[2] = vis;
     bw.zero_bytes[2] = vis ? static_cast<size_t>(b.total_setup) : 0;
     bw.keys = keys;
+    bw.rects = reinterpret_cast<ScreenRect*>(ws + L.rect_off);
     bw.key_bytes = keys ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0;
     begin_kernel<<<begin_blocks(bw.zero_bytes[0] + bw.zero_bytes[2] + bw.key_bytes, b.n_jobs, sms), 256, 0, s>>>(b, bw);
     prof.mark("begin_kernel");
     if (b.total_setup > 0) {
       const unsigned grid = L.fmap_blocks;
       if (keys)
-        setup_bin_kernel<true><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, bbox, counts, keys, small_area,
-                                                             binned, misc + 6);
+        setup_bin_kernel<true><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, flag, counts, keys, small_area,
+                                                             binned, misc + 6, bw.rects);
       else
-        setup_bin_kernel<false><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, bbox, counts, nullptr, 0,
-                                                              binned, misc + 6);
+        setup_bin_kernel<false><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, flag, counts, nullptr, 0,
+                                                              binned, misc + 6, bw.rects);
       prof.mark("setup_bin_kernel");
       offsets_kernel<<<static_cast<unsigned>(L.n_scan_blocks), 256, 0, s>>>(
           counts, offsets, L.n_tiles, L.bin_capacity, misc + 1, reinterpret_cast<unsigned long long*>(misc + 2));
@@ -1415,18 +1490,18 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
         // the key path exists only when ties are not counted and no job is
         // layered
         if (keys)
-          launch_raster<true, false, 1>(ts, wpt, sms, s, b, L, setup, bbox, counts, offsets, bins, winner, misc, vis, keys);
+          launch_raster<true, false, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, keys);
         else if (b.max_layers > 0 && b.near_ties)
-          launch_raster<false, true, RAST_MAX_LAYERS>(ts, wpt, sms, s, b, L, setup, bbox, counts, offsets, bins, winner,
+          launch_raster<false, true, RAST_MAX_LAYERS>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner,
                                                       misc, vis, nullptr);
         else if (b.max_layers > 0)
-          launch_raster<false, false, RAST_MAX_LAYERS>(ts, wpt, sms, s, b, L, setup, bbox, counts, offsets, bins, winner,
+          launch_raster<false, false, RAST_MAX_LAYERS>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner,
                                                        misc, vis, nullptr);
         else if (b.near_ties)
-          launch_raster<false, true, 1>(ts, wpt, sms, s, b, L, setup, bbox, counts, offsets, bins, winner, misc, vis,
+          launch_raster<false, true, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis,
                                         nullptr);
         else
-          launch_raster<false, false, 1>(ts, wpt, sms, s, b, L, setup, bbox, counts, offsets, bins, winner, misc, vis,
+          launch_raster<false, false, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis,
                                          nullptr);
       } else {
         if (cudaMemsetAsync(winner, 0xff, static_cast<size_t>(b.total_pixels) * 4 * L.winner_layers, s) !=
