@@ -37,9 +37,7 @@ constexpr int kScanBlock = 1024;       // elements per scan block (256 threads x
 constexpr int kRasterWarps = 4;        // warps per CTA of the raster kernel
 constexpr int kStage = 32;             // bin entries staged per warp round
 constexpr uint32_t kOverflow = 0x80000000u;
-constexpr int kFaceThreads = 256;      // threads and faces per block of the face varyings
-constexpr int kVaryRowsPerThread = 16;
-constexpr int kVaryRows = kFaceThreads * kVaryRowsPerThread;
+constexpr int kFaceThreads = 128;      // threads per block of the face varyings
 
 // Tile shapes offered to the autotuner.  (tw, th): tw pixels along x
 // (axis 0 of the buffers), th along y (contiguous in memory).
@@ -630,8 +628,6 @@ struct BeginWork {
   int2* fmap;
   unsigned fmap_blocks;
   int map_rows;  // faces per block of the map
-  int2* vmap;    // the face varyings' map (kVaryRows faces per block)
-  unsigned vmap_blocks;
   void* zero[3];
   size_t zero_bytes[3];
   void* keys;  // small path: every key starts as kEmptyKey
@@ -644,7 +640,6 @@ __global__ void __launch_bounds__(256) begin_kernel(RastBatch B, BeginWork w) {
   for (int k = 0; k < 3; ++k) fill_words(w.zero[k], w.zero_bytes[k], 0u);
   fill_words(w.keys, w.key_bytes, 0xffffffffu);
   fill_block_map<kMapFaces>(B.jobs, B.n_jobs, w.map_rows, w.fmap, w.fmap_blocks);
-  fill_block_map<kMapFaces>(B.jobs, B.n_jobs, kVaryRows, w.vmap, w.vmap_blocks);
   for (int j = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); j < B.n_jobs;
        j += static_cast<int>(gridDim.x * blockDim.x))
     w.rects[j] = screen_rect(B.jobs[j]);
@@ -813,7 +808,7 @@ __global__ void __launch_bounds__(32 * kRasterWarps, raster_min_blocks<TW, TH, k
 raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const unsigned char* __restrict__ binned_flag,
               const uint32_t* __restrict__ counts, const uint32_t* __restrict__ offsets,
               const int32_t* __restrict__ bins, int32_t* __restrict__ winner,
-              unsigned int* __restrict__ work, int64_t n_units, unsigned char* __restrict__ visible,
+              unsigned int* __restrict__ work, int64_t n_units, uint32_t* __restrict__ visible,
               const unsigned long long* __restrict__ keys) {
   constexpr int PPL = TW * TH / 32;
   constexpr bool kPairs = kL == 1 && !kTies;
@@ -1085,6 +1080,29 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
     }
     const bool depth_only = J.shader == RAST_SHADER_DEPTH;
     const int layers = kL > 1 ? job_layers(J, B.max_layers) : 0;
+    // Faces whose varyings the shade needs (winners, and face 0 for the
+    // default chooser's fallback): one bit each, set by the first pixel of a
+    // run of equal winners.
+    auto mark = [&](int w, bool shown) {
+      const int prev = __shfl_up_sync(0xffffffffu, shown ? w : -1, 1);
+      if (shown && (lane == 0 || prev != w)) {
+        const int64_t row = J.setup_begin + w;
+        atomicOr(visible + (row >> 5), 1u << (row & 31));
+      }
+    };
+    if (visible && !depth_only && J.n_faces > 0) {
+#pragma unroll
+      for (int q = 0; q < PPL; ++q) {
+        const bool inside = x0 + q * LPC + lane / TH < W && pj < H;
+#pragma unroll
+        for (int l = 0; l < kL; ++l) {
+          const uint32_t o = static_cast<uint32_t>(best[q][l] >> 32);
+          const bool found = !(best[q][l] == kEmptyKey || o == kInfOrder);
+          mark(found ? static_cast<int>(best[q][l] & 0xffffffffu) : 0,
+               inside && (l == 0 ? found || layers == 0 : found && l < layers));
+        }
+      }
+    }
 #pragma unroll
     for (int q = 0; q < PPL; ++q) {
       const int pi = x0 + q * LPC + lane / TH;
@@ -1096,16 +1114,12 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
         if (!depth_only) {
           const int32_t w = found ? static_cast<int32_t>(best[q][0] & 0xffffffffu) : -1;
           winner[pix] = w;
-          // faces whose varyings the shade needs: winners, and face 0 for the
-          // default chooser's fallback
-          if (visible && J.n_faces > 0 && (layers == 0 || w >= 0)) visible[J.setup_begin + (w < 0 ? 0 : w)] = 1;
 #pragma unroll
           for (int l = 1; l < kL; ++l) {
             const uint32_t o = static_cast<uint32_t>(best[q][l] >> 32);
             const int32_t wl = (best[q][l] == kEmptyKey || o == kInfOrder) ? -1
                                                                           : static_cast<int32_t>(best[q][l] & 0xffffffffu);
             winner[l * B.total_pixels + pix] = wl;
-            if (visible && wl >= 0 && l < layers) visible[J.setup_begin + wl] = 1;
           }
           continue;
         }
@@ -1152,40 +1166,72 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
 
 // Vertex varyings of the three corners of every face some pixel needs
 // (marked by the raster kernel), stored per face: the shade then reads them
-// instead of re-running the vertex shader per pixel.  A block covers
-// kVaryRows faces of one job (its own block map): it queues the visible ones
-// in shared memory, then one thread per (visible face, corner) runs the
-// vertex shader, so faces nobody sees leave no idle lanes and the block's
-// job load and queue are paid once per kVaryRows faces.
-
-__global__ void __launch_bounds__(kFaceThreads)
-face_varyings_kernel(RastBatch B, const int2* __restrict__ vmap, const unsigned char* __restrict__ visible,
-                     float* __restrict__ fvar, int vstride) {
-  __shared__ RastJob sJ;
-  __shared__ int s_face[kVaryRows];
-  __shared__ int s_n;
-  const int2 blk = vmap[blockIdx.x];
+// instead of re-running the vertex shader per pixel.  `split` warps per entry
+// of the set-up's block map: each lists the entry's marked faces in shared
+// memory (eight mark bits per lane), then takes one (face, corner) per lane
+// and round, in memory order.  Gathers and normalisation chains bound it, at
+// 4096 brax-like scenes the sectors that 3.8 M faces' corners and rows touch
+// (1.2 GB): warps independent of one another (no block barrier, no shared job
+// copy) and 40 registers take it to 266 us, from 294 with blocks that queued
+// 4,096 faces.  A list that the raster kernel appended to balanced small
+// batches as well but lost the memory order (336 us).  Few entries (a batch
+// of 16 scenes has 700) take several warps each, so that a warp's rounds,
+// 2-3 us of latency each, do not follow one another while SMs idle.
+template <int kRows>
+__global__ void __launch_bounds__(kFaceThreads, 12)
+face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entries, unsigned split,
+                     const uint32_t* __restrict__ visible, float* __restrict__ fvar, int vstride) {
+  static_assert(kRows <= 256 && kRows % 32 == 0, "eight faces per lane, list entries of one byte");
+  __shared__ unsigned char s_list[kFaceThreads / 32][kRows];
+  const int lane = threadIdx.x & 31;
+  unsigned char* list = s_list[threadIdx.x >> 5];
+  const unsigned wid = (blockIdx.x * kFaceThreads + threadIdx.x) >> 5;
+  const unsigned entry = wid / split;
+  if (entry >= entries) return;  // whole warps
+  const int2 blk = fmap[entry];
   if (blk.x < 0) return;
-  const int jid = blk.x;
-  const int nf = __ldg(&B.jobs[jid].n_faces);
-  if (__ldg(&B.jobs[jid].shader) == RAST_SHADER_DEPTH) return;
-  load_job_to_shared(B.jobs + jid, &sJ);
-  if (threadIdx.x == 0) s_n = 0;
-  __syncthreads();
-  const RastJob& J = sJ;
-  const int pairs = 3 * block_queue_rows<kVaryRowsPerThread, kFaceThreads>(
-                            [&](int r) { return blk.y + r < nf && visible[J.setup_begin + blk.y + r]; }, s_face, &s_n);
+  const RastJob& J = B.jobs[blk.x];
+  if (J.shader == RAST_SHADER_DEPTH) return;
+  // lane l: the mark bits of faces [8 l, 8 l + 8) of the entry
+  const int64_t row0 = J.setup_begin + blk.y;
+  const int left = min(kRows, J.n_faces - blk.y) - 8 * lane;
+  unsigned bits = 0;
+  if (left > 0) {
+    const int64_t at = row0 + 8 * lane;
+    const unsigned shift = static_cast<unsigned>(at & 31);
+    bits = visible[at >> 5] >> shift;
+    if (shift > 24 && left > 32 - static_cast<int>(shift)) bits |= visible[(at >> 5) + 1] << (32 - shift);
+    bits &= left >= 8 ? 0xffu : (1u << left) - 1u;
+  }
+  int incl = __popc(bits);
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  const int total = 3 * __shfl_sync(0xffffffffu, incl, 31);
+  int slot = incl - __popc(bits);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if ((bits >> k) & 1u) list[slot++] = static_cast<unsigned char>(8 * lane + k);
+  __syncwarp();
   const int nv = varying_count(J.shader);
-  for (int t = threadIdx.x; t < pairs; t += kFaceThreads) {
+  for (int t = static_cast<int>(wid - entry * split) * 32 + lane; t < total; t += 32 * static_cast<int>(split)) {
     const int q = t / 3, k = t - 3 * q;
-    const int fq = blk.y + s_face[q];
+    const int fq = blk.y + list[q];
     const int32_t* face = B.pools.faces + (J.face_begin + fq) * 3;
     float var[kMaxVarying], clip[4];
     vertex_shader<false>(J, B.pools, gather_clamp(__ldg(face + k), J.n_verts), clip, var);
     float* out = fvar + ((J.setup_begin + fq) * 3 + k) * vstride;
+    if (vstride % 2 == 0) {  // rows of whole float2 (a job with an odd count leaves one float of its row unset)
 #pragma unroll
-    for (int v = 0; v < kMaxVarying; ++v)
-      if (v < nv) out[v] = var[v];
+      for (int v = 0; v < kMaxVarying; v += 2)
+        if (v < nv) *reinterpret_cast<float2*>(out + v) = make_float2(var[v], var[v + 1]);
+    } else {
+#pragma unroll
+      for (int v = 0; v < kMaxVarying; ++v)
+        if (v < nv) out[v] = var[v];
+    }
   }
 }
 
@@ -1262,8 +1308,8 @@ inline uint64_t default_bin_capacity(const RastBatch& b) {
 
 struct Layout {
   size_t setup_off, flag_off, binned_off, counts_off, offsets_off, cursors_off, bins_off, winner_off, vis_off, fvar_off,
-      fmap_off, vmap_off, rect_off, keys_off, misc_off, total;
-  unsigned fmap_blocks, vmap_blocks;  // face block maps: setup/scatter, face varyings
+      fmap_off, rect_off, keys_off, misc_off, total;
+  unsigned fmap_blocks;  // face block map of the set-up
   bool small_path;  // setup kernel rasterises small faces (not when near ties are counted)
   int vstride;
   int winner_layers;  // chooser slots kept per pixel: 1, or RAST_MAX_LAYERS with layered jobs
@@ -1306,13 +1352,11 @@ static Layout layout(const RastBatch& b, TileShape ts, uint64_t bin_capacity, in
     if (b.shader_mask & (1 << sh)) vstride = std::max(vstride, varying_count(sh));
   L.vstride = vstride;
   const bool shading = vstride > 0;
-  L.vis_off = take(shading ? static_cast<size_t>(b.total_setup) : 0);
+  L.vis_off = take(shading ? (static_cast<size_t>(b.total_setup) + 31) / 32 * 4 : 0);
   L.fvar_off = take(shading ? static_cast<size_t>(b.total_setup) * 3 * vstride * sizeof(float) : 0);
   L.small_path = b.near_ties == nullptr && small_area > 0 && b.max_layers == 0;
   L.fmap_blocks = block_map_capacity(b.total_setup, b.n_jobs, setup_rows(L.small_path));
   L.fmap_off = take(static_cast<size_t>(L.fmap_blocks) * sizeof(int2));
-  L.vmap_blocks = shading ? block_map_capacity(b.total_setup, b.n_jobs, kVaryRows) : 0;
-  L.vmap_off = take(static_cast<size_t>(L.vmap_blocks) * sizeof(int2));
   L.keys_off = take(L.small_path ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0);
   L.rect_off = take(static_cast<size_t>(b.n_jobs) * sizeof(ScreenRect));
   L.misc_off = take(256);
@@ -1367,8 +1411,7 @@ template <bool kKeys, bool kTies, int kL>
 // tiles x warps per tile).
 static void launch_raster(TileShape ts, int wpt, int sms, cudaStream_t s, const RastBatch& b, const Layout& L,
                           const float4* setup, const unsigned char* flag, const uint32_t* counts, const uint32_t* offsets, const int32_t* bins,
-                          int32_t* winner, unsigned int* misc, unsigned char* vis,
-                          const unsigned long long* keys) {
+                          int32_t* winner, unsigned int* misc, uint32_t* vis, const unsigned long long* keys) {
   const unsigned block = 32 * kRasterWarps;
   auto go = [&](auto kernel) {
     int per_sm = 0;
@@ -1440,7 +1483,7 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
   Profiler prof(profile, s, "rast_render_tiled");
 
   const bool cover = (phase & RAST_PHASE_COVERAGE) != 0, shade = (phase & RAST_PHASE_SHADE) != 0;
-  unsigned char* vis = L.vstride > 0 ? reinterpret_cast<unsigned char*>(ws + L.vis_off) : nullptr;
+  uint32_t* vis = L.vstride > 0 ? reinterpret_cast<uint32_t*>(ws + L.vis_off) : nullptr;
   float* fvar = L.vstride > 0 ? reinterpret_cast<float*>(ws + L.fvar_off) : nullptr;
   // shaded jobs resolve in the deferred shade (from the per-face varyings when there are faces)
   const bool shading = b.total_pixels > 0 && (b.shader_mask != (1 << RAST_SHADER_DEPTH) || b.total_setup == 0);
@@ -1455,14 +1498,12 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
     bw.fmap = fmap;
     bw.fmap_blocks = b.total_setup > 0 ? L.fmap_blocks : 0u;
     bw.map_rows = setup_rows(L.small_path);
-    bw.vmap = reinterpret_cast<int2*>(ws + L.vmap_off);
-    bw.vmap_blocks = pre ? L.vmap_blocks : 0u;
     bw.zero[0] = counts;  // counts and cursors are adjacent
     bw.zero_bytes[0] = L.offsets_off - L.counts_off;
     bw.zero[1] = misc;
     bw.zero_bytes[1] = 256;
     bw.zero[2] = vis;
-    bw.zero_bytes[2] = vis ? static_cast<size_t>(b.total_setup) : 0;
+    bw.zero_bytes[2] = vis ? (static_cast<size_t>(b.total_setup) + 31) / 32 * 4 : 0;
     bw.keys = keys;
     bw.rects = reinterpret_cast<ScreenRect*>(ws + L.rect_off);
     bw.key_bytes = keys ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0;
@@ -1498,11 +1539,9 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
           launch_raster<false, false, RAST_MAX_LAYERS>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner,
                                                        misc, vis, nullptr);
         else if (b.near_ties)
-          launch_raster<false, true, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis,
-                                        nullptr);
+          launch_raster<false, true, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, nullptr);
         else
-          launch_raster<false, false, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis,
-                                         nullptr);
+          launch_raster<false, false, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, nullptr);
       } else {
         if (cudaMemsetAsync(winner, 0xff, static_cast<size_t>(b.total_pixels) * 4 * L.winner_layers, s) !=
             cudaSuccess)
@@ -1510,7 +1549,15 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
       }
       prof.mark("raster_kernel");
       if (pre) {
-        face_varyings_kernel<<<L.vmap_blocks, kFaceThreads, 0, s>>>(b, bw.vmap, vis, fvar, L.vstride);
+        // up to four warps per entry while all of them are resident at once
+        const unsigned split = std::min(4u, std::max(1u, static_cast<unsigned>(sms) * 48u / std::max(L.fmap_blocks, 1u)));
+        const unsigned vgrid = (L.fmap_blocks * split + kFaceThreads / 32 - 1) / (kFaceThreads / 32);
+        if (L.small_path)
+          face_varyings_kernel<setup_rows(true)><<<vgrid, kFaceThreads, 0, s>>>(b, fmap, L.fmap_blocks, split, vis, fvar,
+                                                                              L.vstride);
+        else
+          face_varyings_kernel<setup_rows(false)><<<vgrid, kFaceThreads, 0, s>>>(b, fmap, L.fmap_blocks, split, vis, fvar,
+                                                                              L.vstride);
         prof.mark("face_varyings_kernel");
       }
     }
