@@ -269,6 +269,21 @@ int rast_render_tiled(const RastBatch* batch, const RastTiledConfig* cfg, void* 
 int rast_render_tiled_phase(const RastBatch* batch, const RastTiledConfig* cfg, void* workspace,
                             size_t workspace_bytes, void* stream, int phase);
 
+/* rast_render_tiled_phase into buffers that take their defaults: the same
+ * outputs as when every zbuffer pixel of the batch held `depth` and every
+ * canvas pixel (when pools.canvas is set) the three floats at `colour`
+ * (device memory) before the call, without the caller's passes over both
+ * buffers: the kernels that store a pixel store its default where nothing is
+ * kept.  Both phases of one pass take the same RastClear.  `clear` NULL:
+ * RAST_ERR_INVALID_ARGUMENT, and so is a NULL colour with a canvas. */
+typedef struct RastClear {
+  const float* colour;   /* DEVICE, 3 floats (create_buffers' colour_default); unused without a canvas */
+  float depth;           /* create_buffers' zbuffer_default */
+  int32_t reserved;
+} RastClear;
+int rast_render_tiled_clear(const RastBatch* batch, const RastTiledConfig* cfg, const RastClear* clear, void* workspace,
+                            size_t workspace_bytes, void* stream, int phase);
+
 /* rast_render_tiled with per-kernel timing (synchronises `stream`). */
 int rast_render_tiled_profiled(const RastBatch* batch, const RastTiledConfig* cfg, void* workspace,
                                size_t workspace_bytes, void* stream, RastProfile* profile);

@@ -151,6 +151,10 @@ class RastTiledConfig(ctypes.Structure):
                 ("warps_per_tile", c_int32)]
 
 
+class RastClear(ctypes.Structure):
+    _fields_ = [("colour", c_void_p), ("depth", ctypes.c_float), ("reserved", c_int32)]
+
+
 class RastTiledStats(ctypes.Structure):
     _fields_ = [("bin_entries", c_uint64), ("bin_capacity", c_uint64), ("tiles", c_uint64),
                 ("overflow", ctypes.c_uint32), ("binned_faces", ctypes.c_uint32), ("pixel_tests", c_uint64)]
@@ -210,6 +214,8 @@ PROTOTYPES = [
     ("rast_autotune", c_int, [POINTER(RastBatch), c_void_p, POINTER(RastTiledConfig)]),
     ("rast_render_tiled_phase", c_int, [POINTER(RastBatch), POINTER(RastTiledConfig), c_void_p, c_size_t, c_void_p,
                                         c_int]),
+    ("rast_render_tiled_clear", c_int, [POINTER(RastBatch), POINTER(RastTiledConfig), POINTER(RastClear), c_void_p,
+                                        c_size_t, c_void_p, c_int]),
     ("rast_tiled_stats", c_int,
      [POINTER(RastBatch), POINTER(RastTiledConfig), c_void_p, c_void_p, POINTER(RastTiledStats)]),
     ("rast_backward_workspace_bytes", c_size_t, [POINTER(RastBatch)]),
@@ -280,6 +286,7 @@ __all__ = [
     "RastBatch",
     "RastProfile",
     "RastTiledConfig",
+    "RastClear",
     "RastTiledStats",
     "RastGradPools",
     "RastError",

@@ -505,11 +505,18 @@ class BatchRunner:
             return self.lib.rast_plain_workspace_bytes(ctypes.byref(b))
         return self.lib.rast_tiled_workspace_bytes(ctypes.byref(b), self._cfg(name))
 
-    def launch(self, name, stream_handle, profile=None, phase: int = 3) -> None:
+    def launch(self, name, stream_handle, profile=None, phase: int = 3, clear=None) -> None:
         """Render pass `name` on the stream; `phase` (tiled form) selects
-        rast_render_tiled_phase's coverage (1) or shade (2) half, 3 both."""
+        rast_render_tiled_phase's coverage (1) or shade (2) half, 3 both.
+        `clear` (a RastClear, tiled form): the pass's buffers take these
+        defaults instead of what they hold."""
         b = self.shadow_batch if name == "shadow" else self.main_batch
         buf, nbytes = self.ws[name]
+        if clear is not None:
+            st = self.lib.rast_render_tiled_clear(ctypes.byref(b), self._cfg(name), ctypes.byref(clear), buf.data_ptr(),
+                                                  nbytes, stream_handle, int(phase))
+            _lib.check(st, "rast_render_tiled_clear")
+            return
         if self.form == "tiled" and phase != 3 and profile is None:
             st = self.lib.rast_render_tiled_phase(ctypes.byref(b), self._cfg(name), buf.data_ptr(), nbytes,
                                                   stream_handle, int(phase))
@@ -665,23 +672,28 @@ class BatchRunner:
         capture records as two branches."""
         s = stream if stream is not None else torch.cuda.current_stream(self.sb.device)
         with torch.cuda.stream(s):
-            self._reset(zbuffer_default)
+            clear = {"shadow": None, "main": None}
+            if self.form == "tiled":  # the kernels store the defaults themselves
+                clear = {"shadow": _lib.RastClear(None, float(np.finfo(np.float32).max)),
+                         "main": _lib.RastClear(self._colour.data_ptr(), zbuffer_default)}
+            else:
+                self._reset(zbuffer_default)
             if self.form == "tiled" and self.shadow_batch is not None and self.overlap_passes:
                 side = self._side_stream()
                 side.wait_stream(s)
                 with torch.cuda.stream(side):
                     torch.cuda.nvtx.range_push("shadow pass")
-                    self.launch("shadow", side.cuda_stream)
+                    self.launch("shadow", side.cuda_stream, clear=clear["shadow"])
                     torch.cuda.nvtx.range_pop()
                 torch.cuda.nvtx.range_push("main pass")
-                self.launch("main", s.cuda_stream, phase=_lib.PHASE_COVERAGE)
+                self.launch("main", s.cuda_stream, phase=_lib.PHASE_COVERAGE, clear=clear["main"])
                 s.wait_stream(side)
-                self.launch("main", s.cuda_stream, phase=_lib.PHASE_SHADE)
+                self.launch("main", s.cuda_stream, phase=_lib.PHASE_SHADE, clear=clear["main"])
                 torch.cuda.nvtx.range_pop()
             else:
                 for name, _ in self.batches():
                     torch.cuda.nvtx.range_push(f"{name} pass")
-                    self.launch(name, s.cuda_stream)
+                    self.launch(name, s.cuda_stream, clear=clear[name])
                     torch.cuda.nvtx.range_pop()
         return self.outputs()
 

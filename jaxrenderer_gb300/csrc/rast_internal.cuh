@@ -507,20 +507,28 @@ __device__ __forceinline__ void insert_key(unsigned long long (&best)[L], unsign
   if (key < best[0]) best[0] = key;
 }
 
-// merge_buffers (pipeline.py:401-440): overwrite where kept, no depth test;
+// Defaults of a pass into cleared buffers (rast_render_tiled_clear), or off.
+struct Clear {
+  const float* colour = nullptr;
+  float depth = 0.0f;
+  bool on = false;
+};
+
+// merge_buffers (pipeline.py:401-440): overwrite where kept, no depth test
+// (with `clear`, the default where not kept, as if the buffer had held it);
 // then the shadow pass's offset (shadow.py:116) when the job asks for it.
 __device__ __forceinline__ void store_pixel(const RastJob& J, const RastPools& P, int64_t pix,
-                                            const PixelResult& r) {
+                                            const PixelResult& r, const Clear& clear = Clear()) {
   const bool offset = (J.flags & RAST_JOB_APPLY_DEPTH_OFFSET) != 0;
-  if (r.keep || offset) {
-    float zb = r.keep ? r.z : P.zbuffer[pix];
+  if (r.keep || offset || clear.on) {
+    float zb = r.keep ? r.z : clear.on ? clear.depth : P.zbuffer[pix];
     if (offset) zb = zb + J.depth_offset;
     P.zbuffer[pix] = zb;
   }
-  if (r.keep && J.shader != RAST_SHADER_DEPTH && P.canvas) {
-    P.canvas[pix * 3 + 0] = r.colour[0];
-    P.canvas[pix * 3 + 1] = r.colour[1];
-    P.canvas[pix * 3 + 2] = r.colour[2];
+  const bool coloured = r.keep && J.shader != RAST_SHADER_DEPTH;
+  if ((coloured || clear.on) && P.canvas) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) P.canvas[pix * 3 + k] = coloured ? r.colour[k] : __ldg(clear.colour + k);
   }
   if (P.prim_id) P.prim_id[pix] = r.prim;
 }

@@ -141,28 +141,29 @@ __device__ __forceinline__ void clip_push0(ClipStage& s, ClipStage& s1, ClipStag
 // The job's screen rectangle one pixel wider on every side, in NDC (pixels
 // -1 and W), computed once per job by begin_kernel.
 struct ScreenRect {
-  float xl, xh, yl, yh, X, Y;
-  float gx, gy;  // half a pixel in NDC (0: rounding could reach it, see off_screen)
-  int ok;  // finite, non-degenerate viewport
+  float xl, xh, yl, yh;
+  float gx, gy;  // half a pixel in NDC (0: rounding could reach it, see off_screen); gx < 0: no usable viewport
+  __device__ __forceinline__ float X() const { return fmaxf(fabsf(xl), fabsf(xh)); }
+  __device__ __forceinline__ float Y() const { return fmaxf(fabsf(yl), fabsf(yh)); }
+  __device__ __forceinline__ bool ok() const { return gx >= 0.0f; }  // finite, non-degenerate viewport
 };
 
 __device__ __forceinline__ ScreenRect screen_rect(const RastJob& J) {
   ScreenRect r{};
   const float sx = J.viewport[0], ox = J.viewport[3];
   const float sy = J.viewport[5], oy = J.viewport[7];
-  r.ok = (sx != 0.0f) && (sy != 0.0f) && isfinite(sx) && isfinite(sy);
+  const bool ok = (sx != 0.0f) && (sy != 0.0f) && isfinite(sx) && isfinite(sy);
   const float xa = (-1.0f - ox) / sx, xb = (static_cast<float>(J.width) - ox) / sx;
   const float ya = (-1.0f - oy) / sy, yb = (static_cast<float>(J.height) - oy) / sy;
   r.xl = fminf(xa, xb);
   r.xh = fmaxf(xa, xb);
   r.yl = fminf(ya, yb);
   r.yh = fmaxf(ya, yb);
-  r.X = fmaxf(fabsf(r.xl), fabsf(r.xh));
-  r.Y = fmaxf(fabsf(r.yl), fabsf(r.yh));
   r.gx = 0.5f / fabsf(sx);
   r.gy = 0.5f / fabsf(sy);
-  if (!(r.X * 4.8e-7f < r.gx)) r.gx = 0.0f;  // 8 u X
-  if (!(r.Y * 4.8e-7f < r.gy)) r.gy = 0.0f;
+  if (!(r.X() * 4.8e-7f < r.gx)) r.gx = 0.0f;  // 8 u X
+  if (!(r.Y() * 4.8e-7f < r.gy)) r.gy = 0.0f;
+  if (!ok) r.gx = -1.0f;
   return r;
 }
 
@@ -207,14 +208,14 @@ __device__ __forceinline__ bool off_screen(const float* m, float det, const Scre
   side(-1.0f, x0, x1, x2, R.xl, R.gx);
   side(1.0f, y0, y1, y2, R.yh, R.gy);
   side(-1.0f, y0, y1, y2, R.yl, R.gy);
-  if (!(l0 > 0.0f) || !R.ok) return false;
+  if (!(l0 > 0.0f) || !R.ok()) return false;
   const float xmin = fminf(x0, fminf(x1, x2)), xmax = fmaxf(x0, fmaxf(x1, x2));
   const float ymin = fminf(y0, fminf(y1, y2)), ymax = fmaxf(y0, fmaxf(y1, y2));
   const float Mx = fmaxf(xmax, -xmin), My = fmaxf(ymax, -ymin), Mw = fmaxf(wmax, -wmin);
   const float Dx = xmax - xmin, Dy = ymax - ymin, Dw = wmax - wmin;
   const float Cx = __fmaf_rn(My, Dw, Mw * Dy), Cy = __fmaf_rn(Mx, Dw, Mw * Dx), Cw = __fmaf_rn(Mx, Dy, My * Dx);
   const float S = __fmaf_rn(Mx, Cx, __fmaf_rn(My, Cy, Mw * Cw));
-  const float T = __fmaf_rn(R.X, Cx, __fmaf_rn(R.Y, Cy, Cw));
+  const float T = __fmaf_rn(R.X(), Cx, __fmaf_rn(R.Y(), Cy, Cw));
   const float d = det - 48.0f * 5.9604645e-08f * (Mx * My * Mw);  // the determinant's own rounding: 42 u MxMyMw
   const float eS = 85.0f * 5.9604645e-08f * S;
   return fmaxf(Mx, fmaxf(My, Mw)) <= 1073741824.0f && 20.0f * eS <= d && 5.0f * eS * l1 <= l0 * d &&
@@ -263,10 +264,10 @@ __device__ __forceinline__ bool coverage_bbox(const float* inv, const RastJob& J
   const int W = J.width, H = J.height;
   const float sx = J.viewport[0], ox = J.viewport[3];
   const float sy = J.viewport[5], oy = J.viewport[7];
-  const float xl = R.xl, xh = R.xh, yl = R.yl, yh = R.yh, X = R.X, Y = R.Y;
+  const float xl = R.xl, xh = R.xh, yl = R.yl, yh = R.yh, X = R.X(), Y = R.Y();
   // edge k: a_k x + b_k y + (c_k + eps_k), kept in scalars (no arrays: the
   // clip stages below capture them)
-  bool small = R.ok;  // |c_k| < 1e37 on the rectangle: no overflow below (NaN and infinite entries fail)
+  bool small = R.ok();  // |c_k| < 1e37 on the rectangle: no overflow below (NaN and infinite entries fail)
   auto widened = [&](float a, float b, float c) {
     const float bound = X * fabsf(a) + Y * fabsf(b) + fabsf(c);
     small = small && bound < 1e37f;
@@ -640,9 +641,10 @@ __global__ void __launch_bounds__(256) begin_kernel(RastBatch B, BeginWork w) {
   for (int k = 0; k < 3; ++k) fill_words(w.zero[k], w.zero_bytes[k], 0u);
   fill_words(w.keys, w.key_bytes, 0xffffffffu);
   fill_block_map<kMapFaces>(B.jobs, B.n_jobs, w.map_rows, w.fmap, w.fmap_blocks);
-  for (int j = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); j < B.n_jobs;
-       j += static_cast<int>(gridDim.x * blockDim.x))
-    w.rects[j] = screen_rect(B.jobs[j]);
+  if (w.fmap_blocks > 0)
+    for (int j = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); j < B.n_jobs;
+         j += static_cast<int>(gridDim.x * blockDim.x))
+      w.rects[j] = screen_rect(B.jobs[j]);
 }
 
 // Bin offsets: a tile only needs a contiguous range of the bins, in no
@@ -809,7 +811,7 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
               const uint32_t* __restrict__ counts, const uint32_t* __restrict__ offsets,
               const int32_t* __restrict__ bins, int32_t* __restrict__ winner,
               unsigned int* __restrict__ work, int64_t n_units, uint32_t* __restrict__ visible,
-              const unsigned long long* __restrict__ keys) {
+              const unsigned long long* __restrict__ keys, Clear clear) {
   constexpr int PPL = TW * TH / 32;
   constexpr bool kPairs = kL == 1 && !kTies;
   constexpr int kPW = kPairs ? kRasterWarps : 1;  // pair-path arrays only where used
@@ -1152,7 +1154,7 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
         r.z = z;
         r.prim = keep ? prim : -1;
         r.colour[0] = r.colour[1] = r.colour[2] = 0.0f;
-        store_pixel(J, B.pools, pix, r);
+        store_pixel(J, B.pools, pix, r, clear);
       }
     }
   }
@@ -1250,7 +1252,7 @@ face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entrie
 template <bool kLayered>
 __global__ void __launch_bounds__(256, kLayered ? 4 : 8)
 tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t* __restrict__ winner,
-                   bool depth_resolved, const float* __restrict__ fvar, int vstride) {
+                   bool depth_resolved, const float* __restrict__ fvar, int vstride, Clear clear) {
   __shared__ RastJob sJ;
   __shared__ WarpFrags s_frags[kLayered ? 8 : 1];  // per warp, layered "over" jobs
   const int jid = blockIdx.y;
@@ -1273,7 +1275,7 @@ tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t*
     resolve_over_warp(J, B.pools, rec, active, i, j, winner + (active ? pix : 0), B.total_pixels, L, src,
                       s_frags[threadIdx.x >> 5], &r);
     if (active) {
-      store_pixel(J, B.pools, pix, r);
+      store_pixel(J, B.pools, pix, r, clear);
       save_layers(B.pools, winner + pix, B.total_pixels, pix, L);
     }
     return;
@@ -1288,13 +1290,13 @@ tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t*
     r.keep = false;
     r.prim = -1;
     r.z = 0.0f;
-    store_pixel(J, B.pools, pix, r);
+    store_pixel(J, B.pools, pix, r, clear);
     return;
   }
   resolve_pixel(J, B.pools, rec, i, j, w0, src, &r);  // the winner, or the layered chooser's slot 0
   if (kLayered && L > 1 && !r.keep)  // slot 0 discarded by its fragment shader: the next kept slot
     resolve_layers(J, B.pools, rec, i, j, winner + pix, B.total_pixels, L, src, &r, 1);
-  store_pixel(J, B.pools, pix, r);
+  store_pixel(J, B.pools, pix, r, clear);
 }
 
 // ------------------------------------------------------------------ layout
@@ -1358,7 +1360,7 @@ static Layout layout(const RastBatch& b, TileShape ts, uint64_t bin_capacity, in
   L.fmap_blocks = block_map_capacity(b.total_setup, b.n_jobs, setup_rows(L.small_path));
   L.fmap_off = take(static_cast<size_t>(L.fmap_blocks) * sizeof(int2));
   L.keys_off = take(L.small_path ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0);
-  L.rect_off = take(static_cast<size_t>(b.n_jobs) * sizeof(ScreenRect));
+  L.rect_off = take(b.total_setup > 0 ? static_cast<size_t>(b.n_jobs) * sizeof(ScreenRect) : 0);
   L.misc_off = take(256);
   L.total = off;
   return L;
@@ -1411,7 +1413,8 @@ template <bool kKeys, bool kTies, int kL>
 // tiles x warps per tile).
 static void launch_raster(TileShape ts, int wpt, int sms, cudaStream_t s, const RastBatch& b, const Layout& L,
                           const float4* setup, const unsigned char* flag, const uint32_t* counts, const uint32_t* offsets, const int32_t* bins,
-                          int32_t* winner, unsigned int* misc, uint32_t* vis, const unsigned long long* keys) {
+                          int32_t* winner, unsigned int* misc, uint32_t* vis, const unsigned long long* keys,
+                          const Clear& clear) {
   const unsigned block = 32 * kRasterWarps;
   auto go = [&](auto kernel) {
     int per_sm = 0;
@@ -1420,7 +1423,7 @@ static void launch_raster(TileShape ts, int wpt, int sms, cudaStream_t s, const 
       per_sm = 8;
     const unsigned grid = static_cast<unsigned>(std::max(sms, 1) * per_sm);
     kernel<<<grid, block, 0, s>>>(b, L.G, setup, flag, counts, offsets, bins, winner, misc, L.n_tiles * wpt, vis,
-                                  keys);
+                                  keys, clear);
   };
   if (wpt == 2) {  // the warp's sub-tile is (tw, th / 2)
     if (ts.tw == 8 && ts.th == 16)
@@ -1451,7 +1454,7 @@ static void launch_raster(TileShape ts, int wpt, int sms, cudaStream_t s, const 
 
 static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* workspace,
                   size_t workspace_bytes, void* stream, RastProfile* profile,
-                  int phase = RAST_PHASE_COVERAGE | RAST_PHASE_SHADE) {
+                  int phase = RAST_PHASE_COVERAGE | RAST_PHASE_SHADE, const Clear& clear = Clear()) {
   int st = check_batch(batch);
   if (st != RAST_OK) return st;
   if (phase < 1 || phase > (RAST_PHASE_COVERAGE | RAST_PHASE_SHADE)) return RAST_ERR_INVALID_ARGUMENT;
@@ -1531,17 +1534,17 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
         // the key path exists only when ties are not counted and no job is
         // layered
         if (keys)
-          launch_raster<true, false, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, keys);
+          launch_raster<true, false, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, keys, clear);
         else if (b.max_layers > 0 && b.near_ties)
           launch_raster<false, true, RAST_MAX_LAYERS>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner,
-                                                      misc, vis, nullptr);
+                                                      misc, vis, nullptr, clear);
         else if (b.max_layers > 0)
           launch_raster<false, false, RAST_MAX_LAYERS>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner,
-                                                       misc, vis, nullptr);
+                                                       misc, vis, nullptr, clear);
         else if (b.near_ties)
-          launch_raster<false, true, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, nullptr);
+          launch_raster<false, true, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, nullptr, clear);
         else
-          launch_raster<false, false, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, nullptr);
+          launch_raster<false, false, 1>(ts, wpt, sms, s, b, L, setup, flag, counts, offsets, bins, winner, misc, vis, nullptr, clear);
       } else {
         if (cudaMemsetAsync(winner, 0xff, static_cast<size_t>(b.total_pixels) * 4 * L.winner_layers, s) !=
             cudaSuccess)
@@ -1567,9 +1570,9 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
     const dim3 sgrid(static_cast<unsigned>((max_px + 255) / 256), static_cast<unsigned>(b.n_jobs));
     const float* fv = pre ? fvar : nullptr;
     if (b.max_layers > 0)
-      tiled_shade_kernel<true><<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, fv, L.vstride);
+      tiled_shade_kernel<true><<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, fv, L.vstride, clear);
     else
-      tiled_shade_kernel<false><<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, fv, L.vstride);
+      tiled_shade_kernel<false><<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, fv, L.vstride, clear);
     prof.mark("tiled_shade_kernel");
   }
   const cudaError_t e = cudaGetLastError();
@@ -1621,6 +1624,13 @@ extern "C" int rast_render_tiled(const RastBatch* batch, const RastTiledConfig* 
 extern "C" int rast_render_tiled_phase(const RastBatch* batch, const RastTiledConfig* cfg, void* workspace,
                                        size_t workspace_bytes, void* stream, int phase) {
   return tiled::render(batch, cfg, workspace, workspace_bytes, stream, nullptr, phase);
+}
+
+extern "C" int rast_render_tiled_clear(const RastBatch* batch, const RastTiledConfig* cfg, const RastClear* clear,
+                                       void* workspace, size_t workspace_bytes, void* stream, int phase) {
+  if (!batch || !clear || (batch->pools.canvas && !clear->colour)) return RAST_ERR_INVALID_ARGUMENT;
+  return tiled::render(batch, cfg, workspace, workspace_bytes, stream, nullptr, phase,
+                       Clear{clear->colour, clear->depth, true});
 }
 
 extern "C" int rast_render_tiled_profiled(const RastBatch* batch, const RastTiledConfig* cfg,
