@@ -501,6 +501,25 @@ int rast_merge_objects(const RastMergeBatch* batch, void* workspace, size_t work
 int rast_display_u8(const float* canvas, int64_t n_images, int32_t width, int32_t height, int32_t channels,
                     int32_t flip_vertical, uint8_t* out, void* stream);
 
+/* Camera matrices of n cameras from their eyes (Renderer.create_camera_from_
+ * parameters, renderer.py:141-196): view = lookAt(eye, centre, up),
+ * world_to_clip = projection * view, world_to_eye_norm = the transposed
+ * inverse of view.  eye / centre / up: device rows of 3 floats, *_stride
+ * floats apart (0: one row for every camera); projection (16) and the
+ * outputs (n, 16) device, row-major.  Stream-ordered. */
+int rast_camera_matrices(int32_t n, const float* eye, int64_t eye_stride, const float* centre, int64_t centre_stride,
+                         const float* up, int64_t up_stride, const float* projection, float* world_to_clip,
+                         float* world_to_eye_norm, float* view, void* stream);
+
+/* Reverse mode of rast_camera_matrices: gradients of the three outputs (16
+ * floats per camera, *_stride floats apart; NULL: zero) -> dL/d eye, centre
+ * and up per camera ((n, 3), written; NULL: skipped). */
+int rast_camera_matrices_backward(int32_t n, const float* eye, int64_t eye_stride, const float* centre,
+                                  int64_t centre_stride, const float* up, int64_t up_stride, const float* projection,
+                                  const float* grad_world_to_clip, int64_t w2c_stride, const float* grad_world_to_eye_norm,
+                                  int64_t w2e_stride, const float* grad_view, int64_t view_stride, float* grad_eye,
+                                  float* grad_centre, float* grad_up, void* stream);
+
 /* Host-side validation of one job against pool sizes (no device access):
  * returns RAST_ERR_INVALID_ARGUMENT for inconsistent sizes. */
 int rast_validate_job(const RastJob* job);

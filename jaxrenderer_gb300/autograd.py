@@ -103,15 +103,80 @@ def camera_matrices(eye: torch.Tensor, params, target=None, up=None) -> Tuple[to
     target = vec(target, params.target)
     up = vec(up, params.up)
     target = target.expand_as(eye)
-    v = view_matrix(eye, target, up)
-    vinv = view_matrix_inv(eye, target, up)
     aspect = np.tan(np.radians(params.hfov) / 2.0) / np.tan(np.radians(params.vfov) / 2.0)
     key = (float(params.vfov), float(aspect), float(params.near), float(params.far), dt, dev)
     p = _PROJECTIONS.get(key)
     if p is None:  # built once per camera and device: later calls copy nothing from the host
         p = perspective_projection_matrix(params.vfov, aspect, params.near, params.far, dtype=dt, device=dev)
         _PROJECTIONS[key] = p
-    return p @ v, vinv.transpose(-1, -2), v
+    if _native_cameras(eye, target, up):
+        return _CameraFunction.apply(eye, target, up.expand_as(eye), p)
+    return _camera_tensors(eye, target, up, p)
+
+
+def _camera_tensors(eye, target, up, projection):
+    """The same as tensor operations: any dtype, device, shape or transform."""
+    v = view_matrix(eye, target, up)
+    return projection @ v, view_matrix_inv(eye, target, up).transpose(-1, -2), v
+
+
+def _native_cameras(*tensors) -> bool:
+    """Whether the kernels take these: float32 rows of one GPU, with nothing
+    watching the operations (functorch transforms, forward-mode duals, tracing,
+    autocast, dispatch modes and tensor subclasses see the tensor operations)."""
+    eye = tensors[0]
+    return (eye.dim() == 2 and eye.shape[0] > 0 and eye.shape[1] == 3
+            and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.float32
+                    and t.device == eye.device and t.shape[-1] == 3 and t.stride(-1) == 1 for t in tensors)
+            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
+            and torch._C._len_torch_dispatch_stack() == 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
+            and not torch.is_autocast_enabled())
+
+
+class _CameraFunction(torch.autograd.Function):
+    """camera_matrices as one kernel per direction (rast_camera_matrices)."""
+
+    @staticmethod
+    def forward(ctx, eye, target, up, projection):
+        n = eye.shape[0]
+        w2c, w2e, view = (torch.empty((n, 4, 4), dtype=eye.dtype, device=eye.device) for _ in range(3))
+        with torch.cuda.device(eye.device):
+            s = torch.cuda.current_stream(eye.device).cuda_stream
+            _lib.check(_lib.load().rast_camera_matrices(n, *_rows(eye), *_rows(target), *_rows(up), projection.data_ptr(),
+                                                        w2c.data_ptr(), w2e.data_ptr(), view.data_ptr(), s),
+                       "rast_camera_matrices")
+        ctx.save_for_backward(eye, target, up, projection)
+        ctx.set_materialize_grads(False)
+        return w2c, w2e, view
+
+    @staticmethod
+    def backward(ctx, *grads):
+        eye, target, up, projection = ctx.saved_tensors
+        wanted = ctx.needs_input_grad[:3]
+        if torch.is_grad_enabled():  # create_graph: gradients of gradients follow the tensor operations
+            inputs = [t for t, w in zip((eye, target, up), wanted) if w]
+            outs, gs = zip(*((o, g) for o, g in zip(_camera_tensors(eye, target, up, projection), grads) if g is not None))
+            got = iter(torch.autograd.grad(outs, inputs, gs, create_graph=True, allow_unused=True))
+            return (*(next(got) if w else None for w in wanted), None)
+        n = eye.shape[0]
+        mats = [_mats(g) for g in grads]
+        out = [torch.empty((n, 3), dtype=eye.dtype, device=eye.device) if w else None for w in wanted]
+        with torch.cuda.device(eye.device):
+            s = torch.cuda.current_stream(eye.device).cuda_stream
+            _lib.check(_lib.load().rast_camera_matrices_backward(
+                n, *_rows(eye), *_rows(target), *_rows(up), projection.data_ptr(),
+                *(x for g in mats for x in ((g.data_ptr(), g.stride(0)) if g is not None else (None, 0))),
+                *(t.data_ptr() if t is not None else None for t in out), s), "rast_camera_matrices_backward")
+        return (*out, None)
+
+
+def _rows(t: torch.Tensor):
+    return t.data_ptr(), t.stride(0)
+
+
+def _mats(g):
+    """A gradient of (N, 4, 4) matrices with each matrix contiguous."""
+    return g if g is None or g.stride()[1:] == (4, 1) else g.contiguous()
 
 
 _PROJECTIONS: dict = {}
