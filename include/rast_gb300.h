@@ -520,6 +520,11 @@ int rast_camera_matrices_backward(int32_t n, const float* eye, int64_t eye_strid
                                   int64_t w2e_stride, const float* grad_view, int64_t view_stride, float* grad_eye,
                                   float* grad_centre, float* grad_up, void* stream);
 
+/* jnp.linalg.inv of n row-major 4x4 matrices on the host (no device access):
+ * the LU inverse rast_merge_objects runs per instance, bit for bit.  `out`
+ * must not overlap `matrices`. */
+int rast_lu_inverse4(const float* matrices, int64_t n, float* out);
+
 /* Host-side validation of one job against pool sizes (no device access):
  * returns RAST_ERR_INVALID_ARGUMENT for inconsistent sizes. */
 int rast_validate_job(const RastJob* job);

@@ -232,6 +232,7 @@ PROTOTYPES = [
     ("rast_camera_matrices", c_int, [c_int32] + [c_void_p, c_int64] * 3 + [c_void_p] * 5),
     ("rast_camera_matrices_backward", c_int, [c_int32] + [c_void_p, c_int64] * 3 + [c_void_p] + [c_void_p, c_int64] * 3
      + [c_void_p] * 4),
+    ("rast_lu_inverse4", c_int, [c_void_p, c_int64, c_void_p]),
     ("rast_validate_job", c_int, [POINTER(RastJob)]),
     ("rast_error_string", ctypes.c_char_p, [c_int]),
     ("rast_abi_version", c_int, []),
@@ -246,6 +247,11 @@ class RastError(RuntimeError):
     def __init__(self, status: int, where: str):
         self.status = status
         super().__init__(f"{where}: {STATUS_NAMES.get(status, status)}")
+
+
+def loaded():
+    """The library if this process has loaded it, else None (never builds)."""
+    return _LIB
 
 
 def library_path() -> Path:

@@ -31,23 +31,34 @@ TWO_WARP_SHAPES = ((8, 8), (8, 16), (16, 16))  # two warps per tile, half of the
 LAYERED_SHAPES = ((8, 8), (16, 8), (8, 4), (4, 8))  # one-warp shapes with a layered-chooser raster variant
 SMALL_AREAS = (0, 32)  # small-face rasterisation in the setup kernel: off, or rectangles up to 32 pixels
 _LOCK = threading.Lock()
+_DEFAULT_PATH = Path(__file__).resolve().parent / "_build" / "autotune.json"
 
 
 def cache_path() -> Path:
     env = os.environ.get("JAXRENDERER_GB300_AUTOTUNE")
-    if env:
-        return Path(env)
-    return Path(__file__).resolve().parent / "_build" / "autotune.json"
+    return Path(env) if env else _DEFAULT_PATH
+
+
+# The file as last read: (path, modification time, size) and its entries.
+_READ: tuple = (None, {})
 
 
 def _load() -> dict:
+    """The file's entries (the caller holds _LOCK and does not change them),
+    read again when the file has changed."""
+    global _READ
     p = cache_path()
-    if p.exists():
+    try:
+        st = os.stat(p)
+    except OSError:
+        return {}
+    mark = (str(p), st.st_mtime_ns, st.st_size, st.st_ino)
+    if _READ[0] != mark:
         try:
-            return json.loads(p.read_text())
+            _READ = (mark, json.loads(p.read_text()))
         except (OSError, ValueError):
             return {}
-    return {}
+    return _READ[1]
 
 
 def _store(d: dict) -> None:
@@ -74,29 +85,38 @@ def tiled_config_for(runner, name: str, b, jobs: np.ndarray) -> "_lib.RastTiledC
     return tiled_config_for_batch(runner.sb.device, b, jobs)
 
 
+def known_config(device: torch.device, b, jobs: np.ndarray):
+    """The RastTiledConfig the file holds for this pass's workload class, or
+    None.  Renders nothing."""
+    key = workload_key(jobs, device)
+    with _LOCK:
+        hit = _load().get(key)
+    if hit is None:
+        return None
+    return _lib.RastTiledConfig(int(hit["tile_w"]), int(hit["tile_h"]), int(hit["bin_capacity"]),
+                                int(hit.get("small_area", 0)), int(hit.get("warps_per_tile", 1)))
+
+
 def tiled_config_for_batch(device: torch.device, b, jobs: np.ndarray) -> "_lib.RastTiledConfig":
     """Tuned RastTiledConfig for a RastBatch `b` whose job table is `jobs`
     (structured array with the RastJob layout).  Tuning renders `b` several
     times into its own output pools: pass a batch whose outputs may be
     overwritten."""
+    cfg = known_config(device, b, jobs)
+    if cfg is not None:
+        return cfg
     key = workload_key(jobs, device)
-    with _LOCK:
-        cache = _load()
-        hit = cache.get(key)
-    if hit is not None:
-        return _lib.RastTiledConfig(int(hit["tile_w"]), int(hit["tile_h"]), int(hit["bin_capacity"]),
-                                    int(hit.get("small_area", 0)), int(hit.get("warps_per_tile", 1)))
     cfg = _lib.RastTiledConfig()
     with torch.cuda.device(device):
         s = torch.cuda.current_stream(device)
         _lib.check(_lib.load().rast_autotune(ctypes.byref(b), s.cuda_stream, ctypes.byref(cfg)), "rast_autotune")
     with _LOCK:
-        cache = _load()
+        cache = dict(_load())
         cache[key] = {"tile_w": cfg.tile_w, "tile_h": cfg.tile_h, "bin_capacity": int(cfg.bin_capacity),
                       "small_area": cfg.small_area, "warps_per_tile": cfg.warps_per_tile}
         _store(cache)
     return cfg
 
 
-__all__ = ["tiled_config_for", "tiled_config_for_batch", "workload_key", "cache_path", "SHAPES", "TWO_WARP_SHAPES",
+__all__ = ["tiled_config_for", "tiled_config_for_batch", "known_config", "workload_key", "cache_path", "SHAPES", "TWO_WARP_SHAPES",
            "LAYERED_SHAPES", "SMALL_AREAS"]

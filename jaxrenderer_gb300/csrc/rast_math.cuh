@@ -172,6 +172,91 @@ __device__ __forceinline__ void inv3(const float* m, float* out) {
   }
 }
 
+// jnp.linalg.inv of one N x N matrix: LU with partial pivoting (first index
+// of the largest |a|, no swap for a zero pivot column), reciprocal scaling
+// for normal pivots, then the two triangular solves per column of the
+// permuted identity, skipping zero right-hand sides -- the same sequence as
+// geometry.lu_inverse on the host.
+template <int N>
+__host__ __device__ __forceinline__ void inv_lu(const float* m, float* out) {
+  float a[N * N];
+#pragma unroll
+  for (int k = 0; k < N * N; ++k) a[k] = m[k];
+  int perm[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) perm[k] = k;
+#pragma unroll
+  for (int j = 0; j < N - 1; ++j) {
+    int p = j;
+    float best = fabsf(a[N * j + j]);
+#pragma unroll
+    for (int r = j + 1; r < N; ++r) {
+      const float v = fabsf(a[N * r + j]);
+      if (v > best) {
+        best = v;
+        p = r;
+      }
+    }
+    // pivot value after the (conditional) swap, selected without dynamic indexing
+    float pv = a[N * j + j];
+#pragma unroll
+    for (int r = j + 1; r < N; ++r)
+      if (p == r) pv = a[N * r + j];
+    const bool nz = pv != 0.0f;
+    if (nz && p != j) {
+#pragma unroll
+      for (int r = j + 1; r < N; ++r) {
+        if (p == r) {
+#pragma unroll
+          for (int c = 0; c < N; ++c) {
+            const float t = a[N * j + c];
+            a[N * j + c] = a[N * r + c];
+            a[N * r + c] = t;
+          }
+          const int t = perm[j];
+          perm[j] = perm[r];
+          perm[r] = t;
+        }
+      }
+    }
+    const float piv = a[N * j + j];
+    if (nz) {
+      if (fabsf(piv) >= 1.17549435e-38f) {
+        const float rcp = 1.0f / piv;
+#pragma unroll
+        for (int r = j + 1; r < N; ++r) a[N * r + j] = a[N * r + j] * rcp;
+      } else {
+#pragma unroll
+        for (int r = j + 1; r < N; ++r) a[N * r + j] = a[N * r + j] / piv;
+      }
+    }
+#pragma unroll
+    for (int r = j + 1; r < N; ++r)
+#pragma unroll
+      for (int c = j + 1; c < N; ++c) a[N * r + c] = a[N * r + c] - a[N * r + j] * a[N * j + c];
+  }
+#pragma unroll
+  for (int col = 0; col < N; ++col) {
+    float b[N];
+#pragma unroll
+    for (int r = 0; r < N; ++r) b[r] = (perm[r] == col) ? 1.0f : 0.0f;
+#pragma unroll
+    for (int k = 0; k < N; ++k)
+      if (b[k] != 0.0f)
+#pragma unroll
+        for (int i = k + 1; i < N; ++i) b[i] = b[i] - b[k] * a[N * i + k];
+#pragma unroll
+    for (int k = N - 1; k >= 0; --k)
+      if (b[k] != 0.0f) {
+        b[k] = b[k] / a[N * k + k];
+#pragma unroll
+        for (int i = 0; i < k; ++i) b[i] = b[i] - b[k] * a[N * i + k];
+      }
+#pragma unroll
+    for (int r = 0; r < N; ++r) out[N * r + col] = b[r];
+  }
+}
+
 // min that propagates NaN (PTX min.NaN): min_nan(a, min_nan(b, c)) >= 0 is
 // exactly (a >= 0 && b >= 0 && c >= 0), NaN failing as in the reference.
 __device__ __forceinline__ float min_nan(float a, float b) {

@@ -25,91 +25,6 @@ namespace merge {
 
 constexpr int kThreads = 256;
 
-// jnp.linalg.inv of one N x N matrix: LU with partial pivoting (first index
-// of the largest |a|, no swap for a zero pivot column), reciprocal scaling
-// for normal pivots, then the two triangular solves per column of the
-// permuted identity, skipping zero right-hand sides -- the same sequence as
-// geometry.lu_inverse on the host.
-template <int N>
-__device__ __forceinline__ void inv_lu(const float* m, float* out) {
-  float a[N * N];
-#pragma unroll
-  for (int k = 0; k < N * N; ++k) a[k] = m[k];
-  int perm[N];
-#pragma unroll
-  for (int k = 0; k < N; ++k) perm[k] = k;
-#pragma unroll
-  for (int j = 0; j < N - 1; ++j) {
-    int p = j;
-    float best = fabsf(a[N * j + j]);
-#pragma unroll
-    for (int r = j + 1; r < N; ++r) {
-      const float v = fabsf(a[N * r + j]);
-      if (v > best) {
-        best = v;
-        p = r;
-      }
-    }
-    // pivot value after the (conditional) swap, selected without dynamic indexing
-    float pv = a[N * j + j];
-#pragma unroll
-    for (int r = j + 1; r < N; ++r)
-      if (p == r) pv = a[N * r + j];
-    const bool nz = pv != 0.0f;
-    if (nz && p != j) {
-#pragma unroll
-      for (int r = j + 1; r < N; ++r) {
-        if (p == r) {
-#pragma unroll
-          for (int c = 0; c < N; ++c) {
-            const float t = a[N * j + c];
-            a[N * j + c] = a[N * r + c];
-            a[N * r + c] = t;
-          }
-          const int t = perm[j];
-          perm[j] = perm[r];
-          perm[r] = t;
-        }
-      }
-    }
-    const float piv = a[N * j + j];
-    if (nz) {
-      if (fabsf(piv) >= 1.17549435e-38f) {
-        const float rcp = 1.0f / piv;
-#pragma unroll
-        for (int r = j + 1; r < N; ++r) a[N * r + j] = a[N * r + j] * rcp;
-      } else {
-#pragma unroll
-        for (int r = j + 1; r < N; ++r) a[N * r + j] = a[N * r + j] / piv;
-      }
-    }
-#pragma unroll
-    for (int r = j + 1; r < N; ++r)
-#pragma unroll
-      for (int c = j + 1; c < N; ++c) a[N * r + c] = a[N * r + c] - a[N * r + j] * a[N * j + c];
-  }
-#pragma unroll
-  for (int col = 0; col < N; ++col) {
-    float b[N];
-#pragma unroll
-    for (int r = 0; r < N; ++r) b[r] = (perm[r] == col) ? 1.0f : 0.0f;
-#pragma unroll
-    for (int k = 0; k < N; ++k)
-      if (b[k] != 0.0f)
-#pragma unroll
-        for (int i = k + 1; i < N; ++i) b[i] = b[i] - b[k] * a[N * i + k];
-#pragma unroll
-    for (int k = N - 1; k >= 0; --k)
-      if (b[k] != 0.0f) {
-        b[k] = b[k] / a[N * k + k];
-#pragma unroll
-        for (int i = 0; i < k; ++i) b[i] = b[i] - b[k] * a[N * i + k];
-      }
-#pragma unroll
-    for (int r = 0; r < N; ++r) out[N * r + col] = b[r];
-  }
-}
-
 // gather index semantics of jnp indexing: negative wraps once, then clamp
 __device__ __forceinline__ int wrap_clamp(int i, int n) {
   if (i < 0) i += n;
@@ -387,4 +302,13 @@ extern "C" int rast_merge_objects(const RastMergeBatch* batch, void* workspace, 
                                   void* stream) {
   rast::NvtxRange range("rast_merge_objects");
   return merge::run(batch, workspace, workspace_bytes, stream);
+}
+
+// Host inverse of n matrices: the same function as the instances' inverse,
+// compiled for the host (without contraction: _build.py), for the set-up code
+// that calls it a few matrices at a time (20 us a matrix as NumPy operations).
+extern "C" int rast_lu_inverse4(const float* matrices, int64_t n, float* out) {
+  if (n < 0 || (n > 0 && (!matrices || !out))) return RAST_ERR_INVALID_ARGUMENT;
+  for (int64_t k = 0; k < n; ++k) inv_lu<4>(matrices + 16 * k, out + 16 * k);
+  return RAST_OK;
 }

@@ -27,6 +27,7 @@ FORMS = ("auto", "plain", "tiled")
 TILED_MIN_PAIRS = 1 << 27
 # the tiled form's per-face pixel rectangles are 16-bit
 TILED_MAX_SIDE = 65535
+JOB_DTYPE = np.dtype(_lib.RastJob)
 _state = threading.local()
 
 
@@ -59,15 +60,19 @@ def choose(packed: _jobs.PackedBatch, form: Optional[str] = None) -> str:
 
 def job_array(packed: _jobs.PackedBatch) -> np.ndarray:
     """The batch's job table as a structured array with the RastJob layout."""
-    return np.frombuffer(bytes(packed.jobs), dtype=np.dtype(_lib.RastJob)).copy()
+    return np.frombuffer(bytes(packed.jobs), dtype=JOB_DTYPE).copy()
 
 
 def tuned_config(packed: _jobs.PackedBatch) -> "_lib.RastTiledConfig":
     """The autotuner's RastTiledConfig for this pass (cached per workload
     class).  When it has to time candidates it renders into scratch copies of
     the outputs, so the caller's buffers see one render only."""
-    from .autotune import tiled_config_for_batch
+    from .autotune import known_config, tiled_config_for_batch
 
+    jobs = job_array(packed)
+    cfg = known_config(packed.zbuffer.device, packed.batch, jobs)
+    if cfg is not None:
+        return cfg
     b = _lib.RastBatch.from_buffer_copy(packed.batch)
     scratch = []
 
@@ -82,7 +87,7 @@ def tuned_config(packed: _jobs.PackedBatch) -> "_lib.RastTiledConfig":
     alias("prim_id", packed.prim_id)
     alias("layer_prim", packed.layer_prim)
     b.near_ties = None
-    cfg = tiled_config_for_batch(packed.zbuffer.device, b, job_array(packed))
+    cfg = tiled_config_for_batch(packed.zbuffer.device, b, jobs)
     del scratch
     return cfg
 

@@ -24,7 +24,7 @@ def _arr(x, dtype=None) -> np.ndarray:
     a = np.asarray(x)
     if dtype is not None:
         a = a.astype(dtype, copy=False)
-    elif not np.issubdtype(a.dtype, np.floating):
+    elif a.dtype.kind != "f":
         a = a.astype(F32)
     return a
 
@@ -47,9 +47,11 @@ def matvec(m: np.ndarray, v: np.ndarray) -> np.ndarray:
     m = np.asarray(m)
     v = np.asarray(v)
     dt = np.result_type(m, v)
-    acc = v[..., 0:1].astype(dt) * m[:, 0].astype(dt)
+    m = m.astype(dt, copy=False)
+    v = v.astype(dt, copy=False)
+    acc = v[..., 0:1] * m[:, 0]
     for k in range(1, v.shape[-1]):
-        acc = acc + v[..., k : k + 1].astype(dt) * m[:, k].astype(dt)
+        acc = acc + v[..., k : k + 1] * m[:, k]
     return acc
 
 
@@ -139,8 +141,20 @@ def cross(a, b) -> np.ndarray:
 def lu_inverse(m) -> np.ndarray:
     """jnp.linalg.inv of a batch of n x n matrices: LU with partial pivoting
     (reference LAPACK getf2 order) and two triangular solves (reference BLAS
-    trsm order), vectorised over the leading axes."""
-    a = _arr(m).copy()
+    trsm order), vectorised over the leading axes.  float32 4x4 matrices go
+    through the library's host function once it is loaded (the same
+    operations, bit for bit)."""
+    a = _arr(m)
+    if a.shape[-2:] == (4, 4) and a.dtype == F32:
+        from . import _lib
+
+        lib = _lib.loaded()
+        if lib is not None:
+            src = np.ascontiguousarray(a)
+            out = np.empty(a.shape, F32)
+            _lib.check(lib.rast_lu_inverse4(src.ctypes.data, src.size // 16, out.ctypes.data), "rast_lu_inverse4")
+            return out
+    a = a.copy()
     dt = a.dtype
     n = a.shape[-1]
     batch = a.shape[:-2]

@@ -174,11 +174,61 @@ class _Pool:
         self.rows += n
         return begin
 
+    def host_bytes(self) -> Optional[int]:
+        """Bytes of the pool when every part is a host array, else None."""
+        if not self.parts or any(isinstance(p, torch.Tensor) for p in self.parts):
+            return None
+        return 4 * sum(int(np.size(p)) for p in self.parts)
+
+    def host_into(self, buf: np.ndarray) -> None:
+        """Write the parts into `buf` (the pool's bytes)."""
+        out = buf.view(np.float32 if self.dtype == torch.float32 else np.int32)
+        at = 0
+        for p in self.parts:
+            a = np.asarray(p).reshape(-1)
+            out[at : at + a.size] = a
+            at += a.size
+
+    def fresh(self, device) -> Optional[torch.Tensor]:
+        """tensor(), never sharing memory with a part."""
+        t = self.tensor(device)
+        shared = len(self.parts) == 1 and isinstance(self.parts[0], torch.Tensor) and t.device == self.parts[0].device
+        return t.clone() if shared else t
+
     def tensor(self, device) -> Optional[torch.Tensor]:
         if not self.parts:
             return None
         ts = [_to_dev(p, self.dtype, device).reshape(-1) for p in self.parts]
         return ts[0] if len(ts) == 1 else torch.cat(ts)
+
+
+# Host pools up to this many bytes in all go to the device in one copy: each
+# copy of its own is 20 us of host time (half of packing one cube's pass).
+ONE_COPY_BYTES = 1 << 20
+
+
+def _upload(pools, extra: bytes, device):
+    """({name: device tensor}, device copy of `extra`): the pools whose parts
+    are all host arrays as slices of one buffer when they are small."""
+    sizes = {k: n for k, n in ((k, p.host_bytes()) for k, p in pools.items()) if n}
+    step = lambda n: -(-n // 256) * 256  # noqa: E731
+    total = step(len(extra)) + sum(map(step, sizes.values()))
+    if total > ONE_COPY_BYTES:
+        sizes, total = {}, len(extra)
+    host = np.empty(total, np.uint8)
+    host[: len(extra)] = np.frombuffer(extra, np.uint8)
+    at = {}
+    end = step(len(extra))
+    for k, n in sizes.items():
+        pools[k].host_into(host[end : end + n])
+        at[k] = end
+        end += step(n)
+    dev = torch.from_numpy(host).to(device)
+    out = {k: dev[a : a + sizes[k]].view(pools[k].dtype) for k, a in at.items()}
+    for k, p in pools.items():
+        if k not in out and p.parts:
+            out[k] = p.tensor(device)
+    return out, dev[: len(extra)]
 
 
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
@@ -286,30 +336,21 @@ def pack(specs: Sequence[JobSpec], zbuffers: Sequence[Any], canvases: Sequence[A
         mask |= 1 << s.shader
         maxw, maxh, maxv, maxf = max(maxw, s.width), max(maxh, s.height), max(maxv, V), max(maxf, F)
 
-    keep = []
-
-    def dev(pool):
-        t = pool.tensor(device)
-        if t is not None:
-            keep.append(t)
-        return t
-
-    tensors = {name: dev(p) for name, p in (
-        ("position", pos), ("normal", nrm), ("uv", uvp), ("colour", col), ("texture_index", tix),
-        ("id_to_face", i2f), ("faces", fac), ("darboux_faces", dfc), ("texture", tex),
-        ("specular_map", spm), ("normal_map", nmp), ("texture_shape", tsh), ("shadow_map", shm),
-        ("face_alpha", alp))}
-    zbuf = zb.tensor(device).clone()
+    tensors, jobs_dev = _upload({"position": pos, "normal": nrm, "uv": uvp, "colour": col, "texture_index": tix,
+                                 "id_to_face": i2f, "faces": fac, "darboux_faces": dfc, "texture": tex,
+                                 "specular_map": spm, "normal_map": nmp, "texture_shape": tsh, "shadow_map": shm,
+                                 "face_alpha": alp}, bytes(jobs), device)
+    keep = list(tensors.values())
+    zbuf = zb.fresh(device)
     canvas = None
     if cv.parts:
         if cv.rows < pixels:
             cv.add(np.zeros((pixels - cv.rows, 3), np.float32))
-        canvas = cv.tensor(device).clone()
+        canvas = cv.fresh(device)
     prim = torch.empty(pixels, dtype=torch.int32, device=device) if want_prim_id else None
     # layered jobs: the chooser's slots, saved for the backward
     layer_prim = torch.empty((_lib.MAX_LAYERS, pixels), dtype=torch.int32, device=device) if max_layers > 0 else None
     ties = torch.zeros(1, dtype=torch.int64, device=device) if count_ties else None
-    jobs_dev = torch.frombuffer(bytearray(bytes(jobs)), dtype=torch.uint8).to(device)
     keep.append(jobs_dev)
 
     b = _lib.RastBatch()
@@ -328,7 +369,7 @@ def pack(specs: Sequence[JobSpec], zbuffers: Sequence[Any], canvases: Sequence[A
     P.layer_prim = _ptr(layer_prim)
     b.near_ties = _ptr(ties)
     return PackedBatch(b, keep, zbuf, canvas, prim, ties, pixel_begin,
-                       {k: v for k, v in tensors.items() if v is not None}, jobs, layer_prim)
+                       tensors, jobs, layer_prim)
 
 
 def render_plain(packed: PackedBatch, stream: Optional[torch.cuda.Stream] = None) -> None:

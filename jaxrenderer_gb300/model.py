@@ -96,11 +96,10 @@ class MergedModel(NamedTuple):
         dims = maps[0].ndim
         single = tuple(max(m.shape[i] for m in maps) for i in range(dims))
         dtype = np.result_type(*maps)
-        padded = [
-            np.pad(m, [(0, single[i] - m.shape[i]) for i in range(dims)]).astype(dtype)
-            for m in maps
-        ]
-        return np.concatenate(padded, axis=0), (single[0], single[1])
+        out = np.zeros((len(maps) * single[0],) + single[1:], dtype)
+        for i, m in enumerate(maps):
+            out[i * single[0] : (i + 1) * single[0]][tuple(slice(0, n) for n in m.shape)] = m
+        return out, (single[0], single[1])
 
     @staticmethod
     def uv_repeat(uv, shape, map_index, offset) -> np.ndarray:

@@ -68,6 +68,8 @@ def gather_rows(arr, idx) -> np.ndarray:
     a = np.asarray(arr)
     i = np.asarray(idx).astype(np.int64)
     n = a.shape[0]
+    if i.size and i.min() >= 0 and i.max() < n:  # in range: nothing to wrap or clamp
+        return a.take(i, axis=0)
     i = np.where(i < 0, i + n, i)
     return a[np.clip(i, 0, n - 1)]
 
@@ -184,8 +186,10 @@ class Renderer:
                     b = cls._batch_size(v)
                     if b is not None:
                         sizes.add(b)
-                elif name in ranks and np.ndim(v) == ranks[name] + 1:
-                    sizes.add(int(np.shape(v)[0]))
+                elif name in ranks:
+                    shape = v.shape if hasattr(v, "shape") else np.shape(v)
+                    if len(shape) == ranks[name] + 1:
+                        sizes.add(int(shape[0]))
         if len(sizes) > 1:
             raise ValueError(f"batched arguments disagree on the batch size: {sorted(sizes)}")
         return sizes.pop() if sizes else None
