@@ -38,12 +38,12 @@ namespace rast {
 namespace bwd {
 
 constexpr int kThreads = 256;
-// Rows (faces or vertices) per block of the per-face and per-vertex kernels:
-// few rows of a block are visible, so each block scans kRowsPerThread rows
-// per thread and works through the queued ones, paying its job load, queue
-// and parameter reduction once per kRows rows.
-constexpr int kRowsPerThread = 32;
-constexpr int kRows = kThreads * kRowsPerThread;
+// The per-face and per-vertex kernels: a few percent of the rows are visible,
+// so each warp takes one block-map entry of kRows rows, lists the marked ones
+// (list_marked) and works through them, one per lane.
+constexpr int kRows = 256;
+constexpr int kSparseThreads = 128;
+constexpr int kSparseWarps = kSparseThreads / 32;
 
 // Gradient-only arithmetic.  Values that feed gradients alone (checked to a
 // relative tolerance) and no branch of the forward's (the texel index, the
@@ -192,24 +192,7 @@ struct ParamGrad {
   float v[RAST_NPARAM];
 };
 
-struct NoPost {
-  static constexpr bool kActive = false;
-  __device__ void operator()(float*) const {}
-};
-
-// Block reduction of the parameters in BITS, added to this block's scene.
-// Every thread of the block must call it.
-// `active`: this thread contributed; warps without a contributing thread
-// skip their shuffles and add zeros.  `post` (when Post::kActive) maps the
-// block's totals, on one thread, before they are added: the linear maps
-// every pixel's contribution would go through are applied once per block.
-// kTransposed (kernels that reduce once per thread and pixel): the span
-// [kLo, kLo + kSpan) of BITS, up to 32 parameters, is summed by a transpose
-// through shared memory (each lane stores its values, lane n adds parameter
-// kLo + n's 32 values) instead of one shuffle tree per parameter.  Rows of
-// 36 floats: the 128-bit row reads of 8 lanes hit distinct banks.  The
-// transpose uses the caller's shared scratch `cols` of
-// transpose_floats<BITS>() floats (16-byte aligned).
+// Parameters [kLo, kLo + span) that cover BITS.
 template <unsigned long long BITS>
 __host__ __device__ constexpr int param_span() {
   return BITS ? 64 - __builtin_clzll(BITS) - (BITS ? __builtin_ctzll(BITS) : 0) : 0;
@@ -218,52 +201,53 @@ template <unsigned long long BITS>
 __host__ __device__ constexpr int transpose_floats() {
   return (kThreads / 32) * param_span<BITS>() * 36;
 }
-template <unsigned long long BITS, bool kTransposed = false, class Post = NoPost>
-__device__ __forceinline__ void reduce_params(const ParamGrad& pg, float* job_params, bool active, int job,
-                                              const Post& post = Post(), float* cols = nullptr) {
+
+// Sum over the warp of parameter kLo + lane (lanes below the span, at most
+// 32): a transpose through shared memory (each lane stores its values, lane n
+// adds parameter kLo + n's 32 values) instead of one shuffle tree per
+// parameter.  Rows of 36 floats: the 128-bit row reads of 8 lanes hit
+// distinct banks.  `col`: the warp's span * 36 floats, 16-byte aligned.
+template <unsigned long long BITS>
+__device__ __forceinline__ float warp_param_sum(const ParamGrad& pg, float* col) {
   constexpr int kLo = BITS ? __builtin_ctzll(BITS) : 0;
   constexpr int kSpan = param_span<BITS>();
-  constexpr bool kTranspose = kTransposed && kSpan > 0 && kSpan <= 32;
+  static_assert(kSpan <= 32, "one parameter per lane");
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int n = 0; n < kSpan; ++n) col[n * 36 + lane] = ((BITS >> (kLo + n)) & 1ull) ? pg.v[kLo + n] : 0.0f;
+  __syncwarp();
+  if (lane >= kSpan) return 0.0f;
+  float a = 0.0f, b = 0.0f, c = 0.0f, d = 0.0f;
+  const float4* row = reinterpret_cast<const float4*>(col + lane * 36);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float4 t = row[q];
+    a += t.x;
+    b += t.y;
+    c += t.z;
+    d += t.w;
+  }
+  return (a + b) + (c + d);
+}
+
+// Block reduction of the parameters in BITS, added to this block's scene.
+// Every thread of the block must call it.
+// `active`: this thread contributed; warps without a contributing thread add
+// zeros.  `post` maps the block's totals, on one thread, before they are
+// added: the linear maps every pixel's contribution would go through are
+// applied once per block.  `cols`: transpose_floats<BITS>() floats of shared
+// scratch (16-byte aligned).
+template <unsigned long long BITS, class Post>
+__device__ __forceinline__ void reduce_params(const ParamGrad& pg, float* job_params, bool active, int job,
+                                              const Post& post, float* cols) {
+  constexpr int kLo = BITS ? __builtin_ctzll(BITS) : 0;
+  constexpr int kSpan = param_span<BITS>();
   __shared__ float s_red[kThreads / 32][RAST_NPARAM];
-  __shared__ float s_tot[Post::kActive ? RAST_NPARAM : 1];
+  __shared__ float s_tot[RAST_NPARAM];
   if (BITS == 0ull || !job_params) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool warp_active = __any_sync(0xffffffffu, active);
-  if (kTranspose) {
-    if (warp_active) {
-      float* col = cols + warp * kSpan * 36;  // this warp's rows: parameter n at col[n * 36 ...]
-#pragma unroll
-      for (int n = 0; n < kSpan; ++n) col[n * 36 + lane] = ((BITS >> (kLo + n)) & 1ull) ? pg.v[kLo + n] : 0.0f;
-      __syncwarp();
-      if (lane < kSpan) {
-        float a = 0.0f, b = 0.0f, c = 0.0f, d = 0.0f;
-        const float4* row = reinterpret_cast<const float4*>(col + lane * 36);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const float4 t = row[q];
-          a += t.x;
-          b += t.y;
-          c += t.z;
-          d += t.w;
-        }
-        s_red[warp][kLo + lane] = (a + b) + (c + d);
-      }
-    } else if (lane < kSpan) {
-      s_red[warp][kLo + lane] = 0.0f;
-    }
-  } else {
-#pragma unroll
-    for (int k = 0; k < RAST_NPARAM; ++k) {
-      if (!((BITS >> k) & 1ull)) continue;
-      float v = 0.0f;
-      if (warp_active) {
-        v = pg.v[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-      }
-      if (lane == 0) s_red[warp][k] = v;
-    }
-  }
+  const float sum = __any_sync(0xffffffffu, active) ? warp_param_sum<BITS>(pg, cols + warp * kSpan * 36) : 0.0f;
+  if (lane < kSpan) s_red[warp][kLo + lane] = sum;
   __syncthreads();
   const bool mine = threadIdx.x < RAST_NPARAM && ((BITS >> threadIdx.x) & 1ull);
   float v = 0.0f;
@@ -271,13 +255,11 @@ __device__ __forceinline__ void reduce_params(const ParamGrad& pg, float* job_pa
 #pragma unroll
     for (int w = 0; w < kThreads / 32; ++w) v += s_red[w][threadIdx.x];
   }
-  if (Post::kActive) {
-    if (threadIdx.x < RAST_NPARAM) s_tot[threadIdx.x] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) post(s_tot);
-    __syncthreads();
-    if (mine) v = s_tot[threadIdx.x];
-  }
+  if (threadIdx.x < RAST_NPARAM) s_tot[threadIdx.x] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) post(s_tot);
+  __syncthreads();
+  if (mine) v = s_tot[threadIdx.x];
   if (mine && v != 0.0f) atomicAdd(job_params + static_cast<int64_t>(job) * RAST_NPARAM + threadIdx.x, v);
 }
 
@@ -293,7 +275,6 @@ struct LightUnit {
 // the block's total goes through normalise's reverse mode once (it is
 // linear in the incoming gradient).
 struct LightPost {
-  static constexpr bool kActive = true;
   const LightUnit* lu;
   int shader;
   __device__ void operator()(float* tot) const {
@@ -310,25 +291,29 @@ struct LightPost {
 
 // Workspace views (see layout()).
 struct Work {
-  unsigned char* fvis;  // per face (setup rows): shown by some pixel
+  uint32_t* fvis;       // a bit per face (setup rows): shown by some pixel
   float4* frec;         // per face: [m0..3] [m4..7] [m8 z0 z1 z2]
   float* facc;          // per face: dL/dm (9), dL/dz_clip (3)
-  unsigned char* vvis;  // per vertex (vout rows): corner of a shown face
+  uint32_t* vvis;       // a bit per vertex (vout rows): corner of a shown face
   float* vvar;          // per vertex: varyings (vstride)
   float* vacc;          // per vertex: dL/d(eye normal or colour varying) (3), then dL/d of the
                         // phong_darboux NDC triangle (9) when that shader is in the batch
   int vstride;
   int vacc_stride;      // 3, or 12 with phong_darboux
-  int2* fmap;           // face block map (kRows faces per block)
+  int2* fmap;           // face block map (kRows faces per entry)
   int2* vmap;           // vertex block map
+  unsigned fentries, ventries;
+  unsigned fsplit, vsplit;  // warps per entry
   LightUnit* light;     // per job: normalised light directions
 };
 
 // --------------------------------------------------------------- kernels
 
 // Grids: (pixel blocks of the largest job, n_jobs) for the pixel kernel and
-// the mark kernel (whose blocks cover kMarkPixels * kThreads pixels); block
-// maps of kRows faces or vertices of one job for the others.
+// the mark kernel (whose blocks cover kMarkPixels * kThreads pixels); warps
+// per block-map entry (kRows faces or vertices of one job) for the others.
+__device__ __forceinline__ void mark_row(uint32_t* marks, int64_t row) { atomicOr(marks + (row >> 5), 1u << (row & 31)); }
+inline size_t mark_bytes(int64_t rows) { return (static_cast<size_t>(rows) + 31) / 32 * 4; }
 
 // Pixels per thread of the mark kernel: their winners are loaded together,
 // so one block's load latency covers kMarkPixels * kThreads pixels.
@@ -346,7 +331,7 @@ __global__ void __launch_bounds__(kThreads) mark_kernel(RastBatch B, Work w) {
       if (local >= npx) break;
       for (int s = 0; s < layers; ++s) {
         const int p = B.pools.layer_prim[s * B.total_pixels + J.pixel_begin + local];
-        if (p >= 0) w.fvis[J.setup_begin + p] = 1;
+        if (p >= 0) mark_row(w.fvis, J.setup_begin + p);
       }
     }
     return;
@@ -362,7 +347,7 @@ __global__ void __launch_bounds__(kThreads) mark_kernel(RastBatch B, Work w) {
 #pragma unroll
   for (int r = 0; r < kMarkPixels; ++r) {
     const int prev = __shfl_up_sync(kFull, p[r], 1);
-    if (p[r] >= 0 && ((threadIdx.x & 31) == 0 || prev != p[r])) w.fvis[J.setup_begin + p[r]] = 1;
+    if (p[r] >= 0 && ((threadIdx.x & 31) == 0 || prev != p[r])) mark_row(w.fvis, J.setup_begin + p[r]);
   }
 }
 
@@ -371,11 +356,11 @@ __global__ void __launch_bounds__(kThreads) mark_kernel(RastBatch B, Work w) {
 // blocks load it with the job instead of computing it on one thread between
 // two barriers.  One launch where two memsets, four block-map kernels and a
 // light kernel ran one after the other.
-__global__ void __launch_bounds__(kThreads) begin_kernel(RastBatch B, Work w, unsigned fblocks, unsigned vblocks) {
-  fill_words(w.fvis, static_cast<size_t>(B.total_setup), 0u);
-  fill_words(w.vvis, static_cast<size_t>(B.total_vout), 0u);
-  fill_block_map<kMapFaces>(B.jobs, B.n_jobs, kRows, w.fmap, fblocks);
-  fill_block_map<kMapVertices>(B.jobs, B.n_jobs, kRows, w.vmap, vblocks);
+__global__ void __launch_bounds__(kThreads) begin_kernel(RastBatch B, Work w) {
+  fill_words(w.fvis, (static_cast<size_t>(B.total_setup) + 31) / 32 * 4, 0u);
+  fill_words(w.vvis, (static_cast<size_t>(B.total_vout) + 31) / 32 * 4, 0u);
+  fill_block_map<kMapFaces>(B.jobs, B.n_jobs, kRows, w.fmap, w.fentries);
+  fill_block_map<kMapVertices>(B.jobs, B.n_jobs, kRows, w.vmap, w.ventries);
   for (int j = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); j < B.n_jobs;
        j += static_cast<int>(gridDim.x * blockDim.x)) {
     const RastJob& J = B.jobs[j];
@@ -404,7 +389,7 @@ __device__ __forceinline__ void face_prep(const RastBatch& B, const Work& w, con
     M[3 * k + 1] = c[1];
     M[3 * k + 2] = c[3];
     zc[k] = c[2];
-    w.vvis[J.vout_begin + v] = 1;
+    mark_row(w.vvis, J.vout_begin + v);
   }
   float m[9];
   inv3(M, m);
@@ -432,47 +417,47 @@ __device__ __forceinline__ void vertex_prep(const RastBatch& B, const Work& w, c
   for (int k = 0; k < w.vacc_stride; ++k) w.vacc[row * w.vacc_stride + k] = 0.0f;
 }
 
-// The per-face and per-corner kernels cover kRows rows per block: the
-// block's visible faces (or flagged corners) are queued in shared memory
-// first, so only they occupy lanes.  They are latency-bound gathers: their
-// minimum blocks per SM (4 or 5, 48-64 registers) trade a few spills for
-// resident warps (vertex_prep 0.55 -> 0.40 ms on the 4096-scene batch).
-__global__ void __launch_bounds__(kThreads, 4) face_prep_kernel(RastBatch B, Work w) {
-  __shared__ RastJob sJ;
-  __shared__ int s_q[kRows];
-  __shared__ int s_n;
-  const int2 blk = w.fmap[blockIdx.x];
-  if (blk.x < 0) return;
-  const int nf = __ldg(&B.jobs[blk.x].n_faces);
-  load_job_to_shared(B.jobs + blk.x, &sJ);
-  if (threadIdx.x == 0) s_n = 0;
-  __syncthreads();
-  const RastJob& J = sJ;
-  const int n = block_queue_rows<kRowsPerThread, kThreads>(
-      [&](int r) { return blk.y + r < nf && w.fvis[J.setup_begin + blk.y + r]; }, s_q, &s_n);
-  for (int t = threadIdx.x; t < n; t += kThreads) face_prep(B, w, J, blk.y + s_q[t]);
+// The entry and share of this warp among `split` warps per entry: false past
+// the last entry and for empty entries.
+__device__ __forceinline__ bool warp_entry(const int2* __restrict__ map, unsigned entries, unsigned split, unsigned wid,
+                                           int2* blk, int* share) {
+  const unsigned e = wid / split;
+  if (e >= entries) return false;
+  *blk = __ldg(map + e);
+  *share = static_cast<int>(wid - e * split);
+  return blk->x >= 0;
+}
+
+// Latency-bound gathers over the marked rows.  Warps independent of one
+// another take the place of blocks that queued 8,192 rows each behind two
+// barriers, most of whose lanes had no row (19 % of warps active, 25 % issue):
+// 1024 brax-like scenes face_prep 64 -> 54 us at 8 blocks (59 at 10, 66 at
+// 12), vertex_prep 117 -> 104; 256 spheres of 5,120 faces vertex_prep 17 -> 12.
+__global__ void __launch_bounds__(kSparseThreads, 8) face_prep_kernel(RastBatch B, Work w) {
+  __shared__ unsigned char s_list[kSparseWarps][kRows];
+  unsigned char* list = s_list[threadIdx.x >> 5];
+  int2 blk;
+  int share;
+  if (!warp_entry(w.fmap, w.fentries, w.fsplit, (blockIdx.x * kSparseThreads + threadIdx.x) >> 5, &blk, &share)) return;
+  const RastJob& J = B.jobs[blk.x];
+  const int n = list_marked<kRows>(w.fvis, J.setup_begin + blk.y, J.n_faces - blk.y, list);
+  for (int t = share * 32 + static_cast<int>(threadIdx.x & 31); t < n; t += 32 * static_cast<int>(w.fsplit))
+    face_prep(B, w, J, blk.y + list[t]);
 }
 
 // Compiled per shader like the pixel kernel: a single-shader batch's variant
-// holds its vertex shader alone (62 registers without spills for
-// phong_reflection_shadow, against 64 with spills for the any-shader form:
-// 0.397 -> 0.369 ms on the 4096-scene brax-like batch; six blocks per SM at
-// 40 registers measured 0.413 ms, two queued vertices per round 0.391 ms).
+// holds its vertex shader alone.
 template <int SH>
-__global__ void __launch_bounds__(kThreads, 4) vertex_prep_kernel(RastBatch B, Work w) {
-  __shared__ RastJob sJ;
-  __shared__ int s_q[kRows];
-  __shared__ int s_n;
-  const int2 blk = w.vmap[blockIdx.x];
-  if (blk.x < 0) return;
-  const int nvt = __ldg(&B.jobs[blk.x].n_verts);
-  load_job_to_shared(B.jobs + blk.x, &sJ);
-  if (threadIdx.x == 0) s_n = 0;
-  __syncthreads();
-  const RastJob& J = sJ;
-  const int n = block_queue_rows<kRowsPerThread, kThreads>(
-      [&](int r) { return blk.y + r < nvt && w.vvis[J.vout_begin + blk.y + r]; }, s_q, &s_n);
-  for (int t = threadIdx.x; t < n; t += kThreads) vertex_prep<SH>(B, w, J, blk.y + s_q[t]);
+__global__ void __launch_bounds__(kSparseThreads, 8) vertex_prep_kernel(RastBatch B, Work w) {
+  __shared__ unsigned char s_list[kSparseWarps][kRows];
+  unsigned char* list = s_list[threadIdx.x >> 5];
+  int2 blk;
+  int share;
+  if (!warp_entry(w.vmap, w.ventries, w.vsplit, (blockIdx.x * kSparseThreads + threadIdx.x) >> 5, &blk, &share)) return;
+  const RastJob& J = B.jobs[blk.x];
+  const int n = list_marked<kRows>(w.vvis, J.vout_begin + blk.y, J.n_verts - blk.y, list);
+  for (int t = share * 32 + static_cast<int>(threadIdx.x & 31); t < n; t += 32 * static_cast<int>(w.vsplit))
+    vertex_prep<SH>(B, w, J, blk.y + list[t]);
 }
 
 // Reverse mode of the fragment of shader `sh` at one pixel.  In: the three
@@ -1010,7 +995,7 @@ pixel_kernel(RastBatch B, Work w, CanvasGrad cg, const float* __restrict__ grad_
     for (int q = 0; q < 3; ++q) pg.v[RAST_GRAD_BACKGROUND + q] += gcv_px[q] * transmit;
   }
   __syncthreads();  // every warp is done with its table before the transpose reuses the memory
-  reduce_params<kBits, true>(pg, G.job_params, in_job && (over ? shown : P.prim_id[pix] >= 0), blockIdx.y,
+  reduce_params<kBits>(pg, G.job_params, in_job && (over ? shown : P.prim_id[pix] >= 0), blockIdx.y,
                              LightPost{&sL, sh}, s_tab);
 }
 
@@ -1059,23 +1044,32 @@ __device__ __forceinline__ void face_post(const RastBatch& B, const Work& w, con
   }
 }
 
-// One block of face_post work (kRows faces of one job, from the face block
-// map); the block's shared job copy and queue are the caller's.
-__device__ __forceinline__ void face_post_block(const RastBatch& B, const Work& w, const RastGradPools& G, int2 blk,
-                                                RastJob& sJ, int* s_q, int* s_n) {
-  if (blk.x < 0) return;  // uniform over the block
-  const int nf = __ldg(&B.jobs[blk.x].n_faces);
-  load_job_to_shared(B.jobs + blk.x, &sJ);
-  if (threadIdx.x == 0) *s_n = 0;
-  __syncthreads();
-  const RastJob& J = sJ;
-  const int n = block_queue_rows<kRowsPerThread, kThreads>(
-      [&](int r) { return blk.y + r < nf && w.fvis[J.setup_begin + blk.y + r]; }, s_q, s_n);
-  ParamGrad pg;
+// The warp's totals of the parameters in BITS, added to job `job`
+// (warp_param_sum where the span of BITS fits the lanes, shuffles otherwise).
+// `col`: the warp's shared scratch, warp_floats<BITS>() floats, 16-byte
+// aligned.  Every lane of the warp must call it.
+template <unsigned long long BITS>
+__host__ __device__ constexpr int warp_floats() {
+  return param_span<BITS>() <= 32 ? param_span<BITS>() * 36 : 4;
+}
+template <unsigned long long BITS>
+__device__ __forceinline__ void reduce_params_warp(const ParamGrad& pg, float* job_params, int job, float* col) {
+  if (BITS == 0ull || !job_params) return;
+  const int lane = threadIdx.x & 31;
+  float* out = job_params + static_cast<int64_t>(job) * RAST_NPARAM;
+  if constexpr (param_span<BITS>() <= 32) {
+    const float v = warp_param_sum<BITS>(pg, col);
+    if (v != 0.0f) atomicAdd(out + (BITS ? __builtin_ctzll(BITS) : 0) + lane, v);  // zero past the span
+  } else {
 #pragma unroll
-  for (int k = 0; k < 16; ++k) pg.v[RAST_GRAD_WORLD_TO_CLIP + k] = 0.0f;
-  for (int t = threadIdx.x; t < n; t += kThreads) face_post(B, w, J, G, blk.y + s_q[t], pg);
-  reduce_params<kClipBits>(pg, G.job_params, static_cast<int>(threadIdx.x) < n, blk.x);
+    for (int k = 0; k < RAST_NPARAM; ++k) {
+      if (!((BITS >> k) & 1ull)) continue;
+      float v = pg.v[k];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      if (lane == 0 && v != 0.0f) atomicAdd(out + k, v);
+    }
+  }
 }
 
 // Reverse mode of the vertex shader: Gouraud lighting or the eye-space
@@ -1189,48 +1183,60 @@ __device__ __forceinline__ void vertex_post(const RastBatch& B, const Work& w, c
   }
 }
 
-// One block of vertex_post work (kRows vertices of one job, from the
-// vertex block map), like face_post_block.
+// face_post and vertex_post read only what the pixel kernel accumulated and
+// add into the gradients with atomics, so one launch runs both, a warp per
+// map entry: block b takes the face role when floor((b + 1) nfb / (nfb +
+// nvb)) > floor(b nfb / (nfb + nvb)) (face block floor(b nfb / (nfb + nvb))),
+// the vertex role otherwise (vertex block b minus the face blocks before it),
+// so the two kinds are spread evenly over the grid and resident together.
+// Ten blocks per SM for the reflection shaders (1024 brax-like scenes: 112
+// us, 119 at eight, 148 at six; 125 with the blocks of 8,192 rows), eight for
+// the others (256 phong spheres: 37 us, 40 at ten, from 58).
 template <int SH>
-__device__ __forceinline__ void vertex_post_block(const RastBatch& B, const Work& w, const RastGradPools& G, int2 blk,
-                                                  RastJob& sJ, int* s_q, int* s_n) {
-  if (blk.x < 0) return;  // uniform over the block
-  const int nvt = __ldg(&B.jobs[blk.x].n_verts);
-  load_job_to_shared(B.jobs + blk.x, &sJ);
-  if (threadIdx.x == 0) *s_n = 0;
-  __syncthreads();
-  const RastJob& J = sJ;
-  const int sh = SH >= 0 ? SH : J.shader;
-  const int n = sh == RAST_SHADER_DEPTH ? 0 : block_queue_rows<kRowsPerThread, kThreads>(
-      [&](int r) { return blk.y + r < nvt && w.vvis[J.vout_begin + blk.y + r]; }, s_q, s_n);
-  ParamGrad pg;
-#pragma unroll
-  for (int k = 0; k < RAST_NPARAM; ++k) pg.v[k] = 0.0f;
-  for (int t = threadIdx.x; t < n; t += kThreads) vertex_post<SH>(B, w, J, G, blk.y + s_q[t], pg);
-  reduce_params<vertex_bits(SH)>(pg, G.job_params, static_cast<int>(threadIdx.x) < n, blk.x);
+__host__ __device__ constexpr int post_min_blocks() {
+  return SH == RAST_SHADER_PHONG_REFLECTION || SH == RAST_SHADER_PHONG_REFLECTION_SHADOW || SH == kReflectionShaders ? 10 : 8;
 }
 
-// face_post and vertex_post read only what the pixel kernel accumulated and
-// add into the gradients with atomics, so one launch runs both, each a
-// latency-bound gather over sparse rows: block b takes the face role when
-// floor((b + 1) nfb / (nfb + nvb)) > floor(b nfb / (nfb + nvb)) (face block
-// floor(b nfb / (nfb + nvb))), the vertex role otherwise (vertex block b
-// minus the face blocks before it), so the two kinds are spread evenly over
-// the grid and resident together.
 template <int SH>
-__global__ void __launch_bounds__(kThreads, 4) post_kernel(RastBatch B, Work w, RastGradPools G, unsigned nfb,
-                                                            unsigned nvb) {
-  __shared__ RastJob sJ;
-  __shared__ int s_q[kRows];
-  __shared__ int s_n;
+__global__ void __launch_bounds__(kSparseThreads, post_min_blocks<SH>())
+post_kernel(RastBatch B, Work w, RastGradPools G, unsigned nfb, unsigned nvb) {
+  constexpr int kScratch = warp_floats<kClipBits>() > warp_floats<vertex_bits(SH)>() ? warp_floats<kClipBits>()
+                                                                                     : warp_floats<vertex_bits(SH)>();
+  __shared__ __align__(16) float s_col[kSparseWarps][kScratch];
+  __shared__ unsigned char s_list[kSparseWarps][kRows];
+  const int warp = threadIdx.x >> 5;
+  unsigned char* list = s_list[warp];
   const unsigned long long total = static_cast<unsigned long long>(nfb) + nvb;
   const unsigned long long b = blockIdx.x;
   const unsigned f0 = static_cast<unsigned>(b * nfb / total);
   const unsigned f1 = static_cast<unsigned>((b + 1) * nfb / total);
-  if (f1 > f0)
-    face_post_block(B, w, G, w.fmap[f0], sJ, s_q, &s_n);
-  else
-    vertex_post_block<SH>(B, w, G, w.vmap[b - f0], sJ, s_q, &s_n);
+  int2 blk;
+  int share;
+  ParamGrad pg;
+  if (f1 > f0) {
+    if (!warp_entry(w.fmap, w.fentries, w.fsplit, f0 * kSparseWarps + warp, &blk, &share)) return;
+    const RastJob& J = B.jobs[blk.x];
+    const int n = list_marked<kRows>(w.fvis, J.setup_begin + blk.y, J.n_faces - blk.y, list);
+    if (share * 32 >= n) return;  // nothing for this warp
+#pragma unroll
+    for (int k = 0; k < 16; ++k) pg.v[RAST_GRAD_WORLD_TO_CLIP + k] = 0.0f;
+    for (int t = share * 32 + static_cast<int>(threadIdx.x & 31); t < n; t += 32 * static_cast<int>(w.fsplit))
+      face_post(B, w, J, G, blk.y + list[t], pg);
+    __syncwarp();
+    reduce_params_warp<kClipBits>(pg, G.job_params, blk.x, s_col[warp]);
+    return;
+  }
+  if (!warp_entry(w.vmap, w.ventries, w.vsplit, (static_cast<unsigned>(b) - f0) * kSparseWarps + warp, &blk, &share)) return;
+  const RastJob& J = B.jobs[blk.x];
+  if ((SH >= 0 ? SH : J.shader) == RAST_SHADER_DEPTH) return;
+  const int n = list_marked<kRows>(w.vvis, J.vout_begin + blk.y, J.n_verts - blk.y, list);
+  if (share * 32 >= n) return;
+#pragma unroll
+  for (int k = 0; k < RAST_NPARAM; ++k) pg.v[k] = 0.0f;
+  for (int t = share * 32 + static_cast<int>(threadIdx.x & 31); t < n; t += 32 * static_cast<int>(w.vsplit))
+    vertex_post<SH>(B, w, J, G, blk.y + list[t], pg);
+  __syncwarp();
+  reduce_params_warp<vertex_bits(SH)>(pg, G.job_params, blk.x, s_col[warp]);
 }
 
 // ------------------------------------------------------------------ layout
@@ -1255,10 +1261,10 @@ static Layout layout(const RastBatch& b) {
     return o;
   };
   const size_t F = static_cast<size_t>(b.total_setup), V = static_cast<size_t>(b.total_vout);
-  L.fvis_off = take(F);
+  L.fvis_off = take(mark_bytes(b.total_setup));
   L.frec_off = take(F * 3 * sizeof(float4));
   L.facc_off = take(F * 12 * sizeof(float));
-  L.vvis_off = take(V);
+  L.vvis_off = take(mark_bytes(b.total_vout));
   L.vvar_off = take(V * vstride * sizeof(float));
   L.vacc_stride = (b.shader_mask & (1 << RAST_SHADER_PHONG_DARBOUX)) ? 12 : 3;
   L.vacc_off = take(V * L.vacc_stride * sizeof(float));
@@ -1273,26 +1279,26 @@ static Layout layout(const RastBatch& b) {
 
 template <int SH>
 static void launch_all(const RastBatch& b, const Work& w, const Layout& L, const CanvasGrad& gc, const float* gz,
-                       const RastGradPools& G, cudaStream_t s, Profiler& prof) {
+                       const RastGradPools& G, cudaStream_t s, Profiler& prof, int sms) {
   const int64_t max_px = static_cast<int64_t>(b.max_width) * b.max_height;
   const dim3 pgrid(static_cast<unsigned>((max_px + kThreads - 1) / kThreads), static_cast<unsigned>(b.n_jobs));
-  const unsigned fgrid = L.fblocks, vgrid = L.vblocks;
-  begin_kernel<<<begin_blocks(static_cast<size_t>(b.total_setup) + static_cast<size_t>(b.total_vout), b.n_jobs, sm_count()),
-                 kThreads, 0, s>>>(b, w, fgrid, vgrid);
+  begin_kernel<<<begin_blocks(mark_bytes(b.total_setup) + mark_bytes(b.total_vout), b.n_jobs, sms), kThreads, 0, s>>>(b, w);
   const int64_t mark_px = static_cast<int64_t>(kThreads) * kMarkPixels;
   mark_kernel<<<dim3(static_cast<unsigned>((max_px + mark_px - 1) / mark_px), static_cast<unsigned>(b.n_jobs)),
                 kThreads, 0, s>>>(b, w);
   prof.mark("backward_mark_kernels");
-  face_prep_kernel<<<fgrid, kThreads, 0, s>>>(b, w);
+  const unsigned fgrid = (w.fentries * w.fsplit + kSparseWarps - 1) / kSparseWarps;
+  const unsigned vgrid = (w.ventries * w.vsplit + kSparseWarps - 1) / kSparseWarps;
+  face_prep_kernel<<<fgrid, kSparseThreads, 0, s>>>(b, w);
   prof.mark("backward_face_prep_kernel");
-  vertex_prep_kernel<SH><<<vgrid, kThreads, 0, s>>>(b, w);
+  if (vgrid > 0) vertex_prep_kernel<SH><<<vgrid, kSparseThreads, 0, s>>>(b, w);
   prof.mark("backward_vertex_prep_kernel");
   if (b.max_layers > 0)
     pixel_kernel<SH, true><<<pgrid, kThreads, 0, s>>>(b, w, gc, gz, G);
   else
     pixel_kernel<SH, false><<<pgrid, kThreads, 0, s>>>(b, w, gc, gz, G);
   prof.mark("backward_pixel_kernel");
-  if (fgrid + vgrid > 0) post_kernel<SH><<<fgrid + vgrid, kThreads, 0, s>>>(b, w, G, fgrid, vgrid);
+  if (fgrid + vgrid > 0) post_kernel<SH><<<fgrid + vgrid, kSparseThreads, 0, s>>>(b, w, G, fgrid, vgrid);
   prof.mark("backward_post_kernel");
 }
 
@@ -1313,30 +1319,32 @@ static int run(const RastBatch* batch, const CanvasGrad& grad_canvas, const floa
   if (b.total_pixels == 0 || b.total_setup == 0) return RAST_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(workspace);
-  Work w{reinterpret_cast<unsigned char*>(ws + L.fvis_off), reinterpret_cast<float4*>(ws + L.frec_off),
-         reinterpret_cast<float*>(ws + L.facc_off), reinterpret_cast<unsigned char*>(ws + L.vvis_off),
+  const int sms = sm_count();
+  Work w{reinterpret_cast<uint32_t*>(ws + L.fvis_off), reinterpret_cast<float4*>(ws + L.frec_off),
+         reinterpret_cast<float*>(ws + L.facc_off), reinterpret_cast<uint32_t*>(ws + L.vvis_off),
          reinterpret_cast<float*>(ws + L.vvar_off), reinterpret_cast<float*>(ws + L.vacc_off), L.vstride,
          L.vacc_stride,
          reinterpret_cast<int2*>(ws + L.fmap_off), reinterpret_cast<int2*>(ws + L.vmap_off),
+         L.fblocks, L.vblocks, warps_per_entry(L.fblocks, sms), warps_per_entry(L.vblocks, sms),
          reinterpret_cast<LightUnit*>(ws + L.light_off)};
   Profiler prof(profile, s, "rast_backward");
   const int mask = b.shader_mask;
   auto only = [&](int sh) { return mask == (1 << sh); };
-  if (only(RAST_SHADER_DEPTH)) launch_all<RAST_SHADER_DEPTH>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
-  else if (only(RAST_SHADER_GOURAUD)) launch_all<RAST_SHADER_GOURAUD>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
+  if (only(RAST_SHADER_DEPTH)) launch_all<RAST_SHADER_DEPTH>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
+  else if (only(RAST_SHADER_GOURAUD)) launch_all<RAST_SHADER_GOURAUD>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
   else if (only(RAST_SHADER_GOURAUD_TEXTURE))
-    launch_all<RAST_SHADER_GOURAUD_TEXTURE>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
-  else if (only(RAST_SHADER_PHONG)) launch_all<RAST_SHADER_PHONG>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
+    launch_all<RAST_SHADER_GOURAUD_TEXTURE>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
+  else if (only(RAST_SHADER_PHONG)) launch_all<RAST_SHADER_PHONG>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
   else if (only(RAST_SHADER_PHONG_REFLECTION))
-    launch_all<RAST_SHADER_PHONG_REFLECTION>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
+    launch_all<RAST_SHADER_PHONG_REFLECTION>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
   else if (only(RAST_SHADER_PHONG_REFLECTION_SHADOW))
-    launch_all<RAST_SHADER_PHONG_REFLECTION_SHADOW>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
+    launch_all<RAST_SHADER_PHONG_REFLECTION_SHADOW>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
   else if (only(RAST_SHADER_PHONG_DARBOUX))
-    launch_all<RAST_SHADER_PHONG_DARBOUX>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
+    launch_all<RAST_SHADER_PHONG_DARBOUX>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
   else if (mask == ((1 << RAST_SHADER_PHONG_REFLECTION) | (1 << RAST_SHADER_PHONG_REFLECTION_SHADOW)))
-    launch_all<kReflectionShaders>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
+    launch_all<kReflectionShaders>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
   else
-    launch_all<kAnyShader>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof);
+    launch_all<kAnyShader>(b, w, L, grad_canvas, grad_zbuffer, *grads, s, prof, sms);
   if (cudaGetLastError() != cudaSuccess) return RAST_ERR_CUDA;
   return prof.finish();
 }

@@ -177,6 +177,45 @@ __device__ __forceinline__ void fill_block_map(const RastJob* __restrict__ jobs,
   }
 }
 
+// The marked ones among the n (at most kRows) rows from row0 on, one mark bit
+// per row in `marks`: their offsets from row0 go to the warp's `list` in
+// order (eight bits per lane, one prefix sum), and every lane gets their
+// number.  All 32 lanes must call.
+template <int kRows>
+__device__ __forceinline__ int list_marked(const uint32_t* __restrict__ marks, int64_t row0, int n, unsigned char* list) {
+  static_assert(kRows <= 256 && kRows % 32 == 0, "eight rows per lane, list entries of one byte");
+  const int lane = threadIdx.x & 31;
+  const int left = min(kRows, n) - 8 * lane;
+  unsigned bits = 0;
+  if (left > 0) {
+    const int64_t at = row0 + 8 * lane;
+    const unsigned shift = static_cast<unsigned>(at & 31);
+    bits = marks[at >> 5] >> shift;
+    if (shift > 24 && left > 32 - static_cast<int>(shift)) bits |= marks[(at >> 5) + 1] << (32 - shift);
+    bits &= left >= 8 ? 0xffu : (1u << left) - 1u;
+  }
+  int incl = __popc(bits);
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  int slot = incl - __popc(bits);
+#pragma unroll
+  for (int k = 0; k < 8; ++k)
+    if ((bits >> k) & 1u) list[slot++] = static_cast<unsigned char>(8 * lane + k);
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, incl, 31);
+}
+
+// Warps per map entry of the kernels that work through list_marked: up to
+// four while all of them are resident at once, so that a warp's rounds, 2-3
+// us of latency each, do not follow one another while SMs idle.
+inline unsigned warps_per_entry(unsigned entries, int sms) {
+  const unsigned k = static_cast<unsigned>(sms) * 48u / (entries > 0 ? entries : 1u);
+  return k < 1u ? 1u : k > 4u ? 4u : k;
+}
+
 // Sets `bytes` bytes at p (16-byte aligned; the last 16-byte word may run
 // past `bytes`, inside the workspace's 256-byte granules), the whole grid
 // striding over them.

@@ -1170,7 +1170,7 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
 // (marked by the raster kernel), stored per face: the shade then reads them
 // instead of re-running the vertex shader per pixel.  `split` warps per entry
 // of the set-up's block map: each lists the entry's marked faces in shared
-// memory (eight mark bits per lane), then takes one (face, corner) per lane
+// memory, then takes one (face, corner) per lane
 // and round, in memory order.  Gathers and normalisation chains bound it, at
 // 4096 brax-like scenes the sectors that 3.8 M faces' corners and rows touch
 // (1.2 GB): warps independent of one another (no block barrier, no shared job
@@ -1183,7 +1183,6 @@ template <int kRows>
 __global__ void __launch_bounds__(kFaceThreads, 12)
 face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entries, unsigned split,
                      const uint32_t* __restrict__ visible, float* __restrict__ fvar, int vstride) {
-  static_assert(kRows <= 256 && kRows % 32 == 0, "eight faces per lane, list entries of one byte");
   __shared__ unsigned char s_list[kFaceThreads / 32][kRows];
   const int lane = threadIdx.x & 31;
   unsigned char* list = s_list[threadIdx.x >> 5];
@@ -1194,29 +1193,7 @@ face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entrie
   if (blk.x < 0) return;
   const RastJob& J = B.jobs[blk.x];
   if (J.shader == RAST_SHADER_DEPTH) return;
-  // lane l: the mark bits of faces [8 l, 8 l + 8) of the entry
-  const int64_t row0 = J.setup_begin + blk.y;
-  const int left = min(kRows, J.n_faces - blk.y) - 8 * lane;
-  unsigned bits = 0;
-  if (left > 0) {
-    const int64_t at = row0 + 8 * lane;
-    const unsigned shift = static_cast<unsigned>(at & 31);
-    bits = visible[at >> 5] >> shift;
-    if (shift > 24 && left > 32 - static_cast<int>(shift)) bits |= visible[(at >> 5) + 1] << (32 - shift);
-    bits &= left >= 8 ? 0xffu : (1u << left) - 1u;
-  }
-  int incl = __popc(bits);
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += v;
-  }
-  const int total = 3 * __shfl_sync(0xffffffffu, incl, 31);
-  int slot = incl - __popc(bits);
-#pragma unroll
-  for (int k = 0; k < 8; ++k)
-    if ((bits >> k) & 1u) list[slot++] = static_cast<unsigned char>(8 * lane + k);
-  __syncwarp();
+  const int total = 3 * list_marked<kRows>(visible, J.setup_begin + blk.y, J.n_faces - blk.y, list);
   const int nv = varying_count(J.shader);
   for (int t = static_cast<int>(wid - entry * split) * 32 + lane; t < total; t += 32 * static_cast<int>(split)) {
     const int q = t / 3, k = t - 3 * q;
@@ -1552,8 +1529,7 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
       }
       prof.mark("raster_kernel");
       if (pre) {
-        // up to four warps per entry while all of them are resident at once
-        const unsigned split = std::min(4u, std::max(1u, static_cast<unsigned>(sms) * 48u / std::max(L.fmap_blocks, 1u)));
+        const unsigned split = warps_per_entry(L.fmap_blocks, sms);
         const unsigned vgrid = (L.fmap_blocks * split + kFaceThreads / 32 - 1) / (kFaceThreads / 32);
         if (L.small_path)
           face_varyings_kernel<setup_rows(true)><<<vgrid, kFaceThreads, 0, s>>>(b, fmap, L.fmap_blocks, split, vis, fvar,
