@@ -725,8 +725,10 @@ class BatchRunner:
 
 class MultiRunner:
     """Several SceneBatches (e.g. one per resolution class of a mixed batch),
-    each with its own BatchRunner and autotuned tiled config, rendered in
-    order on one stream; `capture()` records all of them into ONE CUDA graph
+    each with its own BatchRunner and autotuned tiled config, rendered beside
+    one another (each class on a stream of its own between a fork from and a
+    join into the caller's, so that one class's small launches fill the SMs
+    another's leave idle); `capture()` records all of them into ONE CUDA graph
     so a replay re-issues the whole mixed batch with a single launch."""
 
     def __init__(self, batches: Sequence[SceneBatch], form: str = "tiled", want_prim_id: bool = True,
@@ -738,6 +740,7 @@ class MultiRunner:
         self.form = form
         self.device = batches[0].device
         self.graph = None
+        self._streams = [torch.cuda.Stream(self.device) for _ in self.runners[1:]]
 
     @property
     def n_scenes(self) -> int:
@@ -745,7 +748,13 @@ class MultiRunner:
 
     def run(self, stream: Optional[torch.cuda.Stream] = None) -> List[BatchOutputs]:
         s = stream if stream is not None else torch.cuda.current_stream(self.device)
-        return [r.run(s) for r in self.runners]
+        for side in self._streams:
+            side.wait_stream(s)
+        try:
+            return [r.run(on) for r, on in zip(self.runners, [s, *self._streams])]
+        finally:
+            for side in self._streams:
+                s.wait_stream(side)
 
     def capture(self) -> None:
         dev = self.device
