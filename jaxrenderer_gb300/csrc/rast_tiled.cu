@@ -139,32 +139,23 @@ __device__ __forceinline__ void clip_push0(ClipStage& s, ClipStage& s1, ClipStag
 // the corners' error and the rounding of the pixel <-> NDC maps.  Returns
 // false when no pixel can be covered.
 // The job's screen rectangle one pixel wider on every side, in NDC (pixels
-// -1 and W), computed once per job by begin_kernel.
+// -1 and W), computed once per block, an axis per thread, while the others
+// load the job.
 struct ScreenRect {
   float xl, xh, yl, yh;
-  float gx, gy;  // half a pixel in NDC (0: rounding could reach it, see off_screen); gx < 0: no usable viewport
+  float gx, gy;  // half a pixel in NDC (0: rounding could reach it, see off_screen; below 0: no usable viewport)
   __device__ __forceinline__ float X() const { return fmaxf(fabsf(xl), fabsf(xh)); }
   __device__ __forceinline__ float Y() const { return fmaxf(fabsf(yl), fabsf(yh)); }
-  __device__ __forceinline__ bool ok() const { return gx >= 0.0f; }  // finite, non-degenerate viewport
+  __device__ __forceinline__ bool ok() const { return gx >= 0.0f && gy >= 0.0f; }  // finite, non-degenerate viewport
 };
 
-__device__ __forceinline__ ScreenRect screen_rect(const RastJob& J) {
-  ScreenRect r{};
-  const float sx = J.viewport[0], ox = J.viewport[3];
-  const float sy = J.viewport[5], oy = J.viewport[7];
-  const bool ok = (sx != 0.0f) && (sy != 0.0f) && isfinite(sx) && isfinite(sy);
-  const float xa = (-1.0f - ox) / sx, xb = (static_cast<float>(J.width) - ox) / sx;
-  const float ya = (-1.0f - oy) / sy, yb = (static_cast<float>(J.height) - oy) / sy;
-  r.xl = fminf(xa, xb);
-  r.xh = fmaxf(xa, xb);
-  r.yl = fminf(ya, yb);
-  r.yh = fmaxf(ya, yb);
-  r.gx = 0.5f / fabsf(sx);
-  r.gy = 0.5f / fabsf(sy);
-  if (!(r.X() * 4.8e-7f < r.gx)) r.gx = 0.0f;  // 8 u X
-  if (!(r.Y() * 4.8e-7f < r.gy)) r.gy = 0.0f;
-  if (!ok) r.gx = -1.0f;
-  return r;
+__device__ __forceinline__ void screen_axis(float scale, float offset, int size, float* lo, float* hi, float* g) {
+  const float a = (-1.0f - offset) / scale, b = (static_cast<float>(size) - offset) / scale;
+  *lo = fminf(a, b);
+  *hi = fmaxf(a, b);
+  const float half = 0.5f / fabsf(scale);
+  const float m = fmaxf(fabsf(*lo), fabsf(*hi));
+  *g = (scale != 0.0f && isfinite(scale)) ? (m * 4.8e-7f < half ? half : 0.0f) : -1.0f;  // 8 u m against half a pixel
 }
 
 // True when no pixel of the job can pass the edge tests against the inverse
@@ -464,7 +455,7 @@ __global__ void __launch_bounds__(kSetupThreads, setup_min_blocks(kSmall))
 setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4* __restrict__ setup,
                  unsigned char* __restrict__ binned_flag, uint32_t* __restrict__ counts,
                  unsigned long long* __restrict__ keys, int small_area, int4* __restrict__ binned,
-                 unsigned int* __restrict__ n_binned, const ScreenRect* __restrict__ rects) {
+                 unsigned int* __restrict__ n_binned) {
   constexpr int kRounds = setup_rounds(kSmall), kRows = setup_rows(kSmall);
   __shared__ RastJob sJ;
   __shared__ float s_m[12][kRows];
@@ -482,9 +473,14 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
   const int jid = blk.x;
   const int nf = __ldg(&B.jobs[jid].n_faces);
   load_job_to_shared(B.jobs + jid, &sJ);
-  if (threadIdx.x < sizeof(ScreenRect) / 4)
-    reinterpret_cast<int*>(&s_rect)[threadIdx.x] = __ldg(reinterpret_cast<const int*>(rects + jid) + threadIdx.x);
-  if (threadIdx.x == 0) s_qn = s_sn = 0;
+  if (threadIdx.x == 96) s_qn = s_sn = 0;
+  if (threadIdx.x == 32) {
+    const RastJob& g = B.jobs[jid];
+    screen_axis(g.viewport[0], g.viewport[3], g.width, &s_rect.xl, &s_rect.xh, &s_rect.gx);
+  } else if (threadIdx.x == 64) {
+    const RastJob& g = B.jobs[jid];
+    screen_axis(g.viewport[5], g.viewport[7], g.height, &s_rect.yl, &s_rect.yh, &s_rect.gy);
+  }
   __syncthreads();
   const RastJob& J = sJ;
   const float sx = J.viewport[0], ox = J.viewport[3], sy = J.viewport[5], oy = J.viewport[7];
@@ -633,7 +629,6 @@ struct BeginWork {
   size_t zero_bytes[3];
   void* keys;  // small path: every key starts as kEmptyKey
   size_t key_bytes;
-  ScreenRect* rects;  // per job
 };
 
 __global__ void __launch_bounds__(256) begin_kernel(RastBatch B, BeginWork w) {
@@ -641,10 +636,6 @@ __global__ void __launch_bounds__(256) begin_kernel(RastBatch B, BeginWork w) {
   for (int k = 0; k < 3; ++k) fill_words(w.zero[k], w.zero_bytes[k], 0u);
   fill_words(w.keys, w.key_bytes, 0xffffffffu);
   fill_block_map<kMapFaces>(B.jobs, B.n_jobs, w.map_rows, w.fmap, w.fmap_blocks);
-  if (w.fmap_blocks > 0)
-    for (int j = static_cast<int>(blockIdx.x * blockDim.x + threadIdx.x); j < B.n_jobs;
-         j += static_cast<int>(gridDim.x * blockDim.x))
-      w.rects[j] = screen_rect(B.jobs[j]);
 }
 
 // Bin offsets: a tile only needs a contiguous range of the bins, in no
@@ -1287,7 +1278,7 @@ inline uint64_t default_bin_capacity(const RastBatch& b) {
 
 struct Layout {
   size_t setup_off, flag_off, binned_off, counts_off, offsets_off, cursors_off, bins_off, winner_off, vis_off, fvar_off,
-      fmap_off, rect_off, keys_off, misc_off, total;
+      fmap_off, keys_off, misc_off, total;
   unsigned fmap_blocks;  // face block map of the set-up
   bool small_path;  // setup kernel rasterises small faces (not when near ties are counted)
   int vstride;
@@ -1337,7 +1328,6 @@ static Layout layout(const RastBatch& b, TileShape ts, uint64_t bin_capacity, in
   L.fmap_blocks = block_map_capacity(b.total_setup, b.n_jobs, setup_rows(L.small_path));
   L.fmap_off = take(static_cast<size_t>(L.fmap_blocks) * sizeof(int2));
   L.keys_off = take(L.small_path ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0);
-  L.rect_off = take(b.total_setup > 0 ? static_cast<size_t>(b.n_jobs) * sizeof(ScreenRect) : 0);
   L.misc_off = take(256);
   L.total = off;
   return L;
@@ -1485,7 +1475,6 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
     bw.zero[2] = vis;
     bw.zero_bytes[2] = vis ? (static_cast<size_t>(b.total_setup) + 31) / 32 * 4 : 0;
     bw.keys = keys;
-    bw.rects = reinterpret_cast<ScreenRect*>(ws + L.rect_off);
     bw.key_bytes = keys ? static_cast<size_t>(b.total_pixels) * sizeof(unsigned long long) : 0;
     begin_kernel<<<begin_blocks(bw.zero_bytes[0] + bw.zero_bytes[2] + bw.key_bytes, b.n_jobs, sms), 256, 0, s>>>(b, bw);
     prof.mark("begin_kernel");
@@ -1493,10 +1482,10 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
       const unsigned grid = L.fmap_blocks;
       if (keys)
         setup_bin_kernel<true><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, flag, counts, keys, small_area,
-                                                             binned, misc + 6, bw.rects);
+                                                             binned, misc + 6);
       else
         setup_bin_kernel<false><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, flag, counts, nullptr, 0,
-                                                              binned, misc + 6, bw.rects);
+                                                              binned, misc + 6);
       prof.mark("setup_bin_kernel");
       offsets_kernel<<<static_cast<unsigned>(L.n_scan_blocks), 256, 0, s>>>(
           counts, offsets, L.n_tiles, L.bin_capacity, misc + 1, reinterpret_cast<unsigned long long*>(misc + 2));
