@@ -320,6 +320,7 @@ inline size_t mark_bytes(int64_t rows) { return (static_cast<size_t>(rows) + 31)
 constexpr int kMarkPixels = 8;
 
 __global__ void __launch_bounds__(kThreads) mark_kernel(RastBatch B, Work w) {
+  after_previous();
   const RastJob& J = B.jobs[blockIdx.y];
   const int64_t npx = static_cast<int64_t>(J.width) * J.height;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * kThreads * kMarkPixels;
@@ -436,6 +437,7 @@ __device__ __forceinline__ bool warp_entry(const int2* __restrict__ map, unsigne
 __global__ void __launch_bounds__(kSparseThreads, 8) face_prep_kernel(RastBatch B, Work w) {
   __shared__ unsigned char s_list[kSparseWarps][kRows];
   unsigned char* list = s_list[threadIdx.x >> 5];
+  after_previous();
   int2 blk;
   int share;
   if (!warp_entry(w.fmap, w.fentries, w.fsplit, (blockIdx.x * kSparseThreads + threadIdx.x) >> 5, &blk, &share)) return;
@@ -451,6 +453,7 @@ template <int SH>
 __global__ void __launch_bounds__(kSparseThreads, 8) vertex_prep_kernel(RastBatch B, Work w) {
   __shared__ unsigned char s_list[kSparseWarps][kRows];
   unsigned char* list = s_list[threadIdx.x >> 5];
+  after_previous();
   int2 blk;
   int share;
   if (!warp_entry(w.vmap, w.ventries, w.vsplit, (blockIdx.x * kSparseThreads + threadIdx.x) >> 5, &blk, &share)) return;
@@ -781,6 +784,7 @@ pixel_kernel(RastBatch B, Work w, CanvasGrad cg, const float* __restrict__ grad_
   __shared__ RastJob sJ;
   __shared__ LightUnit sL;
   constexpr bool kDarboux = may<SH>(RAST_SHADER_PHONG_DARBOUX);
+  after_previous();
   load_job_to_shared(B.jobs + blockIdx.y, &sJ);
   static_assert(sizeof(LightUnit) == 8 * sizeof(float), "eight floats");
   if (threadIdx.x < 8)
@@ -1206,6 +1210,7 @@ post_kernel(RastBatch B, Work w, RastGradPools G, unsigned nfb, unsigned nvb) {
   __shared__ unsigned char s_list[kSparseWarps][kRows];
   const int warp = threadIdx.x >> 5;
   unsigned char* list = s_list[warp];
+  after_previous();
   const unsigned long long total = static_cast<unsigned long long>(nfb) + nvb;
   const unsigned long long b = blockIdx.x;
   const unsigned f0 = static_cast<unsigned>(b * nfb / total);
@@ -1284,21 +1289,21 @@ static void launch_all(const RastBatch& b, const Work& w, const Layout& L, const
   const dim3 pgrid(static_cast<unsigned>((max_px + kThreads - 1) / kThreads), static_cast<unsigned>(b.n_jobs));
   begin_kernel<<<begin_blocks(mark_bytes(b.total_setup) + mark_bytes(b.total_vout), b.n_jobs, sms), kThreads, 0, s>>>(b, w);
   const int64_t mark_px = static_cast<int64_t>(kThreads) * kMarkPixels;
-  mark_kernel<<<dim3(static_cast<unsigned>((max_px + mark_px - 1) / mark_px), static_cast<unsigned>(b.n_jobs)),
-                kThreads, 0, s>>>(b, w);
+  launch_after(mark_kernel, dim3(static_cast<unsigned>((max_px + mark_px - 1) / mark_px), static_cast<unsigned>(b.n_jobs)),
+               kThreads, s, b, w);
   prof.mark("backward_mark_kernels");
   const unsigned fgrid = (w.fentries * w.fsplit + kSparseWarps - 1) / kSparseWarps;
   const unsigned vgrid = (w.ventries * w.vsplit + kSparseWarps - 1) / kSparseWarps;
-  face_prep_kernel<<<fgrid, kSparseThreads, 0, s>>>(b, w);
+  launch_after(face_prep_kernel, fgrid, kSparseThreads, s, b, w);
   prof.mark("backward_face_prep_kernel");
-  if (vgrid > 0) vertex_prep_kernel<SH><<<vgrid, kSparseThreads, 0, s>>>(b, w);
+  if (vgrid > 0) launch_after(vertex_prep_kernel<SH>, vgrid, kSparseThreads, s, b, w);
   prof.mark("backward_vertex_prep_kernel");
   if (b.max_layers > 0)
-    pixel_kernel<SH, true><<<pgrid, kThreads, 0, s>>>(b, w, gc, gz, G);
+    launch_after(pixel_kernel<SH, true>, pgrid, kThreads, s, b, w, gc, gz, G);
   else
-    pixel_kernel<SH, false><<<pgrid, kThreads, 0, s>>>(b, w, gc, gz, G);
+    launch_after(pixel_kernel<SH, false>, pgrid, kThreads, s, b, w, gc, gz, G);
   prof.mark("backward_pixel_kernel");
-  if (fgrid + vgrid > 0) post_kernel<SH><<<fgrid + vgrid, kSparseThreads, 0, s>>>(b, w, G, fgrid, vgrid);
+  if (fgrid + vgrid > 0) launch_after(post_kernel<SH>, fgrid + vgrid, kSparseThreads, s, b, w, G, fgrid, vgrid);
   prof.mark("backward_post_kernel");
 }
 

@@ -107,6 +107,7 @@ __global__ void __launch_bounds__(kThreads)
 instance_kernel(RastMergeBatch B, const float* __restrict__ mesh_norm, float* __restrict__ mpos,
                 int* __restrict__ mobj, float* __restrict__ mnrm, float* __restrict__ muv) {
   __shared__ float stage[kThreads / 32][128];
+  after_previous();
   const int o = static_cast<int>((static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (o >= B.n_instances) return;  // whole warps
@@ -167,6 +168,7 @@ instance_kernel(RastMergeBatch B, const float* __restrict__ mesh_norm, float* __
 __global__ void __launch_bounds__(kThreads)
 corner_kernel(RastMergeBatch B, const float* __restrict__ mpos, const int* __restrict__ mobj,
               const float* __restrict__ mnrm, const float* __restrict__ muv) {
+  after_previous();
   const int o = static_cast<int>((static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (o >= B.n_instances) return;
@@ -283,8 +285,11 @@ static int run(const RastMergeBatch* batch, void* workspace, size_t workspace_by
   if (b.n_meshes > 0 && b.normal)
     mesh_norm_kernel<<<static_cast<unsigned>((static_cast<int64_t>(b.n_meshes) * 32 + kThreads - 1) / kThreads),
                        kThreads, 0, s>>>(b, mesh_norm);
-  instance_kernel<<<wg, kThreads, 0, s>>>(b, mesh_norm, mpos, mobj, mnrm, muv);
-  corner_kernel<<<wg, kThreads, 0, s>>>(b, mpos, mobj, mnrm, muv);
+  if (b.n_meshes > 0 && b.normal)
+    launch_after(instance_kernel, wg, kThreads, s, b, mesh_norm, mpos, mobj, mnrm, muv);
+  else
+    instance_kernel<<<wg, kThreads, 0, s>>>(b, mesh_norm, mpos, mobj, mnrm, muv);
+  launch_after(corner_kernel, wg, kThreads, s, b, mpos, mobj, mnrm, muv);
   return cudaGetLastError() == cudaSuccess ? RAST_OK : RAST_ERR_CUDA;
 }
 

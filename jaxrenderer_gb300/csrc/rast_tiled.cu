@@ -468,6 +468,7 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
   __shared__ float s_xs[kT], s_ys[kT];
   __shared__ int s_qn, s_sn;
   __shared__ ScreenRect s_rect;
+  after_previous();
   const int2 blk = fmap[blockIdx.x];
   if (blk.x < 0) return;
   const int jid = blk.x;
@@ -649,6 +650,7 @@ offsets_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ offse
                unsigned int* __restrict__ status, unsigned long long* __restrict__ cursor) {
   __shared__ uint32_t s_warp[8];
   __shared__ unsigned long long s_base;
+  after_previous();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t base = static_cast<int64_t>(blockIdx.x) * kScanBlock + threadIdx.x * 4;
   uint32_t v[4], t = 0;
@@ -699,6 +701,7 @@ offsets_kernel(const uint32_t* __restrict__ counts, uint32_t* __restrict__ offse
 __global__ void __launch_bounds__(kSetupThreads)
 scatter_kernel(Geometry G, const int4* __restrict__ binned, const unsigned int* __restrict__ n_binned,
                const uint32_t* __restrict__ offsets, uint32_t* __restrict__ cursors, int32_t* __restrict__ bins) {
+  after_previous();
   const unsigned n = *n_binned;
   const int lane = threadIdx.x & 31;
   constexpr unsigned kWarps = kSetupThreads / 32;
@@ -816,6 +819,7 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
   unsigned long long* sbest = s_best[kPairs ? warp : 0];
   float* tx_ndc = s_x[kPairs ? warp : 0];
   float* ty_ndc = s_y[kPairs ? warp : 0];
+  after_previous();
   unsigned long long tie_count = 0;
   unsigned long long tests = 0;  // pixel-triangle pairs this warp tested
   // The next tile is grabbed (one atomic on the shared counter) when this
@@ -1179,6 +1183,7 @@ face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entrie
   unsigned char* list = s_list[threadIdx.x >> 5];
   const unsigned wid = (blockIdx.x * kFaceThreads + threadIdx.x) >> 5;
   const unsigned entry = wid / split;
+  after_previous();
   if (entry >= entries) return;  // whole warps
   const int2 blk = fmap[entry];
   if (blk.x < 0) return;
@@ -1223,6 +1228,7 @@ tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t*
                    bool depth_resolved, const float* __restrict__ fvar, int vstride, Clear clear) {
   __shared__ RastJob sJ;
   __shared__ WarpFrags s_frags[kLayered ? 8 : 1];  // per warp, layered "over" jobs
+  after_previous();
   const int jid = blockIdx.y;
   const int64_t npx = static_cast<int64_t>(__ldg(&B.jobs[jid].width)) * __ldg(&B.jobs[jid].height);
   if (static_cast<int64_t>(blockIdx.x) * 256 >= npx) return;
@@ -1389,7 +1395,7 @@ static void launch_raster(TileShape ts, int wpt, int sms, cudaStream_t s, const 
         per_sm <= 0)
       per_sm = 8;
     const unsigned grid = static_cast<unsigned>(std::max(sms, 1) * per_sm);
-    kernel<<<grid, block, 0, s>>>(b, L.G, setup, flag, counts, offsets, bins, winner, misc, L.n_tiles * wpt, vis,
+    launch_after(kernel, grid, block, s, b, L.G, setup, flag, counts, offsets, bins, winner, misc, L.n_tiles * wpt, vis,
                                   keys, clear);
   };
   if (wpt == 2) {  // the warp's sub-tile is (tw, th / 2)
@@ -1481,18 +1487,18 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
     if (b.total_setup > 0) {
       const unsigned grid = L.fmap_blocks;
       if (keys)
-        setup_bin_kernel<true><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, flag, counts, keys, small_area,
+        launch_after(setup_bin_kernel<true>, grid, kSetupThreads, s, b, L.G, fmap, setup, flag, counts, keys, small_area,
                                                              binned, misc + 6);
       else
-        setup_bin_kernel<false><<<grid, kSetupThreads, 0, s>>>(b, L.G, fmap, setup, flag, counts, nullptr, 0,
+        launch_after(setup_bin_kernel<false>, grid, kSetupThreads, s, b, L.G, fmap, setup, flag, counts, nullptr, 0,
                                                               binned, misc + 6);
       prof.mark("setup_bin_kernel");
-      offsets_kernel<<<static_cast<unsigned>(L.n_scan_blocks), 256, 0, s>>>(
+      launch_after(offsets_kernel, static_cast<unsigned>(L.n_scan_blocks), 256, s,
           counts, offsets, L.n_tiles, L.bin_capacity, misc + 1, reinterpret_cast<unsigned long long*>(misc + 2));
       prof.mark("offsets_kernel");
       // the list's length is on the device: a full wave of blocks strides over it
       const unsigned sgrid = static_cast<unsigned>(sms * (2048 / kSetupThreads));
-      scatter_kernel<<<std::min(sgrid, grid), kSetupThreads, 0, s>>>(L.G, binned, misc + 6, offsets, cursors, bins);
+      launch_after(scatter_kernel, std::min(sgrid, grid), kSetupThreads, s, L.G, binned, misc + 6, offsets, cursors, bins);
       prof.mark("scatter_kernel");
     }
     if (b.total_pixels > 0) {
@@ -1521,10 +1527,10 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
         const unsigned split = warps_per_entry(L.fmap_blocks, sms);
         const unsigned vgrid = (L.fmap_blocks * split + kFaceThreads / 32 - 1) / (kFaceThreads / 32);
         if (L.small_path)
-          face_varyings_kernel<setup_rows(true)><<<vgrid, kFaceThreads, 0, s>>>(b, fmap, L.fmap_blocks, split, vis, fvar,
+          launch_after(face_varyings_kernel<setup_rows(true)>, vgrid, kFaceThreads, s, b, fmap, L.fmap_blocks, split, vis, fvar,
                                                                               L.vstride);
         else
-          face_varyings_kernel<setup_rows(false)><<<vgrid, kFaceThreads, 0, s>>>(b, fmap, L.fmap_blocks, split, vis, fvar,
+          launch_after(face_varyings_kernel<setup_rows(false)>, vgrid, kFaceThreads, s, b, fmap, L.fmap_blocks, split, vis, fvar,
                                                                               L.vstride);
         prof.mark("face_varyings_kernel");
       }
@@ -1534,10 +1540,11 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
     const int64_t max_px = static_cast<int64_t>(b.max_width) * b.max_height;
     const dim3 sgrid(static_cast<unsigned>((max_px + 255) / 256), static_cast<unsigned>(b.n_jobs));
     const float* fv = pre ? fvar : nullptr;
-    if (b.max_layers > 0)
-      tiled_shade_kernel<true><<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, fv, L.vstride, clear);
-    else
-      tiled_shade_kernel<false><<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, fv, L.vstride, clear);
+    const auto kernel = b.max_layers > 0 ? tiled_shade_kernel<true> : tiled_shade_kernel<false>;
+    if (cover)
+      launch_after(kernel, sgrid, 256, s, b, setup, winner, b.total_setup > 0, fv, L.vstride, clear);
+    else  // the caller's stream may have waited for another pass
+      kernel<<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, fv, L.vstride, clear);
     prof.mark("tiled_shade_kernel");
   }
   const cudaError_t e = cudaGetLastError();
