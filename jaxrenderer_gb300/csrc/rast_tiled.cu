@@ -761,8 +761,8 @@ __device__ __forceinline__ bool edge_misses_tile(float ea, float eb, float ec, f
 // rectangle (from the set-up) cut to the warp's pixels is usually a few
 // pixels; entries of at most pair_max() such pixels are not tested against
 // every pixel of the tile but as (entry, pixel) pairs spread over the lanes,
-// 32 per round (a lane finds its entry by binary search over the warp's
-// prefix sums), each folding its key into the pixel's minimum in shared
+// 32 per round (a lane finds its entry from the round's mask of first pairs),
+// each folding its key into the pixel's minimum in shared
 // memory with a 64-bit atomicMin.  Larger entries take the dense loop (each
 // lane its own pixels, keys in registers).  The minimum of packed keys does
 // not depend on the order, and both paths evaluate the same operations, so
@@ -809,13 +809,16 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
   constexpr int PPL = TW * TH / 32;
   constexpr bool kPairs = kL == 1 && !kTies;
   constexpr int kPW = kPairs ? kRasterWarps : 1;  // pair-path arrays only where used
+  constexpr int kNoPair = 0x40000000;             // past every round
   __shared__ float4 s_rec[kRasterWarps][kStage][3];
   __shared__ int s_id[kRasterWarps][kStage];
+  __shared__ int4 s_pinf[kPW][kPairs ? kStage : 1];  // per pair entry: first pair, rectangle, reciprocal width
   __shared__ unsigned long long s_best[kPW][kPairs ? TW * TH : 1];  // pixel (li, lj) at li * TH + lj
   __shared__ float s_x[kPW][kPairs ? TW : 1], s_y[kPW][kPairs ? TH : 1];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   float4 (*rec)[3] = s_rec[warp];
   int* ids = s_id[warp];
+  int4* pinf = s_pinf[kPairs ? warp : 0];
   unsigned long long* sbest = s_best[kPairs ? warp : 0];
   float* tx_ndc = s_x[kPairs ? warp : 0];
   float* ty_ndc = s_y[kPairs ? warp : 0];
@@ -997,7 +1000,9 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
         }
         ptotal = __shfl_sync(0xffffffffu, pincl, 31);
       }
-      const int pexcl = pincl - (pair ? cnt : 0);
+      if (kPairs && pair) pinf[m + __popc(pmask & lanemask_lt())] = make_int4(pincl - cnt, pinfo, __float_as_int(prcp), 0);
+      int ppos = pair ? pincl - cnt : kNoPair;  // the entry's first pair, from the round's first
+      int pbefore = m - 1;                      // slot of the last entry begun before the round
       __syncwarp();
       if (base + kStage >= n) grab();  // the last chunk: the next tile's atomic overlaps its tests
       // prefetch the next chunk while this one is tested
@@ -1027,26 +1032,23 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
       }
       if (kPairs) {
         for (int pb = 0; pb < ptotal; pb += 32) {
+          // entries whose pairs begin in this round, a bit each at their
+          // first pair: a pair's entry is the last one begun at or before it
+          const unsigned begun = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(ppos) < 32u ? 1u << ppos : 0u);
+          const int slot = pbefore + __popc(begun & (lanemask_lt() << 1 | 1u));
+          pbefore += __popc(begun);
+          ppos -= 32;
           const int pk = pb + lane;
-          int owner = 0;  // lanes whose pairs all precede pair pk
-#pragma unroll
-          for (int step = 16; step > 0; step >>= 1) {
-            const int v = __shfl_sync(0xffffffffu, pincl, owner + step - 1);
-            if (v <= pk) owner += step;
-          }
-          const int o_excl = __shfl_sync(0xffffffffu, pexcl, owner);
-          const int o_info = __shfl_sync(0xffffffffu, pinfo, owner);
-          const float o_rcp = __shfl_sync(0xffffffffu, prcp, owner);
           if (pk < ptotal) {
             // pair -> pixel of the owner's rectangle, row-major over its
-            // width w (w <= 32 and pk - o_excl < TW * TH: the rounded
-            // quotient (k + 1/2) / w stays more than 1/64 from an integer)
-            const int k = pk - o_excl;
-            const int w = o_info >> 16;
-            const int r = __float2int_rz((static_cast<float>(k) + 0.5f) * o_rcp);
-            const int li = min((o_info & 0xff) + (k - r * w), TW - 1);
-            const int lj = min(((o_info >> 8) & 0xff) + r, TH - 1);
-            const int slot = m + __popc(pmask & ((1u << owner) - 1u));
+            // width w (w <= 32 and k < TW * TH: the rounded quotient (k +
+            // 1/2) / w stays more than 1/64 from an integer)
+            const int4 o = pinf[slot];
+            const int k = pk - o.x;
+            const int w = o.y >> 16;
+            const int r = __float2int_rz((static_cast<float>(k) + 0.5f) * __int_as_float(o.z));
+            const int li = min((o.y & 0xff) + (k - r * w), TW - 1);
+            const int lj = min(((o.y >> 8) & 0xff) + r, TH - 1);
             const float px = tx_ndc[li], py = ty_ndc[lj];
             const float4 a = rec[slot][0], b = rec[slot][1], cz = rec[slot][2];
             const float c0 = (px * a.x + py * a.w) + b.z;
