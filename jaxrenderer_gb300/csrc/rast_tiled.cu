@@ -414,6 +414,56 @@ __device__ __forceinline__ void warp_tiles(int tx0, int ty0, int tx1, int ty1, i
   }
 }
 
+// warp_tiles with the rectangles staged in shared memory: the lanes with tiles stage their rectangle in slots numbered in
+// lane order (put(slot, rectangle) / get(slot): the warp's shared memory); a
+// pair's slot is the last one whose first pair lies at or before it, found
+// from the mask of first pairs in the round (one OR reduction where warp_tiles
+// takes nine shuffles: the scatter of 4096 brax-like scenes, both passes, 169
+// -> 139 us; the set-up, held to 40 registers, spills more and loses what the
+// search gains, 1,024 -> 1,058 us).  fn(slot,
+// tile index within the job, valid) runs on every lane each round; valid is
+// false past the last pair.  All 32 lanes must call.
+template <class Put, class Get, class Fn>
+__device__ __forceinline__ void warp_tiles_staged(int tx0, int ty0, int tx1, int ty1, int tiles_x, Put&& put, Get&& get, Fn&& fn) {
+  const int lane = threadIdx.x & 31;
+  const int w = tx1 - tx0 + 1;
+  const int n = (tx0 <= tx1 && ty0 <= ty1) ? w * (ty1 - ty0 + 1) : 0;
+  int incl = n;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    if (lane >= d) incl += v;
+  }
+  const int excl = incl - n;
+  const int total = __shfl_sync(0xffffffffu, incl, 31);
+  const unsigned have = __ballot_sync(0xffffffffu, n > 0);
+  // pair -> row of its rectangle by the reciprocal width: the quotient (k +
+  // 1/2) / w is at least 1/(2w) from an integer and its error below 2^-21 n / w
+  if (n > 0)
+    put(__popc(have & lanemask_lt()),
+        make_int4(excl, tx0 | (ty0 << 16), w, n < (1 << 20) ? __float_as_int(__frcp_rn(static_cast<float>(w))) : 0));
+  int first = n > 0 ? excl : 0x40000000;  // this lane's first pair, from the round's first
+  int before = -1;                        // last slot begun before the round
+  __syncwarp();
+  for (int base = 0; base < total; base += 32) {
+    const unsigned begun = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(first) < 32u ? 1u << first : 0u);
+    const int slot = before + __popc(begun & (lanemask_lt() << 1 | 1u));
+    before += __popc(begun);
+    first -= 32;
+    const int k = base + lane;
+    const bool valid = k < total;
+    int tile = 0;
+    if (valid) {
+      const int4 o = get(slot);
+      const int local = k - o.x;
+      const int r = o.w ? __float2int_rz((static_cast<float>(local) + 0.5f) * __int_as_float(o.w)) : local / o.z;
+      tile = ((o.y >> 16) + r) * tiles_x + (o.y & 0xffff) + (local - r * o.z);
+    }
+    fn(slot, tile, valid);
+  }
+  __syncwarp();  // every lane is done with the staged rectangles
+}
+
 // Phase 1, one thread per face and round: clip positions, determinant,
 // keep/front flags and the off-screen test.  The faces that remain
 // (candidates: kept, front-facing and not known to miss the screen) and face
@@ -707,6 +757,10 @@ scatter_kernel(Geometry G, const int4* __restrict__ binned, const unsigned int* 
   constexpr unsigned kWarps = kSetupThreads / 32;
   const unsigned warps = gridDim.x * kWarps, wid = blockIdx.x * kWarps + (threadIdx.x >> 5);
   const unsigned per_warp = max(1u, min(32u, (n + warps - 1) / warps));  // listed faces per warp
+  __shared__ int4 s_rect[kWarps][32];
+  __shared__ int2 s_id[kWarps][32];  // job's first tile, face
+  int4* rect = s_rect[threadIdx.x >> 5];
+  int2* ids = s_id[threadIdx.x >> 5];
   for (unsigned base = wid * per_warp; base < n; base += warps * per_warp) {
     const unsigned e = base + lane;
     int jid = 0, fq = 0, tx0 = 1, ty0 = 1, tx1 = 0, ty1 = 0;
@@ -720,17 +774,22 @@ scatter_kernel(Geometry G, const int4* __restrict__ binned, const unsigned int* 
       tx1 = static_cast<int>((hi & 0xffffu) >> G.tws);
       ty1 = static_cast<int>((hi >> 16) >> G.ths);
     }
-    warp_tiles(tx0, ty0, tx1, ty1, G.tiles_x, [&](int owner, int tile, bool valid) {
-      const int64_t gt = static_cast<int64_t>(__shfl_sync(0xffffffffu, jid, owner)) * G.tiles_per_job + tile;
+    auto put = [&](int slot, int4 r) {
+      rect[slot] = r;
+      ids[slot] = make_int2(static_cast<int>(static_cast<unsigned>(jid) * static_cast<unsigned>(G.tiles_per_job)), fq);
+    };
+    warp_tiles_staged(tx0, ty0, tx1, ty1, G.tiles_x, put, [&](int slot) { return rect[slot]; },
+                      [&](int slot, int tile, bool valid) {
+      const int2 id = valid ? ids[slot] : make_int2(0, 0);
+      const unsigned gt = static_cast<unsigned>(id.x) + static_cast<unsigned>(tile);  // work units are 32-bit
       const uint32_t o = valid ? offsets[gt] : kOverflow;
       const bool write = !(o & kOverflow);
-      const unsigned peers = __match_any_sync(0xffffffffu, write ? gt : -1ll);
+      const unsigned peers = __match_any_sync(0xffffffffu, write ? gt : 0xffffffffu);
       const int leader = __ffs(peers) - 1;
-      uint32_t slot = 0;
-      if (write && lane == leader) slot = atomicAdd(cursors + gt, static_cast<unsigned>(__popc(peers)));
-      slot = __shfl_sync(0xffffffffu, slot, leader) + __popc(peers & lanemask_lt());
-      const int fid = __shfl_sync(0xffffffffu, fq, owner);
-      if (write) bins[static_cast<int64_t>(o) + slot] = fid;
+      uint32_t at = 0;
+      if (write && lane == leader) at = atomicAdd(cursors + gt, static_cast<unsigned>(__popc(peers)));
+      at = __shfl_sync(0xffffffffu, at, leader) + __popc(peers & lanemask_lt());
+      if (write) bins[static_cast<int64_t>(o) + at] = id.y;
     });
   }
 }
