@@ -37,7 +37,7 @@
 namespace rast {
 namespace bwd {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;  // of the pixel, mark and begin kernels
 // The per-face and per-vertex kernels: a few percent of the rows are visible,
 // so each warp takes one block-map entry of kRows rows, lists the marked ones
 // (list_marked) and works through them, one per lane.
@@ -749,15 +749,18 @@ __device__ __forceinline__ void fragment_bwd(const RastJob& J, const RastPools& 
   normalise3_bwd(n, nrmn, gn, g_interp);
 }
 
-// Single-shader variants at 4 blocks per SM (64 registers, some spills:
-// more resident warps hide the fragment backward's dependency chains
-// better); the mixed-shader variants at 3 (80 registers: the mixed 1024-scene
-// backward 5.36 -> 4.59 ms, from 2 blocks at 128 registers).
+// Blocks of 128 threads: a block's warps wait for one another at the job load
+// and the parameter reduction, and four wait less than eight (1024 brax-like
+// scenes 595 -> 573 us with seven blocks per SM; 64 threads 638).  Blocks per
+// SM: more resident warps hide the fragment backward's dependency chains until
+// the spills cost more.  The reflection shaders take seven (72 registers; eight
+// 598 us, nine 627), the lighter ones eight (256 phong spheres 219 us; seven
+// 237), phong_darboux and the mixed-shader variants six (80 registers).
 template <int SH>
 __host__ __device__ constexpr int pixel_min_blocks() {
-  return (SH == RAST_SHADER_PHONG_REFLECTION || SH == RAST_SHADER_PHONG_REFLECTION_SHADOW ||
-          SH == RAST_SHADER_PHONG || SH == RAST_SHADER_GOURAUD || SH == RAST_SHADER_GOURAUD_TEXTURE ||
-          SH == RAST_SHADER_DEPTH) ? 4 : 3;
+  return (SH == RAST_SHADER_PHONG_REFLECTION || SH == RAST_SHADER_PHONG_REFLECTION_SHADOW) ? 7
+       : (SH == RAST_SHADER_PHONG || SH == RAST_SHADER_GOURAUD || SH == RAST_SHADER_GOURAUD_TEXTURE ||
+          SH == RAST_SHADER_DEPTH) ? 8 : 6;
 }
 
 // dL/dcanvas: read from a gradient image, or formed from the rendered canvas
