@@ -209,6 +209,7 @@ class _RenderFunction(torch.autograd.Function):
         ctx.names = names
         ctx.shapes = [t.shape for t in tensors]
         ctx.dtypes = [t.dtype for t in tensors]
+        ctx.set_materialize_grads(False)
         db._generation += 1
         ctx.generation = db._generation
         return out.canvas.clone(), out.zbuffer.clone()
@@ -218,10 +219,18 @@ class _RenderFunction(torch.autograd.Function):
         db = ctx.db
         if db._generation != ctx.generation:
             raise RuntimeError("DifferentiableBatch was re-rendered before backward of an earlier render")
-        g = db.runner.backward(g_canvas, g_zbuffer)
+        # the gradients of the given inputs only: the kernels skip the others
+        runner = db.runner
+        g = {k: torch.zeros_like(runner.pools[k]) for k, w in zip(ctx.names, ctx.needs_input_grad[2:])
+             if w and k in POOL_PARAMS}
+        if any(w and k in PARAM_COLUMNS for k, w in zip(ctx.names, ctx.needs_input_grad[2:])):
+            g["job_params"] = torch.zeros((runner.sb.n_scenes, _lib.NPARAM), dtype=torch.float32, device=runner.sb.device)
+        runner.backward(g_canvas, g_zbuffer, out=g, accumulate=True)
         grads = []
-        for name, shape, dt in zip(ctx.names, ctx.shapes, ctx.dtypes):
-            if name in POOL_PARAMS:
+        for name, shape, dt, w in zip(ctx.names, ctx.shapes, ctx.dtypes, ctx.needs_input_grad[2:]):
+            if not w:
+                grads.append(None)
+            elif name in POOL_PARAMS:
                 grads.append(g[name].reshape(shape).to(dt))
             else:
                 col, width = PARAM_COLUMNS[name]
