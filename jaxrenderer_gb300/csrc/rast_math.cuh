@@ -74,9 +74,8 @@ __device__ __forceinline__ int gather_clamp(int idx, int size) {
 // Depth -> monotone uint32: NaN first (it wins argmin), -0 == +0.
 __device__ __forceinline__ uint32_t depth_order(float z) {
   if (z != z) return 0u;
-  if (z == 0.0f) z = 0.0f;
-  const uint32_t b = __float_as_uint(z);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+  const uint32_t b = __float_as_uint(z + 0.0f);  // -0 + 0 = +0
+  return b ^ (static_cast<uint32_t>(static_cast<int32_t>(b) >> 31) | 0x80000000u);  // ~b below zero, b + 2^31 above
 }
 
 // Packed chooser key: (ordered depth << 32) | primitive id.  The minimum

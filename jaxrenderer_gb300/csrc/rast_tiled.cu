@@ -795,17 +795,17 @@ scatter_kernel(Geometry G, const int4* __restrict__ binned, const unsigned int* 
 }
 
 // True when edge function (x ea + y eb) + ec is negative at every pixel of
-// the tile [xa, xb] x [ya, yb] (NDC of its first and last pixel centres)
+// the rectangle [xl, xh] x [yl, yh] (NDC of its outermost pixel centres)
 // whatever the rounding of the per-pixel evaluation: its maximum over the
-// rectangle, max(xa ea, xb ea) + max(ya eb, yb eb) + ec, plus a margin of
-// 16 u (X |ea| + Y |eb| + |ec|) (X, Y: the largest |x|, |y| of the tile;
-// u = 2^-24; the per-pixel and the bound's own rounding are each below
-// 3.1 u times that sum) is below zero.  NaN anywhere gives false.
-__device__ __forceinline__ bool edge_misses_tile(float ea, float eb, float ec, float xa, float xb, float ya, float yb,
+// rectangle, ea >= 0 taking xh and so on, plus a margin of 16 u (X |ea| + Y
+// |eb| + |ec|) (X, Y: the largest |x|, |y|; u = 2^-24; the per-pixel rounding
+// is below 3.1 u times that sum, the bound's own below 2 u) is below zero.
+// NaN anywhere gives false.
+__device__ __forceinline__ bool edge_misses_tile(float ea, float eb, float ec, float xl, float xh, float yl, float yh,
                                                  float X, float Y) {
-  const float bound = (fmaxf(xa * ea, xb * ea) + fmaxf(ya * eb, yb * eb)) + ec;
-  const float margin = 16.0f * 5.9604645e-08f * ((X * fabsf(ea) + Y * fabsf(eb)) + fabsf(ec)) + 1e-30f;
-  return bound + margin < 0.0f;
+  const float bound = __fmaf_rn(ea >= 0.0f ? xh : xl, ea, __fmaf_rn(eb >= 0.0f ? yh : yl, eb, ec));
+  const float sum = __fmaf_rn(X, fabsf(ea), __fmaf_rn(Y, fabsf(eb), fabsf(ec)));
+  return __fmaf_rn(16.0f * 5.9604645e-08f, sum, bound) < -1e-30f;
 }
 
 // Persistent warps: each takes one tile (of any job) at a time.  Lane l owns
@@ -826,17 +826,17 @@ __device__ __forceinline__ bool edge_misses_tile(float ea, float eb, float ec, f
 // lane its own pixels, keys in registers).  The minimum of packed keys does
 // not depend on the order, and both paths evaluate the same operations, so
 // the results are those of the dense loop alone.
-// Blocks per SM: the pair-path variants of at most 128 pixels take eight
-// (64 registers; ten at 48 registers spilled in the pair loop: main 16x8
-// 0.58 -> 0.64 ms on the 4096-scene brax-like batch).  The near-tie
-// counting one-slot variants take ten (48 registers): more resident warps
-// beat their few spills (16x8: 1.02 -> 0.88 ms, 8x8: 1.03 -> 1.01 ms before
-// the pair path; 12 and 16 blocks measured slower).  The layered variants
-// of at most 64 pixels take eight (64 registers: 1.32 -> 1.18 ms with 4
-// layers).  The others keep the compiler's choice (0: no minimum).
+// Blocks per SM: the pair-path variants of at most 128 pixels take nine (56
+// registers; 4096 brax-like scenes, shadow + main: 743 + 505 us, 762 + 513 at
+// eight, 811 + 567 at ten, which spill in the pair loop).  The near-tie
+// counting one-slot variants take ten (48 registers): more resident warps beat
+// their few spills (16x8: 1.02 -> 0.88 ms, 8x8: 1.03 -> 1.01 ms before the
+// pair path; 12 and 16 blocks measured slower).  The layered variants of at
+// most 64 pixels take eight (64 registers: 1.32 -> 1.18 ms with 4 layers).
+// The others keep the compiler's choice (0: no minimum).
 template <int TW, int TH, int kL, bool kPairs>
 __host__ __device__ constexpr int raster_min_blocks() {
-  return kPairs ? (TW * TH <= 128 ? 8 : 0) : (kL == 1 && TW * TH <= 128) ? 10 : (TW * TH <= 64 ? 8 : 0);
+  return kPairs ? (TW * TH <= 128 ? 9 : 0) : (kL == 1 && TW * TH <= 128) ? 10 : (TW * TH <= 64 ? 8 : 0);
 }
 
 // Largest (entry, pixel) pair count of an entry on the pair path: about
@@ -960,7 +960,7 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
     constexpr int LPC = 32 / TH;
     const int pj = y0 + lane % TH;
     float y;
-    float x[PPL], best_z[PPL];
+    float x[PPL];
     if (kPairs) {
       // the pixels' NDC quotients, once per tile: tx_ndc[li] for pixel
       // x0 + li, ty_ndc[lj] for y0 + lj
@@ -986,17 +986,17 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
     const int lxe = min(TW - 1, W - 1 - x0), lye = min(TH - 1, H - 1 - y0);  // last pixel inside the job
     float xa, xb, ya, yb;
     if (kPairs) {
-      xa = tx_ndc[0], xb = tx_ndc[lxe], ya = ty_ndc[0], yb = ty_ndc[lye];
+      xa = xb = ya = yb = 0.0f;  // each entry's own rectangle is tested
     } else {
       xa = (static_cast<float>(x0) - ox) / sx;
       xb = (static_cast<float>(x0 + lxe) - ox) / sx;
       ya = (static_cast<float>(y0) - oy) / sy;
       yb = (static_cast<float>(y0 + lye) - oy) / sy;
     }
+    const float xl = fminf(xa, xb), xh = fmaxf(xa, xb), yl = fminf(ya, yb), yh = fmaxf(ya, yb);
     const float XM = fmaxf(fabsf(xa), fabsf(xb)), YM = fmaxf(fabsf(ya), fabsf(yb));
     unsigned long long best[PPL][kL];
     uint32_t second[PPL];
-    unsigned z_known = 0;  // bit q: best_z[q] holds the depth of best[q] (set by this kernel's tests)
 #pragma unroll
     for (int q = 0; q < PPL; ++q) {
       const int pi = x0 + q * LPC + lane / TH;
@@ -1004,7 +1004,6 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
       best[q][0] = (kKeys && pi < W && pj < H) ? keys[J.pixel_begin + static_cast<int64_t>(pi) * H + pj] : kEmptyKey;
 #pragma unroll
       for (int l = 1; l < kL; ++l) best[q][l] = kEmptyKey;
-      best_z[q] = 0.0f;
       second[q] = 0xffffffffu;
     }
     for (int base = 0; base < n; base += kStage) {
@@ -1022,18 +1021,19 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
         if (take) {
           const float ra = tx_ndc[lx0], rb = tx_ndc[lx1], sa = ty_ndc[ly0], sb = ty_ndc[ly1];
           const float RX = fmaxf(fabsf(ra), fabsf(rb)), RY = fmaxf(fabsf(sa), fabsf(sb));
-          take = !(edge_misses_tile(n0.x, n0.w, n1.z, ra, rb, sa, sb, RX, RY) ||
-                   edge_misses_tile(n0.y, n1.x, n1.w, ra, rb, sa, sb, RX, RY) ||
-                   edge_misses_tile(n0.z, n1.y, n2.x, ra, rb, sa, sb, RX, RY));
+          const float rl = fminf(ra, rb), rh = fmaxf(ra, rb), sl = fminf(sa, sb), sh = fmaxf(sa, sb);
+          take = !(edge_misses_tile(n0.x, n0.w, n1.z, rl, rh, sl, sh, RX, RY) ||
+                   edge_misses_tile(n0.y, n1.x, n1.w, rl, rh, sl, sh, RX, RY) ||
+                   edge_misses_tile(n0.z, n1.y, n2.x, rl, rh, sl, sh, RX, RY));
           const int w = lx1 - lx0 + 1;
           cnt = w * (ly1 - ly0 + 1);
           pinfo = lx0 | (ly0 << 8) | (w << 16);
           prcp = __frcp_rn(static_cast<float>(w));
         }
       } else if (take) {
-        take = !(edge_misses_tile(n0.x, n0.w, n1.z, xa, xb, ya, yb, XM, YM) ||
-                 edge_misses_tile(n0.y, n1.x, n1.w, xa, xb, ya, yb, XM, YM) ||
-                 edge_misses_tile(n0.z, n1.y, n2.x, xa, xb, ya, yb, XM, YM));
+        take = !(edge_misses_tile(n0.x, n0.w, n1.z, xl, xh, yl, yh, XM, YM) ||
+                 edge_misses_tile(n0.y, n1.x, n1.w, xl, xh, yl, yh, XM, YM) ||
+                 edge_misses_tile(n0.z, n1.y, n2.x, xl, xh, yl, yh, XM, YM));
       }
       const bool pair = kPairs && take && cnt <= pair_max<TW, TH>();
       const bool dense = take && !pair;
@@ -1078,13 +1078,7 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
           if (all_nonneg(c0, c1, c2)) {  // staged entries are candidates (id >= 0)
             const float z = ((c0 * cz.y + c1 * cz.z) + c2 * cz.w) * vp22 + vp23;
             const unsigned long long key = pack_key(z, ids[e]);
-            if (key < best[q][0]) {
-              if (kTies) second[q] = min(second[q], static_cast<uint32_t>(best[q][0] >> 32));
-              best_z[q] = z;
-              z_known |= 1u << q;
-            } else if (kTies) {
-              second[q] = min(second[q], static_cast<uint32_t>(key >> 32));
-            }
+            if (kTies) second[q] = min(second[q], static_cast<uint32_t>((key < best[q][0] ? best[q][0] : key) >> 32));
             insert_key<kL>(best[q], key);
           }
         }
@@ -1129,10 +1123,7 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
 #pragma unroll
       for (int q = 0; q < PPL; ++q) {
         const unsigned long long k = sbest[q * 32 + lane];
-        if (k < best[q][0]) {
-          best[q][0] = k;
-          z_known &= ~(1u << q);
-        }
+        if (k < best[q][0]) best[q][0] = k;
       }
       __syncwarp();  // every lane has read its minima before the next tile's reset
     }
@@ -1185,11 +1176,11 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
         // depth, so the pixel resolves here (same operations as
         // resolve_pixel): the winner's depth, or primitive 0's chooser fallback.
         bool keep = found;
-        float z = best_z[q];
+        float z = 0.0f;
         int prim = found ? static_cast<int>(best[q][0] & 0xffffffffu) : 0;
-        if ((kKeys || kPairs) && found && !(z_known & (1u << q)) && !depth_of_order(o1, &z)) {
-          // the winner came from a key alone and its depth is NaN or +-0:
-          // its depth again, with the same operations
+        if (found && !depth_of_order(o1, &z)) {
+          // the winner's depth is NaN or +-0, whose bits its key does not
+          // hold: its depth again, with the same operations
           const float4* r = jrec + static_cast<int64_t>(prim) * 4;
           const float4 a = __ldg(r), b = __ldg(r + 1), cz = __ldg(r + 2);
           const float c0 = (x[q] * a.x + y * a.w) + b.z;

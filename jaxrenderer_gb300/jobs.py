@@ -176,9 +176,12 @@ class _Pool:
 
     def host_bytes(self) -> Optional[int]:
         """Bytes of the pool when every part is a host array, else None."""
-        if not self.parts or any(isinstance(p, torch.Tensor) for p in self.parts):
-            return None
-        return 4 * sum(int(np.size(p)) for p in self.parts)
+        n = 0
+        for p in self.parts:
+            if isinstance(p, torch.Tensor):
+                return None
+            n += 4 * int(np.size(p))
+        return n if self.parts else None
 
     def host_into(self, buf: np.ndarray) -> None:
         """Write the parts into `buf` (the pool's bytes)."""
@@ -210,24 +213,26 @@ ONE_COPY_BYTES = 1 << 20
 def _upload(pools, extra: bytes, device):
     """({name: device tensor}, device copy of `extra`): the pools whose parts
     are all host arrays as slices of one buffer when they are small."""
-    sizes = {k: n for k, n in ((k, p.host_bytes()) for k, p in pools.items()) if n}
-    step = lambda n: -(-n // 256) * 256  # noqa: E731
-    total = step(len(extra)) + sum(map(step, sizes.values()))
-    if total > ONE_COPY_BYTES:
-        sizes, total = {}, len(extra)
-    host = np.empty(total, np.uint8)
-    host[: len(extra)] = np.frombuffer(extra, np.uint8)
-    at = {}
-    end = step(len(extra))
-    for k, n in sizes.items():
-        pools[k].host_into(host[end : end + n])
-        at[k] = end
-        end += step(n)
-    dev = torch.from_numpy(host).to(device)
-    out = {k: dev[a : a + sizes[k]].view(pools[k].dtype) for k, a in at.items()}
+    out, packed, end = {}, [], -(-len(extra) // 256) * 256
     for k, p in pools.items():
-        if k not in out and p.parts:
+        if p.parts:
+            n = p.host_bytes()
+            if n:
+                packed.append((k, p, end, n))
+                end += -(-n // 256) * 256
+            else:
+                out[k] = p.tensor(device)
+    if not packed or end > ONE_COPY_BYTES:
+        for k, p, _, _ in packed:
             out[k] = p.tensor(device)
+        return out, torch.frombuffer(bytearray(extra), dtype=torch.uint8).to(device)
+    host = np.empty(end, np.uint8)
+    host[: len(extra)] = np.frombuffer(extra, np.uint8)
+    for _, p, at, n in packed:
+        p.host_into(host[at : at + n])
+    dev = torch.from_numpy(host).to(device)
+    for k, p, at, n in packed:
+        out[k] = dev[at : at + n].view(p.dtype)
     return out, dev[: len(extra)]
 
 
