@@ -223,8 +223,9 @@ inline unsigned warps_per_entry(unsigned entries, int sms) {
 __device__ __forceinline__ void fill_words(void* p, size_t bytes, unsigned value) {
   uint4* w = static_cast<uint4*>(p);
   const size_t n = (bytes + 15) / 16;
-  for (size_t k = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; k < n;
-       k += static_cast<size_t>(gridDim.x) * blockDim.x)
+  const size_t blocks = static_cast<size_t>(gridDim.x) * gridDim.y;
+  for (size_t k = (static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; k < n;
+       k += blocks * blockDim.x)
     w[k] = make_uint4(value, value, value, value);
 }
 
@@ -250,14 +251,14 @@ struct Same {
 // off a small batch (16 scenes: 67 -> 64 us a replay) and nothing from large
 // ones.  Not for the first kernel after a stream waits for an event.
 template <class... Args>
-inline void launch_after(void (*kernel)(Args...), dim3 grid, unsigned block, cudaStream_t s,
+inline void launch_after(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t s,
                          typename Same<Args>::type... args) {
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
-  cfg.blockDim = dim3(block);
+  cfg.blockDim = block;
   cfg.stream = s;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;

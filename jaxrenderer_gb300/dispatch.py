@@ -22,8 +22,9 @@ from . import _lib
 from . import jobs as _jobs
 
 FORMS = ("auto", "plain", "tiled")
-# ~1e8 pixel-triangle pairs: about where the plain scan's time (at ~1.3e12
-# pairs/s on a GB300) passes the tiled form's fixed launch cost
+# ~1.3e8 pixel-triangle pairs: the plain scan (5e12 pairs/s on a GB300 for closed
+# meshes, half of whose faces look away) then takes as long as the tiled form's
+# chain of launches; a 254x152 pass of 3.5e8 pairs takes 87 against 62 us
 TILED_MIN_PAIRS = 1 << 27
 # the tiled form's per-face pixel rectangles are 16-bit
 TILED_MAX_SIDE = 65535
