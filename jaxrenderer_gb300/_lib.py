@@ -285,8 +285,8 @@ def check(status: int, where: str) -> None:
 
 
 def as_c_floats(dst, values) -> None:
-    for k, v in enumerate(values):
-        dst[k] = float(v)
+    v = [float(x) for x in (values.tolist() if hasattr(values, "tolist") else values)]
+    dst[: len(v)] = v
 
 
 __all__ = [

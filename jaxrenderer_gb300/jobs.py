@@ -9,6 +9,7 @@ per-shader extraction is `job_from_extra`.
 from __future__ import annotations
 
 import ctypes
+import math
 from dataclasses import dataclass, field
 from typing import Any, List, Optional, Sequence
 
@@ -169,7 +170,7 @@ class _Pool:
         if x is None:
             return 0
         begin = self.rows
-        n = int(np.prod(tuple(x.shape))) // self.row
+        n = math.prod(x.shape) // self.row
         self.parts.append(x)
         self.rows += n
         return begin
