@@ -24,43 +24,6 @@ constexpr int kCandidate = kKeep | kFront;
 
 inline size_t align256(size_t x) { return (x + 255) & ~static_cast<size_t>(255); }
 
-// Last job whose *_begin <= row (jobs are laid out in increasing order).
-template <typename Get>
-__device__ __forceinline__ int find_job(const RastJob* jobs, int n, int64_t row, Get get) {
-  int lo = 0, hi = n;  // answer in [lo, hi)
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (get(jobs[mid]) <= row) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-__device__ __forceinline__ int find_job_by_vout(const RastJob* jobs, int n, int64_t row) {
-  return find_job(jobs, n, row, [](const RastJob& j) { return j.vout_begin; });
-}
-__device__ __forceinline__ int find_job_by_setup(const RastJob* jobs, int n, int64_t row) {
-  return find_job(jobs, n, row, [](const RastJob& j) { return j.setup_begin; });
-}
-
-// Job owning rows [row0, row0 + blockDim.x) of a flat per-row launch when
-// they all belong to one job (the common case: one binary search per block,
-// by thread 0), else -1 (each thread then searches for its own row).  Every
-// thread of the block must call it.
-template <typename Begin, typename Count>
-__device__ __forceinline__ int block_uniform_job(const RastJob* jobs, int n, int64_t row0, int64_t total,
-                                                 Begin begin, Count count, int* s_job) {
-  if (threadIdx.x == 0) {
-    int j = -1;
-    if (row0 < total) {
-      const int64_t last = min(row0 + static_cast<int64_t>(blockDim.x) - 1, total - 1);
-      const int f = find_job(jobs, n, row0, begin);
-      if (begin(jobs[f]) + count(jobs[f]) > last) j = f;
-    }
-    *s_job = j;
-  }
-  __syncthreads();
-  return *s_job;
-}
-
 // PerPrimitive.create (pipeline.py:80-113) from the three clip positions.
 // Record: [inv0..3] [inv4..7] [inv8 z0 z1 z2] [det flags 0 0]; the tiled
 // form keeps the face's pixel rectangle in [3].x and [3].z and writes records
@@ -100,39 +63,6 @@ __device__ __forceinline__ void count_near_tie(unsigned long long* counter, bool
 }
 
 __device__ __forceinline__ unsigned lanemask_lt() { return (1u << (threadIdx.x & 31)) - 1u; }
-
-// Block-wide compaction: every thread offers `idx` when `flag`; the flagged
-// indices land in s_q (order unspecified) and the count is returned.  *s_n
-// must be zero and visible to the block on entry; every thread must call.
-__device__ __forceinline__ int block_queue(bool flag, int idx, int* s_q, int* s_n) {
-  const unsigned m = __ballot_sync(0xffffffffu, flag);
-  int base = 0;
-  if ((threadIdx.x & 31) == 0 && m) base = atomicAdd(s_n, __popc(m));
-  base = __shfl_sync(0xffffffffu, base, 0);
-  if (flag) s_q[base + __popc(m & lanemask_lt())] = idx;
-  __syncthreads();
-  return *s_n;
-}
-
-// block_queue over kR rows per thread: row r = threadIdx.x + k * kBlock
-// (k < kR) is offered when flag(r); the offered rows land in s_q (order
-// unspecified, room for kR * kBlock) and the count is returned.  *s_n must be
-// zero and visible to the block on entry; every thread must call.
-template <int kR, int kBlock, class Flag>
-__device__ __forceinline__ int block_queue_rows(Flag flag, int* s_q, int* s_n) {
-#pragma unroll
-  for (int k = 0; k < kR; ++k) {
-    const int r = static_cast<int>(threadIdx.x) + k * kBlock;
-    const bool f = flag(r);
-    const unsigned m = __ballot_sync(0xffffffffu, f);
-    int base = 0;
-    if ((threadIdx.x & 31) == 0 && m) base = atomicAdd(s_n, __popc(m));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (f) s_q[base + __popc(m & lanemask_lt())] = r;
-  }
-  __syncthreads();
-  return *s_n;
-}
 
 // ---- block maps: grids over the faces (or vertices) of every job with no
 // more than one empty block per job.  Job j's blocks of `per_block` items
@@ -294,14 +224,66 @@ __device__ __forceinline__ void load_job_to_shared(const RastJob* job, RastJob* 
   for (int k = tid; k < static_cast<int>(sizeof(RastJob) / 4); k += nthreads) d[k] = __ldg(src + k);
 }
 
-// Where the vertex varyings of a face come from: the vertex kernel's output
-// (plain form) or a recomputation of the vertex shader (tiled form).
-struct VaryingSource {
-  const float* var;   // per-vertex varyings (plain form), or nullptr
+// Where a shade thread reads the three corners' varyings of a face.
+
+// Plain form: the vertex kernel's rows, one per vertex.
+struct VertexRows {
+  const float* var;
   int vstride;
   int64_t vout_begin;
-  const float* fvar = nullptr;  // per-face varyings of visible faces (tiled form): 3 rows of vstride per face
-  int64_t setup_begin = 0;
+  template <int SH>
+  __device__ __forceinline__ void load(const RastJob& J, const RastPools& P, int p, float* v0, float* v1,
+                                       float* v2) const {
+    const int nv = varying_count(SH >= 0 ? SH : J.shader);
+    const int32_t* face = P.faces + (J.face_begin + p) * 3;
+    const float* r0 = var + (vout_begin + gather_clamp(face[0], J.n_verts)) * vstride;
+    const float* r1 = var + (vout_begin + gather_clamp(face[1], J.n_verts)) * vstride;
+    const float* r2 = var + (vout_begin + gather_clamp(face[2], J.n_verts)) * vstride;
+    // constant indices keep the three rows in registers
+#pragma unroll
+    for (int k = 0; k < kMaxVarying; ++k) {
+      if (k < nv) {
+        v0[k] = __ldg(r0 + k);
+        v1[k] = __ldg(r1 + k);
+        v2[k] = __ldg(r2 + k);
+      }
+    }
+  }
+};
+
+// Tiled form: one row of `floats` floats per face (face_floats of the batch's
+// largest shader) for the faces some pixel needs.  The whole float4s of the
+// rows come first, then every row's remaining floats % 4, so that rows of any
+// length read as float4 without padding.
+struct FaceRows {
+  const float4* vec;
+  const float* rest;  // vec + faces * (floats / 4)
+  int floats;
+  int64_t setup_begin;
+  template <int SH>
+  __device__ __forceinline__ void load(const RastJob& J, const RastPools&, int p, float* v0, float* v1,
+                                       float* v2) const {
+    const int n = SH >= 0 ? face_floats(SH) : floats, own = face_floats(SH >= 0 ? SH : J.shader);
+    const float4* a = vec + (setup_begin + p) * (n / 4);
+    const float* t = rest + (setup_begin + p) * (n % 4);
+    float row[kMaxFaceFloats];
+#pragma unroll
+    for (int q = 0; q < kMaxFaceFloats / 4; ++q) {
+      if (4 * q >= own) continue;
+      if (q < n / 4) {
+        const float4 x = __ldg(a + q);
+        row[4 * q] = x.x;
+        row[4 * q + 1] = x.y;
+        row[4 * q + 2] = x.z;
+        row[4 * q + 3] = x.w;
+      } else {
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+          if (c < n % 4) row[4 * q + c] = __ldg(t + c);
+      }
+    }
+    get_corners<SH>(J.shader, row, v0, v1, v2);
+  }
 };
 
 struct PixelResult {
@@ -322,11 +304,13 @@ struct Fragment {
   float colour[3];
 };
 
+// SH >= 0: the job's shader, known at compile time.
 // Without xy_given, (x, y) is computed here from the pixel (i, j).  Chosen
 // primitives are candidates (kept and front-facing) except the default
 // chooser's fallback to primitive 0, whose flags come from its record.
+template <int SH, class Source>
 __device__ __forceinline__ void shade_primitive(const RastJob& J, const RastPools& P, const float4* rec_base,
-                                                int i, int j, float x, float y, int p, const VaryingSource& src,
+                                                int i, int j, float x, float y, int p, const Source& src,
                                                 Fragment* f, bool xy_given, bool fallback = false) {
   const float4* rec = rec_base + static_cast<int64_t>(p) * 4;
   const float4 a = rec[0], b = rec[1], cz = rec[2];
@@ -343,51 +327,20 @@ __device__ __forceinline__ void shade_primitive(const RastJob& J, const RastPool
   const float w_rcp = (c[0] + c[1]) + c[2];
   f->z = ((c[0] * cz.y + c[1] * cz.z) + c[2] * cz.w) * J.viewport[10] + J.viewport[11];
   const float bary[3] = {c[0] / w_rcp, c[1] / w_rcp, c[2] / w_rcp};
-  const int32_t* face = P.faces + (J.face_begin + p) * 3;
-  const int nv = varying_count(J.shader);
   float v0[kMaxVarying], v1[kMaxVarying], v2[kMaxVarying];
-  if (nv > 0) {
-    const int i0 = gather_clamp(face[0], J.n_verts);
-    const int i1 = gather_clamp(face[1], J.n_verts);
-    const int i2 = gather_clamp(face[2], J.n_verts);
-    if (src.fvar || src.var) {
-      const float *r0, *r1, *r2;
-      if (src.fvar) {
-        r0 = src.fvar + ((src.setup_begin + p) * 3) * src.vstride;
-        r1 = r0 + src.vstride;
-        r2 = r1 + src.vstride;
-      } else {
-        r0 = src.var + (src.vout_begin + i0) * src.vstride;
-        r1 = src.var + (src.vout_begin + i1) * src.vstride;
-        r2 = src.var + (src.vout_begin + i2) * src.vstride;
-      }
-      // constant indices keep the three rows in registers
-#pragma unroll
-      for (int k = 0; k < kMaxVarying; ++k) {
-        if (k < nv) {
-          v0[k] = __ldg(r0 + k);
-          v1[k] = __ldg(r1 + k);
-          v2[k] = __ldg(r2 + k);
-        }
-      }
-    } else {
-      float clip[4];
-      vertex_shader<false>(J, P, i0, clip, v0);
-      vertex_shader<false>(J, P, i1, clip, v1);
-      vertex_shader<false>(J, P, i2, clip, v2);
-    }
-  }
+  if ((SH >= 0 ? SH : J.shader) != RAST_SHADER_DEPTH) src.template load<SH>(J, P, p, v0, v1, v2);
   f->colour[0] = f->colour[1] = f->colour[2] = 0.0f;
-  f->keep = fragment_shader(J, P, v0, v1, v2, bary, front, f->colour);
+  f->keep = fragment_shader<SH>(J, P, v0, v1, v2, bary, front, f->colour);
 }
 
 // One pixel after the scan: `w` is the winning candidate (-1: none, or its
 // depth was +inf).  Reproduces the default chooser's fallback to primitive 0
 // (shader.py:215-217), then Shader.interpolate / fragment / mix
 // (pipeline.py:283-359) for the chosen primitive.
+template <int SH, class Source>
 __device__ __forceinline__ void resolve_pixel(const RastJob& J, const RastPools& P,
                                               const float4* rec_base, int i, int j, int w,
-                                              const VaryingSource& src, PixelResult* r) {
+                                              const Source& src, PixelResult* r) {
   r->keep = false;
   r->prim = -1;
   r->z = 0.0f;
@@ -395,7 +348,7 @@ __device__ __forceinline__ void resolve_pixel(const RastJob& J, const RastPools&
   if (J.n_faces <= 0) return;
   const int p = w < 0 ? 0 : w;
   Fragment f;
-  shade_primitive(J, P, rec_base, i, j, 0.0f, 0.0f, p, src, &f, false, w < 0);
+  shade_primitive<SH>(J, P, rec_base, i, j, 0.0f, 0.0f, p, src, &f, false, w < 0);
   r->keep = f.chooser_keep && f.keep;
   r->z = f.z;
   r->prim = r->keep ? p : -1;
@@ -415,9 +368,10 @@ __device__ __forceinline__ int job_layers(const RastJob& J, int max_layers) {
 // interpolation + fragment; the job's mixer combines the kept ones
 // (RastMixer).  first > 0 continues a nearest-mixer pixel whose earlier
 // slots were all discarded.
+template <int SH, class Source>
 __device__ __forceinline__ void resolve_layers(const RastJob& J, const RastPools& P, const float4* rec_base,
                                                int i, int j, const int32_t* w, int64_t wstride, int L,
-                                               const VaryingSource& src, PixelResult* r, int first = 0) {
+                                               const Source& src, PixelResult* r, int first = 0) {
   r->keep = false;
   r->prim = -1;
   r->z = 0.0f;
@@ -438,7 +392,7 @@ __device__ __forceinline__ void resolve_layers(const RastJob& J, const RastPools
     w0 = w1, w1 = w2, w2 = w3, w3 = -1;
     if (p < 0) break;
     Fragment f;
-    shade_primitive(J, P, rec_base, i, j, x, y, p, src, &f, true);
+    shade_primitive<SH>(J, P, rec_base, i, j, x, y, p, src, &f, true);
     if (!(f.chooser_keep && f.keep)) continue;
     if (!r->keep) {
       r->keep = true;
@@ -479,9 +433,10 @@ struct WarpFrags {
 // with fewer layers leave no lane idle while others shade), staged in `wf`,
 // then every lane mixes its own pixel's fragments in slot order.  Same
 // operations and order as resolve_layers.
+template <int SH, class Source>
 __device__ __forceinline__ void resolve_over_warp(const RastJob& J, const RastPools& P, const float4* rec_base,
                                                   bool active, int i, int j, const int32_t* w, int64_t wstride,
-                                                  int L, const VaryingSource& src, WarpFrags& wf,
+                                                  int L, const Source& src, WarpFrags& wf,
                                                   PixelResult* r) {
   const int lane = threadIdx.x & 31;
   r->keep = false;
@@ -523,7 +478,7 @@ __device__ __forceinline__ void resolve_over_warp(const RastJob& J, const RastPo
     if (k < total) {
       const int p = slot == 0 ? a0 : slot == 1 ? a1 : slot == 2 ? a2 : a3;
       Fragment f;
-      shade_primitive(J, P, rec_base, 0, 0, ox, oy, p, src, &f, true);
+      shade_primitive<SH>(J, P, rec_base, 0, 0, ox, oy, p, src, &f, true);
 #pragma unroll
       for (int c = 0; c < 3; ++c) wf.colour[c][k] = f.colour[c];
       wf.z[k] = f.z;

@@ -249,10 +249,10 @@ shade_kernel(RastBatch B, const float4* __restrict__ setup, const float* __restr
   if (i >= W || j >= H) return;
   const int64_t pix = J.pixel_begin + static_cast<int64_t>(i) * H + j;
   PixelResult r;
-  const VaryingSource src{var, vstride, J.vout_begin};
+  const VertexRows src{var, vstride, J.vout_begin};
   const int L = kLayered ? job_layers(J, B.max_layers) : 0;
   if (kLayered && L > 0) {
-    resolve_layers(J, B.pools, setup + J.setup_begin * 4, i, j, winner + pix, B.total_pixels, L, src, &r);
+    resolve_layers<-1>(J, B.pools, setup + J.setup_begin * 4, i, j, winner + pix, B.total_pixels, L, src, &r);
     save_layers(B.pools, winner + pix, B.total_pixels, pix, L);
   } else {
     int w;
@@ -262,7 +262,7 @@ shade_kernel(RastBatch B, const float4* __restrict__ setup, const float* __restr
     } else {
       w = winner[pix];
     }
-    resolve_pixel(J, B.pools, setup + J.setup_begin * 4, i, j, w, src, &r);
+    resolve_pixel<-1>(J, B.pools, setup + J.setup_begin * 4, i, j, w, src, &r);
   }
   store_pixel(J, B.pools, pix, r);
 }

@@ -30,6 +30,67 @@ __host__ __device__ constexpr int varying_count(int shader) {
        : 0;
 }
 
+// Floats of one face's row in the tiled form's face varyings: what the fragment
+// stage reads of the three corners, varying-major, so that a shade thread
+// consumes each 16-byte load before the next.  Varyings 0-4 are [corner 0,
+// corner 1, corner 2]; then the reflection shaders' texture index of corner 0
+// and the shadow coordinates' corner triples; or corner 0's triangles
+// (phong_darboux).
+constexpr int kFaceTail = 15;  // where the shader's own part starts
+__host__ __device__ constexpr int face_floats(int shader) {
+  return shader == RAST_SHADER_DEPTH ? 0
+       : shader == RAST_SHADER_GOURAUD ? 9
+       : shader == RAST_SHADER_PHONG_DARBOUX ? 30
+       : shader == RAST_SHADER_PHONG_REFLECTION ? 16
+       : shader == RAST_SHADER_PHONG_REFLECTION_SHADOW ? 28
+       : 15;
+}
+constexpr int kMaxFaceFloats = 32;
+
+// One corner's varyings (k = 0, 1, 2) into its places of the face's row.
+template <int SH>
+__device__ __forceinline__ void put_corner(int shader, int k, const float* var, float* row) {
+  const int sh = SH >= 0 ? SH : shader;
+#pragma unroll
+  for (int v = 0; v < 5; ++v)
+    if (v < varying_count(sh)) row[3 * v + k] = var[v];
+  if ((sh == RAST_SHADER_PHONG_REFLECTION || sh == RAST_SHADER_PHONG_REFLECTION_SHADOW) && k == 0)
+    row[kFaceTail] = var[kVTexIdx];
+  if (sh == RAST_SHADER_PHONG_REFLECTION_SHADOW) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) row[kFaceTail + 1 + 3 * c + k] = var[kVShadow + c];
+  }
+  if (sh == RAST_SHADER_PHONG_DARBOUX && k == 0) {
+#pragma unroll
+    for (int c = 0; c < 15; ++c) row[kFaceTail + c] = var[kVTri + c];
+  }
+}
+
+// The inverse: a face's row to the three corners' varyings (of corners 1 and 2
+// only what the fragment stage interpolates).
+template <int SH>
+__device__ __forceinline__ void get_corners(int shader, const float* row, float* v0, float* v1, float* v2) {
+  const int sh = SH >= 0 ? SH : shader;
+#pragma unroll
+  for (int v = 0; v < 5; ++v) {
+    v0[v] = row[3 * v];
+    v1[v] = row[3 * v + 1];
+    v2[v] = row[3 * v + 2];
+  }
+  if (sh == RAST_SHADER_PHONG_DARBOUX) {
+#pragma unroll
+    for (int c = 0; c < 15; ++c) v0[kVTri + c] = row[kFaceTail + c];
+  } else {
+    v0[kVTexIdx] = row[kFaceTail];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      v0[kVShadow + c] = row[kFaceTail + 1 + 3 * c];
+      v1[kVShadow + c] = row[kFaceTail + 2 + 3 * c];
+      v2[kVShadow + c] = row[kFaceTail + 3 + 3 * c];
+    }
+  }
+}
+
 __device__ __forceinline__ void load3(const float* p, int64_t row, float* out) {
   out[0] = p[row * 3 + 0];
   out[1] = p[row * 3 + 1];
@@ -128,11 +189,13 @@ __device__ __forceinline__ void texel3(const float* tex, int w, int h, int ch, i
 // Shader.fragment.  v0/v1/v2 are the three vertex varying rows, b the
 // perspective-correct barycentrics (true_clip_coef, pipeline.py:241).
 // Returns the shader's keep (AND-ed by the caller with the chooser's keep).
+// SH >= 0: the job's shader, known at compile time.
+template <int SH = -1>
 __device__ __forceinline__ bool fragment_shader(const RastJob& J, const RastPools& P,
                                                 const float* v0, const float* v1,
                                                 const float* v2, const float* b, bool front,
                                                 float* colour) {
-  const int sh = J.shader;
+  const int sh = SH >= 0 ? SH : J.shader;
   switch (sh) {
     case RAST_SHADER_DEPTH:  // shader.py:333
       return true;

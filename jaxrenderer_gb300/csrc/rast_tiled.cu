@@ -4,18 +4,20 @@
 // tested with the same operations; binning only removes pairs that cannot
 // pass.
 //
+//   begin_kernel       block map of the faces, counters and flags cleared
 //   setup_bin_kernel   one thread per face: clip positions, det/keep/inverse;
 //                      then one thread per candidate (queued in shared memory):
 //                      conservative tile range of its coverage region, bin counts
-//   begin_kernel       block map of the faces, counters and flags cleared
 //   offsets_kernel     bin counts -> bin offsets; tiles whose bins exceed the
 //                      capacity are marked
 //   scatter_kernel     over the binned faces the set-up listed, one warp per 32:
 //                      face id into every bin its rectangle overlaps
 //   raster_kernel      persistent warps, one tile each: bin entries staged in
 //                      shared memory, per-pixel packed (depth | id) minimum
-//   tiled_shade_kernel one thread per pixel: deferred shading of the winner,
-//                      vertex varyings recomputed for its three corners only
+//   face_varyings_kernel  one row per face that some pixel needs: the vertex
+//                      shader's varyings of its three corners
+//   tiled_shade_kernel one thread per pixel: deferred shading of the winner
+//                      from its face's row
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -25,6 +27,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "rast_internal.cuh"
@@ -37,6 +40,7 @@ constexpr int kScanBlock = 1024;       // elements per scan block (256 threads x
 constexpr int kRasterWarps = 4;        // warps per CTA of the raster kernel
 constexpr int kStage = 32;             // bin entries staged per warp round
 constexpr uint32_t kOverflow = 0x80000000u;
+constexpr int kFaceRound = 10;         // faces per warp and round of the face varyings: 30 corners
 constexpr int kFaceThreads = 128;      // threads per block of the face varyings
 
 // Tile shapes offered to the autotuner.  (tw, th): tw pixels along x
@@ -1214,25 +1218,32 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
 }
 
 // Vertex varyings of the three corners of every face some pixel needs
-// (marked by the raster kernel), stored per face: the shade then reads them
-// instead of re-running the vertex shader per pixel.  `split` warps per entry
-// of the set-up's block map: each lists the entry's marked faces in shared
-// memory, then takes one (face, corner) per lane
-// and round, in memory order.  Gathers and normalisation chains bound it, at
-// 4096 brax-like scenes the sectors that 3.8 M faces' corners and rows touch
-// (1.2 GB): warps independent of one another (no block barrier, no shared job
-// copy) and 40 registers take it to 266 us, from 294 with blocks that queued
-// 4,096 faces.  A list that the raster kernel appended to balanced small
-// batches as well but lost the memory order (336 us).  Few entries (a batch
-// of 16 scenes has 700) take several warps each, so that a warp's rounds,
-// 2-3 us of latency each, do not follow one another while SMs idle.
-template <int kRows>
-__global__ void __launch_bounds__(kFaceThreads, 12)
+// (marked by the raster kernel), stored as one row per face (FaceRows): the
+// shade then reads them instead of re-running the vertex shader per pixel.
+// `split` warps per entry of the set-up's block map: each lists the entry's
+// marked faces in shared memory, then takes ten faces a round, one corner per
+// lane, in memory order; the rows are staged in shared memory and leave it as
+// whole float4s.  Gathers and normalisation chains bound it, at 4096
+// brax-like scenes the sectors that 3.8 M faces' corners and rows touch
+// (1.2 GB).  Warps independent of one another (no block barrier, no shared
+// job copy) and 32 registers: 239 us there, from 294 with blocks that queued
+// 4,096 faces and 270 with every corner's floats stored by its own lane.  A
+// list that the raster kernel appended to balanced small batches as well but
+// lost the memory order (336 us).  Few entries (a batch of 16 scenes has 700)
+// take several warps each, so that a warp's rounds, 2-3 us of latency each,
+// do not follow one another while SMs idle.
+// SH: the shader of a single-shader batch, or -1.
+template <int kRows, int SH>
+__global__ void __launch_bounds__(kFaceThreads, SH < 0 || SH == RAST_SHADER_PHONG_DARBOUX ? 12 : 16)
 face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entries, unsigned split,
-                     const uint32_t* __restrict__ visible, float* __restrict__ fvar, int vstride) {
+                     const uint32_t* __restrict__ visible, float4* __restrict__ vec, float* __restrict__ rest,
+                     int floats) {
+  constexpr int kStage = (SH >= 0 ? face_floats(SH) + 3 : kMaxFaceFloats) / 4;  // float4s per staged row
   __shared__ unsigned char s_list[kFaceThreads / 32][kRows];
+  __shared__ float4 s_rows[kFaceThreads / 32][kFaceRound * kStage];
   const int lane = threadIdx.x & 31;
   unsigned char* list = s_list[threadIdx.x >> 5];
+  float4* rows = s_rows[threadIdx.x >> 5];
   const unsigned wid = (blockIdx.x * kFaceThreads + threadIdx.x) >> 5;
   const unsigned entry = wid / split;
   after_previous();
@@ -1240,25 +1251,32 @@ face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entrie
   const int2 blk = fmap[entry];
   if (blk.x < 0) return;
   const RastJob& J = B.jobs[blk.x];
-  if (J.shader == RAST_SHADER_DEPTH) return;
-  const int total = 3 * list_marked<kRows>(visible, J.setup_begin + blk.y, J.n_faces - blk.y, list);
-  const int nv = varying_count(J.shader);
-  for (int t = static_cast<int>(wid - entry * split) * 32 + lane; t < total; t += 32 * static_cast<int>(split)) {
-    const int q = t / 3, k = t - 3 * q;
-    const int fq = blk.y + list[q];
-    const int32_t* face = B.pools.faces + (J.face_begin + fq) * 3;
-    float var[kMaxVarying], clip[4];
-    vertex_shader<false>(J, B.pools, gather_clamp(__ldg(face + k), J.n_verts), clip, var);
-    float* out = fvar + ((J.setup_begin + fq) * 3 + k) * vstride;
-    if (vstride % 2 == 0) {  // rows of whole float2 (a job with an odd count leaves one float of its row unset)
-#pragma unroll
-      for (int v = 0; v < kMaxVarying; v += 2)
-        if (v < nv) *reinterpret_cast<float2*>(out + v) = make_float2(var[v], var[v + 1]);
-    } else {
-#pragma unroll
-      for (int v = 0; v < kMaxVarying; ++v)
-        if (v < nv) out[v] = var[v];
+  if (SH < 0 && J.shader == RAST_SHADER_DEPTH) return;
+  const int count = list_marked<kRows>(visible, J.setup_begin + blk.y, J.n_faces - blk.y, list);
+  const int n = SH >= 0 ? face_floats(SH) : floats, own = face_floats(SH >= 0 ? SH : J.shader);
+  const int vecs = min(n / 4, (own + 3) / 4), tail = own - 4 * (n / 4);
+  const int q = lane / 3, k = lane - 3 * q;
+  for (int f0 = static_cast<int>(wid - entry * split) * kFaceRound; f0 < count;
+       f0 += kFaceRound * static_cast<int>(split)) {
+    const int nf = min(kFaceRound, count - f0);
+    if (q < nf) {
+      const int32_t* face = B.pools.faces + (J.face_begin + blk.y + list[f0 + q]) * 3;
+      float var[kMaxVarying], clip[4];
+      vertex_shader<false, SH>(J, B.pools, gather_clamp(__ldg(face + k), J.n_verts), clip, var);
+      put_corner<SH>(J.shader, k, var, reinterpret_cast<float*>(rows + q * kStage));
     }
+    __syncwarp();
+    const int64_t row0 = J.setup_begin + blk.y;
+    for (int t = lane; t < nf * vecs; t += 32) {
+      const int f = t / vecs;
+      vec[(row0 + list[f0 + f]) * (n / 4) + (t - f * vecs)] = rows[f * kStage + (t - f * vecs)];
+    }
+    for (int t = lane; t < nf * tail; t += 32) {
+      const int f = t / tail;
+      rest[(row0 + list[f0 + f]) * (n % 4) + (t - f * tail)] =
+          reinterpret_cast<const float*>(rows + f * kStage + n / 4)[t - f * tail];
+    }
+    __syncwarp();  // the next round writes the rows anew
   }
 }
 
@@ -1269,28 +1287,32 @@ face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entrie
 // their "over" pixels spread the warp's fragments over its lanes
 // (resolve_over_warp).
 // Grid: (ceil(max pixels per job / 256), n_jobs).
+// SH: the shader of a single-shader batch, compiled alone, or -1: no shader
+// switch and no predicates on the row's length.  With the rows read as seven
+// float4s instead of thirty floats (the L1's wavefronts were 76 % of its peak
+// beside 72 % of the issue slots) the 4096-scene brax-like batch took 750 us,
+// from 972, and 1024 scenes with 4 layers 458, from 653.
 // Eight blocks per SM (32 registers) for the default chooser: more resident
 // warps hide the gathers and division chains better than the spills cost
-// (1.17 -> 0.95 ms on the 4096-scene brax-like batch; 4, 5 and 6 blocks
-// measured slower).  Layered batches take four (64 registers: 2.63 -> 2.56
-// ms on the 4096-scene batch with 4 layers, from three).
-template <bool kLayered>
+// (4096 scenes: 750 us; 825 at six blocks, 891 at five).  Layered batches take
+// four (64 registers).
+template <bool kLayered, int SH>
 __global__ void __launch_bounds__(256, kLayered ? 4 : 8)
 tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t* __restrict__ winner,
-                   bool depth_resolved, const float* __restrict__ fvar, int vstride, Clear clear) {
+                   bool depth_resolved, FaceRows src, Clear clear) {
   __shared__ RastJob sJ;
   __shared__ WarpFrags s_frags[kLayered ? 8 : 1];  // per warp, layered "over" jobs
   after_previous();
   const int jid = blockIdx.y;
   const int64_t npx = static_cast<int64_t>(__ldg(&B.jobs[jid].width)) * __ldg(&B.jobs[jid].height);
   if (static_cast<int64_t>(blockIdx.x) * 256 >= npx) return;
-  if (depth_resolved && __ldg(&B.jobs[jid].shader) == RAST_SHADER_DEPTH) return;  // done by the raster kernel
+  if (SH < 0 && depth_resolved && __ldg(&B.jobs[jid].shader) == RAST_SHADER_DEPTH) return;  // done by the raster kernel
   load_job_to_shared(B.jobs + jid, &sJ);
   __syncthreads();
   const RastJob& J = sJ;
   const int64_t local0 = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
   const int64_t pix = J.pixel_begin + local0;
-  const VaryingSource src{nullptr, vstride, 0, fvar, J.setup_begin};
+  src.setup_begin = J.setup_begin;
   const float4* rec = setup + J.setup_begin * 4;
   const int L = kLayered ? job_layers(J, B.max_layers) : 0;
   if (kLayered && L > 0 && J.mixer == RAST_MIX_OVER) {  // every lane of the warp takes part
@@ -1298,7 +1320,7 @@ tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t*
     int i = 0, j = 0;
     if (active) pixel_of(local0, npx, J.height, &i, &j);
     PixelResult r;
-    resolve_over_warp(J, B.pools, rec, active, i, j, winner + (active ? pix : 0), B.total_pixels, L, src,
+    resolve_over_warp<SH>(J, B.pools, rec, active, i, j, winner + (active ? pix : 0), B.total_pixels, L, src,
                       s_frags[threadIdx.x >> 5], &r);
     if (active) {
       store_pixel(J, B.pools, pix, r, clear);
@@ -1319,9 +1341,9 @@ tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t*
     store_pixel(J, B.pools, pix, r, clear);
     return;
   }
-  resolve_pixel(J, B.pools, rec, i, j, w0, src, &r);  // the winner, or the layered chooser's slot 0
+  resolve_pixel<SH>(J, B.pools, rec, i, j, w0, src, &r);  // the winner, or the layered chooser's slot 0
   if (kLayered && L > 1 && !r.keep)  // slot 0 discarded by its fragment shader: the next kept slot
-    resolve_layers(J, B.pools, rec, i, j, winner + pix, B.total_pixels, L, src, &r, 1);
+    resolve_layers<SH>(J, B.pools, rec, i, j, winner + pix, B.total_pixels, L, src, &r, 1);
   store_pixel(J, B.pools, pix, r, clear);
 }
 
@@ -1339,7 +1361,7 @@ struct Layout {
       fmap_off, keys_off, misc_off, total;
   unsigned fmap_blocks;  // face block map of the set-up
   bool small_path;  // setup kernel rasterises small faces (not when near ties are counted)
-  int vstride;
+  int face_row;  // floats of one face's row of varyings
   int winner_layers;  // chooser slots kept per pixel: 1, or RAST_MAX_LAYERS with layered jobs
   int64_t n_tiles, n_scan_blocks;
   uint64_t bin_capacity;
@@ -1375,13 +1397,12 @@ static Layout layout(const RastBatch& b, TileShape ts, uint64_t bin_capacity, in
   L.bins_off = take(static_cast<size_t>(bin_capacity) * 4);
   L.winner_layers = b.max_layers > 0 ? RAST_MAX_LAYERS : 1;  // the raster variant writes every slot
   L.winner_off = take(static_cast<size_t>(b.total_pixels) * 4 * L.winner_layers);
-  int vstride = 0;
+  L.face_row = 0;
   for (int sh = 0; sh < 7; ++sh)
-    if (b.shader_mask & (1 << sh)) vstride = std::max(vstride, varying_count(sh));
-  L.vstride = vstride;
-  const bool shading = vstride > 0;
+    if (b.shader_mask & (1 << sh)) L.face_row = std::max(L.face_row, face_floats(sh));
+  const bool shading = L.face_row > 0;
   L.vis_off = take(shading ? (static_cast<size_t>(b.total_setup) + 31) / 32 * 4 : 0);
-  L.fvar_off = take(shading ? static_cast<size_t>(b.total_setup) * 3 * vstride * sizeof(float) : 0);
+  L.fvar_off = take(shading ? static_cast<size_t>(b.total_setup) * L.face_row * sizeof(float) : 0);
   L.small_path = b.near_ties == nullptr && small_area > 0 && b.max_layers == 0;
   L.fmap_blocks = block_map_capacity(b.total_setup, b.n_jobs, setup_rows(L.small_path));
   L.fmap_off = take(static_cast<size_t>(L.fmap_blocks) * sizeof(int2));
@@ -1477,6 +1498,21 @@ static void launch_raster(TileShape ts, int wpt, int sms, cudaStream_t s, const 
   }
 }
 
+// Calls f with the shader of a single-shader batch as a constant, or with -1.
+template <class F>
+static void with_shader(int mask, F&& f) {
+  switch (mask) {
+    case 1 << RAST_SHADER_GOURAUD: return f(std::integral_constant<int, RAST_SHADER_GOURAUD>());
+    case 1 << RAST_SHADER_GOURAUD_TEXTURE: return f(std::integral_constant<int, RAST_SHADER_GOURAUD_TEXTURE>());
+    case 1 << RAST_SHADER_PHONG: return f(std::integral_constant<int, RAST_SHADER_PHONG>());
+    case 1 << RAST_SHADER_PHONG_DARBOUX: return f(std::integral_constant<int, RAST_SHADER_PHONG_DARBOUX>());
+    case 1 << RAST_SHADER_PHONG_REFLECTION: return f(std::integral_constant<int, RAST_SHADER_PHONG_REFLECTION>());
+    case 1 << RAST_SHADER_PHONG_REFLECTION_SHADOW:
+      return f(std::integral_constant<int, RAST_SHADER_PHONG_REFLECTION_SHADOW>());
+    default: return f(std::integral_constant<int, -1>());
+  }
+}
+
 static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* workspace,
                   size_t workspace_bytes, void* stream, RastProfile* profile,
                   int phase = RAST_PHASE_COVERAGE | RAST_PHASE_SHADE, const Clear& clear = Clear()) {
@@ -1511,11 +1547,13 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
   Profiler prof(profile, s, "rast_render_tiled");
 
   const bool cover = (phase & RAST_PHASE_COVERAGE) != 0, shade = (phase & RAST_PHASE_SHADE) != 0;
-  uint32_t* vis = L.vstride > 0 ? reinterpret_cast<uint32_t*>(ws + L.vis_off) : nullptr;
-  float* fvar = L.vstride > 0 ? reinterpret_cast<float*>(ws + L.fvar_off) : nullptr;
+  uint32_t* vis = L.face_row > 0 ? reinterpret_cast<uint32_t*>(ws + L.vis_off) : nullptr;
+  float4* fvec = reinterpret_cast<float4*>(ws + L.fvar_off);
+  float* frest = reinterpret_cast<float*>(fvec + b.total_setup * (L.face_row / 4));
+  const FaceRows rows{fvec, frest, L.face_row, 0};
   // shaded jobs resolve in the deferred shade (from the per-face varyings when there are faces)
   const bool shading = b.total_pixels > 0 && (b.shader_mask != (1 << RAST_SHADER_DEPTH) || b.total_setup == 0);
-  const bool pre = shading && fvar != nullptr && b.total_setup > 0;
+  const bool pre = shading && L.face_row > 0 && b.total_setup > 0;
   const int sms = sm_count();
   if (cover) {
     unsigned long long* keys = nullptr;
@@ -1578,12 +1616,12 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
       if (pre) {
         const unsigned split = warps_per_entry(L.fmap_blocks, sms);
         const unsigned vgrid = (L.fmap_blocks * split + kFaceThreads / 32 - 1) / (kFaceThreads / 32);
-        if (L.small_path)
-          launch_after(face_varyings_kernel<setup_rows(true)>, vgrid, kFaceThreads, s, b, fmap, L.fmap_blocks, split, vis, fvar,
-                                                                              L.vstride);
-        else
-          launch_after(face_varyings_kernel<setup_rows(false)>, vgrid, kFaceThreads, s, b, fmap, L.fmap_blocks, split, vis, fvar,
-                                                                              L.vstride);
+        with_shader(b.shader_mask, [&](auto sh) {
+          constexpr int SH = decltype(sh)::value;
+          const auto kernel = L.small_path ? face_varyings_kernel<setup_rows(true), SH>
+                                           : face_varyings_kernel<setup_rows(false), SH>;
+          launch_after(kernel, vgrid, kFaceThreads, s, b, fmap, L.fmap_blocks, split, vis, fvec, frest, L.face_row);
+        });
         prof.mark("face_varyings_kernel");
       }
     }
@@ -1591,12 +1629,14 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
   if (shade && shading) {
     const int64_t max_px = static_cast<int64_t>(b.max_width) * b.max_height;
     const dim3 sgrid(static_cast<unsigned>((max_px + 255) / 256), static_cast<unsigned>(b.n_jobs));
-    const float* fv = pre ? fvar : nullptr;
-    const auto kernel = b.max_layers > 0 ? tiled_shade_kernel<true> : tiled_shade_kernel<false>;
-    if (cover)
-      launch_after(kernel, sgrid, 256, s, b, setup, winner, b.total_setup > 0, fv, L.vstride, clear);
-    else  // the caller's stream may have waited for another pass
-      kernel<<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, fv, L.vstride, clear);
+    with_shader(b.shader_mask, [&](auto sh) {
+      constexpr int SH = decltype(sh)::value;
+      const auto kernel = b.max_layers > 0 ? tiled_shade_kernel<true, SH> : tiled_shade_kernel<false, SH>;
+      if (cover)
+        launch_after(kernel, sgrid, 256, s, b, setup, winner, b.total_setup > 0, rows, clear);
+      else  // the caller's stream may have waited for another pass
+        kernel<<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, rows, clear);
+    });
     prof.mark("tiled_shade_kernel");
   }
   const cudaError_t e = cudaGetLastError();
