@@ -185,6 +185,13 @@ __device__ __forceinline__ void texel3(const float* tex, int w, int h, int ch, i
   }
 }
 
+// The job's normalised light direction: as given, or computed here.
+__device__ __forceinline__ void unit_light(const float* direction, const float* unit, float* out) {
+  if (!unit) return normalise3(direction, out);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) out[c] = unit[c];
+}
+
 // Fragment stage of the chosen primitive: Shader.interpolate then
 // Shader.fragment.  v0/v1/v2 are the three vertex varying rows, b the
 // perspective-correct barycentrics (true_clip_coef, pipeline.py:241).
@@ -194,7 +201,7 @@ template <int SH = -1>
 __device__ __forceinline__ bool fragment_shader(const RastJob& J, const RastPools& P,
                                                 const float* v0, const float* v1,
                                                 const float* v2, const float* b, bool front,
-                                                float* colour) {
+                                                float* colour, const float* light = nullptr) {
   const int sh = SH >= 0 ? SH : J.shader;
   switch (sh) {
     case RAST_SHADER_DEPTH:  // shader.py:333
@@ -266,7 +273,7 @@ __device__ __forceinline__ bool fragment_shader(const RastJob& J, const RastPool
       }
       float tc[3], l[3], lc[3];
       texel3(P.texture + J.texture_begin, J.tex_w, J.tex_h, J.tex_c, ui, wi, tc);
-      normalise3(J.light_direction, l);
+      unit_light(J.light_direction, light, l);
       const float d = dot3(n, l);
       bool nonneg = true;
 #pragma unroll
@@ -325,7 +332,7 @@ __device__ __forceinline__ bool fragment_shader(const RastJob& J, const RastPool
 #pragma unroll
       for (int c = 0; c < 3; ++c) nrm[c] = interp1(b, v0[kVNormal + c], v1[kVNormal + c], v2[kVNormal + c]);
       normalise3(nrm, n);
-      normalise3(J.light_dir_eye, l);
+      unit_light(J.light_dir_eye, light, l);
       const float d = dot3(n, l);
       const float dif = max0(d);
 #pragma unroll

@@ -1296,22 +1296,34 @@ face_varyings_kernel(RastBatch B, const int2* __restrict__ fmap, unsigned entrie
 // warps hide the gathers and division chains better than the spills cost
 // (4096 scenes: 750 us; 825 at six blocks, 891 at five).  Layered batches take
 // four (64 registers).
+// The winner is on its way while the job arrives (736 us), the light's
+// direction is normalised once per block (707): 3 divisions and a square root
+// a pixel.  A pixel without a winner leaves once primitive 0 is seen to miss it
+// (a mixed batch, mostly background: 149 -> 111 us for its three launches; 3
+// us more where every pixel is covered).  Blocks of 128, 64 and 512 threads:
+// 729, 755, 717 us.
 template <bool kLayered, int SH>
 __global__ void __launch_bounds__(256, kLayered ? 4 : 8)
 tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t* __restrict__ winner,
                    bool depth_resolved, FaceRows src, Clear clear) {
   __shared__ RastJob sJ;
+  __shared__ float s_light[3];
   __shared__ WarpFrags s_frags[kLayered ? 8 : 1];  // per warp, layered "over" jobs
   after_previous();
-  const int jid = blockIdx.y;
-  const int64_t npx = static_cast<int64_t>(__ldg(&B.jobs[jid].width)) * __ldg(&B.jobs[jid].height);
-  if (static_cast<int64_t>(blockIdx.x) * 256 >= npx) return;
-  if (SH < 0 && depth_resolved && __ldg(&B.jobs[jid].shader) == RAST_SHADER_DEPTH) return;  // done by the raster kernel
-  load_job_to_shared(B.jobs + jid, &sJ);
+  const RastJob* job = B.jobs + blockIdx.y;
+  load_job_to_shared(job, &sJ);
+  if (threadIdx.x == 255) {
+    const int sh = SH >= 0 ? SH : __ldg(&job->shader);
+    normalise3(sh >= RAST_SHADER_PHONG_REFLECTION ? job->light_dir_eye : job->light_direction, s_light);
+  }
+  const int64_t npx = static_cast<int64_t>(__ldg(&job->width)) * __ldg(&job->height);
+  const int64_t local0 = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
+  const int64_t pix = __ldg(&job->pixel_begin) + local0;
+  const int w0 = local0 < npx ? winner[pix] : -1;  // on its way while the job arrives
   __syncthreads();
   const RastJob& J = sJ;
-  const int64_t local0 = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x;
-  const int64_t pix = J.pixel_begin + local0;
+  if (static_cast<int64_t>(blockIdx.x) * 256 >= npx) return;
+  if (SH < 0 && depth_resolved && J.shader == RAST_SHADER_DEPTH) return;  // done by the raster kernel
   src.setup_begin = J.setup_begin;
   const float4* rec = setup + J.setup_begin * 4;
   const int L = kLayered ? job_layers(J, B.max_layers) : 0;
@@ -1321,7 +1333,7 @@ tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t*
     if (active) pixel_of(local0, npx, J.height, &i, &j);
     PixelResult r;
     resolve_over_warp<SH>(J, B.pools, rec, active, i, j, winner + (active ? pix : 0), B.total_pixels, L, src,
-                      s_frags[threadIdx.x >> 5], &r);
+                      s_frags[threadIdx.x >> 5], &r, s_light);
     if (active) {
       store_pixel(J, B.pools, pix, r, clear);
       save_layers(B.pools, winner + pix, B.total_pixels, pix, L);
@@ -1332,7 +1344,6 @@ tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t*
   int i, j;
   pixel_of(local0, npx, J.height, &i, &j);
   PixelResult r;
-  const int w0 = winner[pix];
   if (kLayered && L > 0) save_layers(B.pools, winner + pix, B.total_pixels, pix, L);
   if (kLayered && L > 0 && w0 < 0) {  // no candidate: the layered chooser keeps nothing
     r.keep = false;
@@ -1341,9 +1352,9 @@ tiled_shade_kernel(RastBatch B, const float4* __restrict__ setup, const int32_t*
     store_pixel(J, B.pools, pix, r, clear);
     return;
   }
-  resolve_pixel<SH>(J, B.pools, rec, i, j, w0, src, &r);  // the winner, or the layered chooser's slot 0
+  resolve_pixel<SH>(J, B.pools, rec, i, j, w0, src, &r, s_light);  // the winner, or the layered chooser's slot 0
   if (kLayered && L > 1 && !r.keep)  // slot 0 discarded by its fragment shader: the next kept slot
-    resolve_layers<SH>(J, B.pools, rec, i, j, winner + pix, B.total_pixels, L, src, &r, 1);
+    resolve_layers<SH>(J, B.pools, rec, i, j, winner + pix, B.total_pixels, L, src, &r, 1, s_light);
   store_pixel(J, B.pools, pix, r, clear);
 }
 
