@@ -960,7 +960,7 @@ def profile_kernels(mr, steps, stream):
                         where[name] = (r, key, kname)
                     acc[name].append(prof.ms[k])
                     if it == 0 and kname != "memset":
-                        launches += 2 if kname == "scan_kernels" else 1
+                        launches += 1
     summary = {n: {"avg_ms": float(np.mean(v)), "launches": len(v)} for n, v in acc.items()}
     total = sum(v["avg_ms"] for v in summary.values())
     for v in summary.values():
@@ -972,6 +972,7 @@ def profile_kernels(mr, steps, stream):
 # bytes a face corner's vertex inputs take, and texel bytes a pixel reads, per shader id
 _CORNER_IN = {0: 12, 1: 36, 2: 32, 3: 32, 4: 32, 5: 36, 6: 36}
 _TEXEL = {0: 0, 1: 0, 2: 12, 3: 12, 4: 24, 5: 16, 6: 20}
+_FACE_ROW = {0: 0, 1: 9, 2: 15, 3: 15, 4: 30, 5: 16, 6: 28}  # floats of a face's row in the tiled form (face_floats)
 _VARYINGS = {0: 0, 1: 3, 2: 5, 3: 5, 4: 20, 5: 6, 6: 10}  # floats per corner (rast_shaders.cuh varying_count)
 
 
@@ -987,6 +988,7 @@ def pass_info(runner, pass_name):
         "corners": float(nv.sum()),
         "cin": float(sum(nv[k] * _CORNER_IN[int(sh[k])] for k in range(len(sh)))),
         "vs": max(_VARYINGS[int(s)] for s in np.unique(sh)),
+        "row": max(_FACE_ROW[int(s)] for s in np.unique(sh)),
         "tests": float((px * jobs["n_faces"].astype(np.int64)).sum()),
         "main": bool((sh != 0).any()),
         "slots": 4 if int(jobs["layers"].max()) > 0 else 1,  # chooser slots written per pixel
@@ -1007,24 +1009,30 @@ def kernel_bytes(kname, info, visible):
     F faces, P pixels, E bin entries, T tiles, B binned faces (those with a
     tile, listed for the scatter), V faces visible in the main
     pass (the front-most kept face of a pixel: with layered choosers a lower
-    bound), vs varyings per corner, S chooser slots written per pixel."""
+    bound), vs varyings per corner, `row` floats of a face's row, S chooser
+    slots written per pixel."""
     F, P, E, T, vs = info["F"], info["P"], info["E"], info["T"], info["vs"]
     S = info.get("slots", 1)
+    B = info.get("B", 0.0)
+    row = info.get("row", 3 * vs + 4)  # without a row length: three corners and the record's last quarter
+    key = 8 if S == 1 else 4 * S  # the plain form's chooser result per pixel
     V = float(visible) if info["main"] else 0.0
     out_px = 16 if info["main"] else 4  # zbuffer (+ canvas) written
     table = {
         # plain form
         "vertex_kernel": info["cin"] + info["corners"] * (16 + 4 * vs),
         "setup_kernel": F * (12 + 3 * 16 + 64),
-        "scan_kernel": F * 48 + P * 4 * S,
-        "shade_kernel": P * (4 * S + out_px) + info["Ptex"] + V * (64 + 3 * (16 + 4 * vs)),
+        "scan_kernel": F * 52 + P * key,
+        "slots_kernel": F * 52 + P * 4 * S,
+        "shade_kernel": P * (key + out_px) + info["Ptex"] + V * (64 + 3 * (16 + 4 * vs)),
         # tiled form
-        "setup_bin_kernel": F * (12 + 36 + 64 + 8) + info.get("B", 0.0) * 16 + E * 4,
-        "scan_kernels": T * 12,
+        "begin_kernel": T * 8 + F * (1 / 8 + 8 / 256),
+        "setup_bin_kernel": F * (12 + 36 + 1) + B * (64 + 1 + 16) + E * 4,
+        "offsets_kernel": T * 12,
         "scatter_kernel": info.get("B", 0.0) * 16 + E * 12,
         "raster_kernel": F * 48 + E * 4 + P * 4 * S,
-        "face_varyings_kernel": F + V * (12 + 3 * (info["cin"] / max(info["corners"], 1)) + 3 * 4 * vs),
-        "tiled_shade_kernel": P * (4 * S + out_px) + info["Ptex"] + V * (64 + 3 * 4 * vs),
+        "face_varyings_kernel": F / 8 + V * (12 + 3 * (info["cin"] / max(info["corners"], 1)) + 4 * row),
+        "tiled_shade_kernel": P * (4 * S + out_px) + info["Ptex"] + V * (48 + 4 * row),
     }
     return table.get(kname, 0.0)
 
