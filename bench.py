@@ -1059,7 +1059,7 @@ def library_digest(files=FORWARD_SOURCES) -> str:
 # library_digest() of the sources the NCU_* counts below were captured on:
 # when the kernels change, the counts no longer describe them and the bench
 # reports traffic and the issue figure as null until they are captured again.
-NCU_SOURCE_DIGEST = "d4e29622dd43f128"
+NCU_SOURCE_DIGEST = "6676f6c95bfe4d04"
 
 
 def ncu_counts_current() -> bool:
@@ -1077,16 +1077,16 @@ def ncu_counts_current() -> bool:
 # Keyed by (pass, kernel); the raster kernel's also by its tile shape and
 # warps per tile.
 NCU_PER_UNIT = {
-    ("shadow", "setup_bin_kernel"): ("F", 97.04, 25.07),
-    ("main", "setup_bin_kernel"): ("F", 103.53, 26.49),
-    ("shadow", "scatter_kernel"): ("F", 1.69, 1.56),
-    ("main", "scatter_kernel"): ("F", 6.74, 3.97),
-    ("shadow", "raster_kernel", 16, 16, 2): ("P", 3.15, 11.62),
-    ("shadow", "raster_kernel", 16, 8, 1): ("P", 3.40, 11.68),
-    ("main", "raster_kernel", 16, 8, 1): ("P", 29.32, 16.66),
-    ("main", "raster_kernel", 8, 8, 1): ("P", 29.22, 19.56),
-    ("main", "face_varyings_kernel"): ("F", 29.90, 4.60),
-    ("main", "tiled_shade_kernel"): ("P", 59.80, 31.21),
+    ("shadow", "setup_bin_kernel"): ("F", 36.94, 15.86),
+    ("main", "setup_bin_kernel"): ("F", 44.35, 24.29),
+    ("shadow", "scatter_kernel"): ("F", 1.69, 1.55),
+    ("main", "scatter_kernel"): ("F", 6.74, 3.49),
+    ("shadow", "raster_kernel", 16, 16, 2): ("P", 2.62, 10.90),
+    ("shadow", "raster_kernel", 16, 8, 1): ("P", 2.72, 10.89),
+    ("main", "raster_kernel", 16, 8, 1): ("P", 24.34, 15.87),
+    ("main", "raster_kernel", 8, 8, 1): ("P", 24.58, 18.92),
+    ("main", "face_varyings_kernel"): ("F", 27.50, 5.36),
+    ("main", "tiled_shade_kernel"): ("P", 38.68, 25.74),
 }
 
 
