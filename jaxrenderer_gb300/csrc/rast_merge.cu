@@ -8,7 +8,7 @@
 //                         normals through the inverse-transpose -- 4x4 LU in
 //                         jnp.linalg.inv's order -- and the global norm of the
 //                         transformed normals, uvs)
-//   corner_kernel         one warp per instance: gathers per face corner
+//   corner_kernel         several warps per instance: gathers per face corner
 //
 // Operation order follows the host merge: apply_pos = to_cartesian(M [p * s,
 // 1]) with products summed in index order; apply_vec = normalise(M [n /
@@ -162,14 +162,18 @@ instance_kernel(RastMergeBatch B, const float* __restrict__ mesh_norm, float* __
   }
 }
 
-// One warp per instance writes the instance's 3 * n_faces corners: merged
-// face indices (local + scene offset), gathered from the scene's merged rows
-// with wrap-once-then-clamp.  Grid: ceil(n_instances * 32 / kThreads).
+// `split` warps per instance write the instance's 3 * n_faces corners in turn:
+// merged face indices (local + scene offset), gathered from the scene's merged
+// rows with wrap-once-then-clamp.  Latency of the gathers bounds it, and with
+// one warp per instance the largest mesh's rounds: 200 brax-like scenes 81 ->
+// 48 us, 200 Ant frames 34 -> 26, the whole merge of 16 scenes 68 -> 30 and of
+// 4096 1,200 -> 1,028.  Grid: ceil(n_instances * split * 32 / kThreads).
 __global__ void __launch_bounds__(kThreads)
 corner_kernel(RastMergeBatch B, const float* __restrict__ mpos, const int* __restrict__ mobj,
-              const float* __restrict__ mnrm, const float* __restrict__ muv) {
+              const float* __restrict__ mnrm, const float* __restrict__ muv, int split) {
   after_previous();
-  const int o = static_cast<int>((static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5);
+  const int64_t warp = (static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x) >> 5;
+  const int o = static_cast<int>(warp / split), part = static_cast<int>(warp - static_cast<int64_t>(o) * split);
   const int lane = threadIdx.x & 31;
   if (o >= B.n_instances) return;
   const RastInstance I = B.instances[o];
@@ -184,7 +188,7 @@ corner_kernel(RastMergeBatch B, const float* __restrict__ mpos, const int* __res
   float* __restrict__ out_uv = B.uv;
   int* __restrict__ out_tix = B.texture_index;
   constexpr int kU = 2;  // corners per lane per round: their gathers are in flight together
-  for (int64_t base = 0; base < corners; base += 32 * kU) {
+  for (int64_t base = part * (32 * kU); base < corners; base += split * (32 * kU)) {
     float pv[kU][3], nv[kU][3], uv[kU][2];
     int tix[kU];
 #pragma unroll
@@ -289,7 +293,12 @@ static int run(const RastMergeBatch* batch, void* workspace, size_t workspace_by
     launch_after(instance_kernel, wg, kThreads, s, b, mesh_norm, mpos, mobj, mnrm, muv);
   else
     instance_kernel<<<wg, kThreads, 0, s>>>(b, mesh_norm, mpos, mobj, mnrm, muv);
-  launch_after(corner_kernel, wg, kThreads, s, b, mpos, mobj, mnrm, muv);
+  // Four warps an instance, up to sixteen while that leaves fewer than 64 per SM: the merge of 16 scenes (340
+  // instances) takes 38 us at four, 32 at eight, 30 at sixteen; the corners of 200 frames (3,600 instances) 26 us
+  // at four, 30 at eight, 32 at sixteen.
+  const int split = static_cast<int>(std::max<int64_t>(4, std::min<int64_t>(16, 64ll * sm_count() / b.n_instances)));
+  const unsigned cg = static_cast<unsigned>((static_cast<int64_t>(b.n_instances) * split * 32 + kThreads - 1) / kThreads);
+  launch_after(corner_kernel, cg, kThreads, s, b, mpos, mobj, mnrm, muv, split);
   return cudaGetLastError() == cudaSuccess ? RAST_OK : RAST_ERR_CUDA;
 }
 
