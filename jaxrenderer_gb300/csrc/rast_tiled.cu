@@ -518,7 +518,7 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
   constexpr int kT = kSmall ? kTableMax : 1;
   __shared__ float s_small[12][kQ];  // inverse (9) and clip depths (3) of small faces
   __shared__ int s_sface[kQ];
-  __shared__ int s_srect[kQ][2];     // i0 | i1 << 16, j0 | j1 << 16
+  __shared__ unsigned s_srect[kQ][2];  // pack_pixel(i0, j0), pack_pixel(i1, j1)
   __shared__ float s_xs[kT], s_ys[kT];
   __shared__ int s_qn, s_sn;
   __shared__ ScreenRect s_rect;
@@ -604,7 +604,7 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
         out[2] = make_float4(iv[8], s_m[9][q], s_m[10][q], s_m[11][q]);
       }
       if (covers) {
-        if (kSmall && (i1 - i0 + 1) * (j1 - j0 + 1) <= small_area) {
+        if (kSmall && static_cast<int64_t>(i1 - i0 + 1) * (j1 - j0 + 1) <= small_area) {
           small = true;  // rasterised in phase 3, not binned
         } else {
           tx0 = i0 >> G.tws;
@@ -629,8 +629,8 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
       for (int k = 0; k < 9; ++k) s_small[k][e] = iv[k];
 #pragma unroll
       for (int k = 0; k < 3; ++k) s_small[9 + k][e] = s_m[9 + k][q];
-      s_srect[e][0] = i0 | (i1 << 16);
-      s_srect[e][1] = j0 | (j1 << 16);
+      s_srect[e][0] = pack_pixel(i0, j0);
+      s_srect[e][1] = pack_pixel(i1, j1);
     }
     // binned faces (those with tiles) join the scatter's list: one atomic per warp
     const bool bin = tx0 <= tx1 && ty0 <= ty1;
@@ -653,9 +653,9 @@ setup_bin_kernel(RastBatch B, Geometry G, const int2* __restrict__ fmap, float4*
   const int lane = threadIdx.x & 31;
   const float vp22 = J.viewport[10], vp23 = J.viewport[11];
   for (int e = threadIdx.x >> 5; e < sn; e += kSetupThreads / 32) {
-    const int ri = s_srect[e][0], rj = s_srect[e][1];
-    const int a0 = ri & 0xffff, b0 = rj & 0xffff;
-    const int bw = (ri >> 16) - a0 + 1, bh = (rj >> 16) - b0 + 1;
+    const unsigned lo = s_srect[e][0], hi = s_srect[e][1];
+    const int a0 = static_cast<int>(lo & 0xffffu), b0 = static_cast<int>(lo >> 16);
+    const int bw = static_cast<int>(hi & 0xffffu) - a0 + 1, bh = static_cast<int>(hi >> 16) - b0 + 1;
     if (lane >= bw * bh) continue;
     const int i = a0 + lane % bw, j = b0 + lane / bw;
     const float x = tables ? s_xs[i] : (static_cast<float>(i) - ox) / sx;
