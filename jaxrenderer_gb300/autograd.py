@@ -154,9 +154,10 @@ class _CameraFunction(torch.autograd.Function):
         eye, target, up, projection = ctx.saved_tensors
         wanted = ctx.needs_input_grad[:3]
         if torch.is_grad_enabled():  # create_graph: gradients of gradients follow the tensor operations
-            inputs = [t for t, w in zip((eye, target, up), wanted) if w]
-            outs, gs = zip(*((o, g) for o, g in zip(_camera_tensors(eye, target, up, projection), grads) if g is not None))
-            got = iter(torch.autograd.grad(outs, inputs, gs, create_graph=True, allow_unused=True))
+            # views of the inputs: a gradient stops at them, and does not run on through an input computed from another
+            rows = [t.view_as(t) for t in (eye, target, up)]
+            outs, gs = zip(*((o, g) for o, g in zip(_camera_tensors(*rows, projection), grads) if g is not None))
+            got = iter(torch.autograd.grad(outs, [t for t, w in zip(rows, wanted) if w], gs, create_graph=True, allow_unused=True))
             return (*(next(got) if w else None for w in wanted), None)
         n = eye.shape[0]
         mats = [_mats(g) for g in grads]
