@@ -153,12 +153,8 @@ class _CameraFunction(torch.autograd.Function):
     def backward(ctx, *grads):
         eye, target, up, projection = ctx.saved_tensors
         wanted = ctx.needs_input_grad[:3]
-        if torch.is_grad_enabled():  # create_graph: gradients of gradients follow the tensor operations
-            # views of the inputs: a gradient stops at them, and does not run on through an input computed from another
-            rows = [t.view_as(t) for t in (eye, target, up)]
-            outs, gs = zip(*((o, g) for o, g in zip(_camera_tensors(*rows, projection), grads) if g is not None))
-            got = iter(torch.autograd.grad(outs, [t for t, w in zip(rows, wanted) if w], gs, create_graph=True, allow_unused=True))
-            return (*(next(got) if w else None for w in wanted), None)
+        if torch.is_grad_enabled() or not all(_has_memory(g) for g in grads if g is not None):
+            return (*_tensor_gradients((eye, target, up), projection, wanted, grads), None)
         n = eye.shape[0]
         mats = [_mats(g) for g in grads]
         out = [torch.empty((n, 3), dtype=eye.dtype, device=eye.device) if w else None for w in wanted]
@@ -169,6 +165,29 @@ class _CameraFunction(torch.autograd.Function):
                 *(x for g in mats for x in ((g.data_ptr(), g.stride(0)) if g is not None else (None, 0))),
                 *(t.data_ptr() if t is not None else None for t in out), s), "rast_camera_matrices_backward")
         return (*out, None)
+
+
+def _tensor_gradients(rows, projection, wanted, grads):
+    """The reverse mode as tensor operations: with create_graph (gradients of
+    gradients follow them), and for gradients the kernel cannot read."""
+    create_graph = torch.is_grad_enabled()
+    with torch.enable_grad():
+        # views of the inputs: a gradient stops at them, and does not run on through an input computed from another
+        rows = [t.view_as(t) if create_graph else t.detach().requires_grad_(w) for t, w in zip(rows, wanted)]
+        outs, gs = zip(*((o, g) for o, g in zip(_camera_tensors(*rows, projection), grads) if g is not None))
+        got = iter(torch.autograd.grad(outs, [t for t, w in zip(rows, wanted) if w], gs, create_graph=create_graph,
+                                       allow_unused=True))
+    return [next(got) if w else None for w in wanted]
+
+
+def _has_memory(t: torch.Tensor) -> bool:
+    """Whether there is memory behind `t` that a kernel can read: not behind
+    the batched tensors of is_grads_batched, whose gradient mode is off and
+    which no query of the active transforms reports."""
+    try:
+        return t.data_ptr() != 0
+    except RuntimeError:
+        return False
 
 
 def _rows(t: torch.Tensor):

@@ -16,6 +16,33 @@ def _double(*tensors):
     return [t.detach().double().requires_grad_() for t in tensors]
 
 
+@pytest.mark.parametrize("n", [1, 5])
+@pytest.mark.parametrize("create_graph", [False, True])
+def test_batched_gradients(n, create_graph):
+    import torch
+
+    from jaxrenderer_gb300 import autograd as A
+
+    e, c, u, _ = _inputs(n, False, n)
+    d = _double(e, c, u)
+    rows = torch.randn((4, n, 4, 4), device="cuda")
+
+    def grads(leaves, rows, batched):
+        ms = A.camera_matrices(leaves[0], _params(), leaves[1], leaves[2])
+        if batched:
+            return torch.autograd.grad(ms[0], leaves, rows, is_grads_batched=True, create_graph=create_graph)
+        return [torch.stack(g) for g in zip(*(torch.autograd.grad(ms[0], leaves, r, retain_graph=True) for r in rows))]
+
+    for a, b in zip(grads((e, c, u), rows, True), grads(d, rows.double(), False)):
+        _close(a, b)
+
+    def w2c(x):
+        return A.camera_matrices(x, _params(), c.detach().to(x.dtype), u.detach().to(x.dtype))[0]
+
+    got = torch.autograd.functional.jacobian(w2c, e.detach(), vectorize=True, create_graph=create_graph)
+    _close(got, torch.autograd.functional.jacobian(w2c, d[0].detach()))
+
+
 def test_gradients_of_gradients_of_inputs_that_depend_on_one_another():
     import torch
 
