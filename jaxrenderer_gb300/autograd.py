@@ -122,15 +122,20 @@ def _camera_tensors(eye, target, up, projection):
 
 def _native_cameras(*tensors) -> bool:
     """Whether the kernels take these: float32 rows of one GPU, with nothing
-    watching the operations (functorch transforms, forward-mode duals, tracing,
-    autocast, dispatch modes and tensor subclasses see the tensor operations)."""
+    watching the operations (_watched, autocast and tensor subclasses see the
+    tensor operations)."""
     eye = tensors[0]
     return (eye.dim() == 2 and eye.shape[0] > 0 and eye.shape[1] == 3
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.float32
                     and t.device == eye.device and t.shape[-1] == 3 and t.stride(-1) == 1 for t in tensors)
-            and not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0
-            and torch._C._len_torch_dispatch_stack() == 0 and not torch.jit.is_tracing() and not torch.compiler.is_compiling()
-            and not torch.is_autocast_enabled())
+            and not _watched() and not torch.is_autocast_enabled())
+
+
+def _watched() -> bool:
+    """Whether something follows the operations one by one: functorch
+    transforms, forward-mode duals, dispatch modes or tracing."""
+    return (torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0
+            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing() or torch.compiler.is_compiling())
 
 
 class _CameraFunction(torch.autograd.Function):
@@ -153,7 +158,7 @@ class _CameraFunction(torch.autograd.Function):
     def backward(ctx, *grads):
         eye, target, up, projection = ctx.saved_tensors
         wanted = ctx.needs_input_grad[:3]
-        if torch.is_grad_enabled() or not all(_has_memory(g) for g in grads if g is not None):
+        if torch.is_grad_enabled() or _watched() or not all(_has_memory(g) for g in grads if g is not None):
             return (*_tensor_gradients((eye, target, up), projection, wanted, grads), None)
         n = eye.shape[0]
         mats = [_mats(g) for g in grads]
@@ -169,7 +174,8 @@ class _CameraFunction(torch.autograd.Function):
 
 def _tensor_gradients(rows, projection, wanted, grads):
     """The reverse mode as tensor operations: with create_graph (gradients of
-    gradients follow them), and for gradients the kernel cannot read."""
+    gradients follow them), where something watches (a tangent of the gradient
+    is asked for inside a dual level), and for gradients the kernel cannot read."""
     create_graph = torch.is_grad_enabled()
     with torch.enable_grad():
         # views of the inputs: a gradient stops at them, and does not run on through an input computed from another

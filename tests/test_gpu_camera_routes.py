@@ -57,3 +57,20 @@ def test_gradients_of_gradients_of_inputs_that_depend_on_one_another():
 
     for a, b in zip(second(e, u, ws), second(*_double(e, u), [w.double() for w in ws])):
         _close(a, b)
+
+
+def test_tangents_of_the_gradient():
+    import torch
+    import torch.autograd.forward_ad as fwd
+
+    from jaxrenderer_gb300 import autograd as A
+
+    e, c, u, ws = _inputs(5, False, 11)
+
+    def tangent(leaves, ws):
+        ms = A.camera_matrices(leaves[0], _params(), leaves[1], leaves[2])
+        with fwd.dual_level():
+            (g,) = torch.autograd.grad(ms[0], leaves[:1], fwd.make_dual(ws[0], ws[1]))
+            return fwd.unpack_dual(g).tangent
+
+    _close(tangent((e, c, u), ws), tangent(_double(e, c, u), [w.double() for w in ws]))
