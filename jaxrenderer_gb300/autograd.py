@@ -124,11 +124,16 @@ def _native_cameras(*tensors) -> bool:
     """Whether the kernels take these: float32 rows of one GPU, with nothing
     watching the operations (_watched, autocast and tensor subclasses see the
     tensor operations)."""
+    return _kernel_rows(*tensors) and not _watched() and not torch.is_autocast_enabled()
+
+
+def _kernel_rows(*tensors) -> bool:
+    """Whether these are rows (or one shared row) of three adjacent float32 on
+    one GPU, as many as the first of them has."""
     eye = tensors[0]
     return (eye.dim() == 2 and eye.shape[0] > 0 and eye.shape[1] == 3
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.float32
-                    and t.device == eye.device and t.shape[-1] == 3 and t.stride(-1) == 1 for t in tensors)
-            and not _watched() and not torch.is_autocast_enabled())
+                    and t.device == eye.device and t.shape[-1] == 3 and t.stride(-1) == 1 for t in tensors))
 
 
 def _watched() -> bool:
@@ -158,7 +163,10 @@ class _CameraFunction(torch.autograd.Function):
     def backward(ctx, *grads):
         eye, target, up, projection = ctx.saved_tensors
         wanted = ctx.needs_input_grad[:3]
-        if torch.is_grad_enabled() or _watched() or not all(_has_memory(g) for g in grads if g is not None):
+        # the saved tensors may have come through hooks that lay them out anew
+        readable = (_kernel_rows(eye, target, up) and projection.is_cuda and projection.dtype == torch.float32
+                    and projection.is_contiguous() and all(_has_memory(g) for g in grads if g is not None))
+        if torch.is_grad_enabled() or _watched() or not readable:
             return (*_tensor_gradients((eye, target, up), projection, wanted, grads), None)
         n = eye.shape[0]
         mats = [_mats(g) for g in grads]
@@ -175,7 +183,7 @@ class _CameraFunction(torch.autograd.Function):
 def _tensor_gradients(rows, projection, wanted, grads):
     """The reverse mode as tensor operations: with create_graph (gradients of
     gradients follow them), where something watches (a tangent of the gradient
-    is asked for inside a dual level), and for gradients the kernel cannot read."""
+    is asked for inside a dual level), and for tensors the kernel cannot read."""
     create_graph = torch.is_grad_enabled()
     with torch.enable_grad():
         # views of the inputs: a gradient stops at them, and does not run on through an input computed from another

@@ -1,5 +1,7 @@
 """camera_matrices where something watches or batches its gradients: the same
 results as the tensor operations give in float64."""
+import contextlib
+
 import pytest
 
 from .test_gpu_camera import _inputs, _loss, _params
@@ -74,3 +76,26 @@ def test_tangents_of_the_gradient():
             return fwd.unpack_dual(g).tangent
 
     _close(tangent((e, c, u), ws), tangent(_double(e, c, u), [w.double() for w in ws]))
+
+
+def _transposed(t):
+    return t.mT.contiguous().mT if t.dim() > 1 else t
+
+
+@pytest.mark.parametrize("hooks", ["cpu", "strides"])
+def test_saved_tensor_hooks(hooks):
+    import torch
+
+    from jaxrenderer_gb300 import autograd as A
+
+    e, c, u, ws = _inputs(65, True, 2)
+    around = (torch.autograd.graph.save_on_cpu() if hooks == "cpu"
+              else torch.autograd.graph.saved_tensors_hooks(lambda t: t, _transposed))
+
+    def grads(leaves, ws, around=contextlib.nullcontext()):
+        with around:
+            ms = A.camera_matrices(leaves[0], _params(), leaves[1], leaves[2])
+        return torch.autograd.grad(_loss(ms, ws), leaves)
+
+    for a, b in zip(grads((e, c, u), ws, around), grads(_double(e, c, u), [w.double() for w in ws])):
+        _close(a, b)
