@@ -163,6 +163,8 @@ class _CameraFunction(torch.autograd.Function):
     def backward(ctx, *grads):
         eye, target, up, projection = ctx.saved_tensors
         wanted = ctx.needs_input_grad[:3]
+        if all(g is None for g in grads):
+            return None, None, None, None
         # the saved tensors may have come through hooks that lay them out anew
         readable = (_kernel_rows(eye, target, up) and projection.is_cuda and projection.dtype == torch.float32
                     and projection.is_contiguous() and all(_has_memory(g) for g in grads if g is not None))

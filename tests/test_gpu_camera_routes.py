@@ -61,6 +61,27 @@ def test_gradients_of_gradients_of_inputs_that_depend_on_one_another():
         _close(a, b)
 
 
+def test_no_gradient_arrives():
+    import torch
+
+    from jaxrenderer_gb300 import autograd as A
+
+    class Nothing(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, x):
+            return x.sum()
+
+        @staticmethod
+        def backward(ctx, g):
+            return None
+
+    e, c, u, _ = _inputs(3, False, 1)
+    for create_graph in (False, True):
+        y = Nothing.apply(A.camera_matrices(e, _params(), c, u)[0])
+        g = torch.autograd.grad(y, (e, c, u), create_graph=create_graph, allow_unused=True)
+        assert all(t is None or not t.any() for t in g)
+
+
 def test_tangents_of_the_gradient():
     import torch
     import torch.autograd.forward_ad as fwd
