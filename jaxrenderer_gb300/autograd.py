@@ -133,7 +133,7 @@ def _kernel_rows(*tensors) -> bool:
     eye = tensors[0]
     return (eye.dim() == 2 and eye.shape[0] > 0 and eye.shape[1] == 3
             and all(type(t) in (torch.Tensor, torch.nn.Parameter) and t.is_cuda and t.dtype == torch.float32
-                    and t.device == eye.device and t.shape[-1] == 3 and t.stride(-1) == 1 for t in tensors))
+                    and t.device == eye.device and t.shape[-1:] == (3,) and t.stride(-1) == 1 for t in tensors))
 
 
 def _watched() -> bool:

@@ -120,3 +120,15 @@ def test_saved_tensor_hooks(hooks):
 
     for a, b in zip(grads((e, c, u), ws, around), grads(_double(e, c, u), [w.double() for w in ws])):
         _close(a, b)
+
+
+@pytest.mark.parametrize("up", [2.0, (0.5,), ((0.1, -0.05, 1.0),)])
+def test_up_of_any_shape_that_broadcasts(up):
+    import torch
+
+    from jaxrenderer_gb300 import autograd as A
+
+    e, c, _, _ = _inputs(5, False, 4)
+    up = torch.tensor(up, device="cuda")
+    for a, b in zip(A.camera_matrices(e, _params(), c, up), A.camera_matrices(e.double(), _params(), c.double(), up.double())):
+        _close(a.detach(), b.detach())
