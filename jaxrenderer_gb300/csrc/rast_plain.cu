@@ -289,9 +289,10 @@ static PlainLayout plain_layout(const RastBatch& b) {
   L.setup_off = off;
   off = align256(off + static_cast<size_t>(b.total_setup) * 4 * sizeof(float4));
   L.winner_off = off;
-  // one key per pixel (scan_kernel), or one winner, or RAST_MAX_LAYERS with layered jobs (slots_kernel)
+  // one key per pixel (scan_kernel), or one winner, or RAST_MAX_LAYERS with layered jobs (slots_kernel); a tie
+  // counter's winners take a key's room, so that a workspace serves its batch with the counter and without
   L.keyed = b.max_layers == 0 && b.near_ties == nullptr;
-  const size_t slots = L.keyed ? 2 : b.max_layers > 0 ? RAST_MAX_LAYERS : 1;
+  const size_t slots = b.max_layers > 0 ? RAST_MAX_LAYERS : 2;
   off = align256(off + static_cast<size_t>(b.total_pixels) * slots * sizeof(int32_t));
   L.total = off;
   return L;
