@@ -312,6 +312,7 @@ static int render_plain(const RastBatch* batch, void* workspace, size_t workspac
   int st = check_batch(batch);
   if (st != RAST_OK) return st;
   const RastBatch& b = *batch;
+  if (b.total_pixels > 0 && (b.max_width < 1 || b.max_height < 1)) return RAST_ERR_INVALID_ARGUMENT;
   const PlainLayout L = plain_layout(b);
   if (workspace_bytes < L.total) return RAST_ERR_WORKSPACE_TOO_SMALL;
   if (L.total > 0 && (workspace == nullptr || (reinterpret_cast<uintptr_t>(workspace) & 255)))

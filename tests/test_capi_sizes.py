@@ -1,9 +1,14 @@
 """Sizes and statuses of the C ABI that need no GPU."""
 import ctypes
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 
 from jaxrenderer_gb300 import _lib
+
+ROOT = Path(__file__).resolve().parent.parent
 
 
 def _batch(width=33, height=17, layers=0):
@@ -23,3 +28,11 @@ def test_plain_workspace_does_not_depend_on_the_tie_counter(layers):
     with_ties, without = _batch(layers=layers), _batch(layers=layers)
     with_ties.near_ties = 256
     assert lib.rast_plain_workspace_bytes(ctypes.byref(with_ties)) == lib.rast_plain_workspace_bytes(ctypes.byref(without))
+
+
+@pytest.mark.parametrize("width,height", [(0, 17), (33, 0)])
+def test_pixels_without_a_width_or_a_height_are_refused(width, height):
+    """In a process of its own: an integer division by zero ends it."""
+    code = ("import ctypes; from tests.test_capi_sizes import _batch, _lib; b = _batch(%d, %d); lib = _lib.load()\n"
+            "assert lib.rast_render_plain(ctypes.byref(b), 256, 1 << 20, None) == 1" % (width, height))
+    subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True)
