@@ -416,6 +416,16 @@ def _rast_batch(jobs: np.ndarray, pools: Dict[str, torch.Tensor], zbuffer: torch
     return b
 
 
+FLOAT32_MAX = float(np.finfo(np.float32).max)
+
+
+def _is_float32(x) -> bool:
+    """Whether `x` is a host number of float32's range, infinities and NaN
+    among them.  Buffers take other defaults by Tensor.fill_: a tensor, read on
+    the device when the pass runs, or what fill_ refuses."""
+    return isinstance(x, (int, float)) and (abs(x) <= FLOAT32_MAX or x != x or abs(x) == float("inf"))
+
+
 @dataclass
 class BatchOutputs:
     canvas: torch.Tensor  # (N, W, H, 3)
@@ -661,7 +671,7 @@ class BatchRunner:
         self.zbuffer.fill_(zbuffer_default)
         self.canvas.copy_(self._colour.expand_as(self.canvas))
         if self.shadow_map is not None:
-            self.shadow_map.fill_(float(np.finfo(np.float32).max))
+            self.shadow_map.fill_(FLOAT32_MAX)
 
     def run(self, stream: Optional[torch.cuda.Stream] = None, zbuffer_default: float = 1.0) -> BatchOutputs:
         """Reset the buffers to their defaults and render every scene on
@@ -673,8 +683,8 @@ class BatchRunner:
         s = stream if stream is not None else torch.cuda.current_stream(self.sb.device)
         with torch.cuda.stream(s):
             clear = {"shadow": None, "main": None}
-            if self.form == "tiled":  # the kernels store the defaults themselves
-                clear = {"shadow": _lib.RastClear(None, float(np.finfo(np.float32).max)),
+            if self.form == "tiled" and _is_float32(zbuffer_default):  # the kernels store the defaults themselves
+                clear = {"shadow": _lib.RastClear(None, FLOAT32_MAX),
                          "main": _lib.RastClear(self._colour.data_ptr(), zbuffer_default)}
             else:
                 self._reset(zbuffer_default)
