@@ -1643,9 +1643,9 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
     with_shader(b.shader_mask, [&](auto sh) {
       constexpr int SH = decltype(sh)::value;
       const auto kernel = b.max_layers > 0 ? tiled_shade_kernel<true, SH> : tiled_shade_kernel<false, SH>;
-      if (cover)
+      if (cover && b.total_setup > 0)
         launch_after(kernel, sgrid, 256, s, b, setup, winner, b.total_setup > 0, rows, clear);
-      else  // the caller's stream may have waited for another pass
+      else  // after a memset (no faces), or the caller's stream may have waited for another pass
         kernel<<<sgrid, 256, 0, s>>>(b, setup, winner, b.total_setup > 0, rows, clear);
     });
     prof.mark("tiled_shade_kernel");
