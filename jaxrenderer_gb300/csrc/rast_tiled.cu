@@ -31,6 +31,7 @@
 #include <vector>
 
 #include "rast_internal.cuh"
+#include "rast_pairs.cuh"
 
 namespace rast {
 namespace tiled {
@@ -386,31 +387,31 @@ template <class Fn>
 __device__ __forceinline__ void warp_tiles(int tx0, int ty0, int tx1, int ty1, int tiles_x, Fn&& fn) {
   const int lane = threadIdx.x & 31;
   const int w = tx1 - tx0 + 1;
-  const int n = (tx0 <= tx1 && ty0 <= ty1) ? w * (ty1 - ty0 + 1) : 0;
-  int incl = n;
+  const unsigned n = (tx0 <= tx1 && ty0 <= ty1) ? static_cast<unsigned>(w * (ty1 - ty0 + 1)) : 0u;
+  unsigned incl = n;  // of 32 rectangles of up to 2^26 tiles
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    const unsigned v = __shfl_up_sync(0xffffffffu, incl, d);
     if (lane >= d) incl += v;
   }
-  const int excl = incl - n;
-  const int total = __shfl_sync(0xffffffffu, incl, 31);
-  for (int base = 0; base < total; base += 32) {
-    const int k = base + lane;
+  const unsigned excl = incl - n;
+  const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
+  for (unsigned base = 0; base < total; base += 32u) {
+    const unsigned k = base + static_cast<unsigned>(lane);
     int owner = 0;  // lanes whose pairs all precede pair k
 #pragma unroll
     for (int step = 16; step > 0; step >>= 1) {
-      const int v = __shfl_sync(0xffffffffu, incl, owner + step - 1);
+      const unsigned v = __shfl_sync(0xffffffffu, incl, owner + step - 1);
       if (v <= k) owner += step;
     }
-    const int o_excl = __shfl_sync(0xffffffffu, excl, owner);
+    const unsigned o_excl = __shfl_sync(0xffffffffu, excl, owner);
     const int o_tx0 = __shfl_sync(0xffffffffu, tx0, owner);
     const int o_ty0 = __shfl_sync(0xffffffffu, ty0, owner);
     const int o_w = __shfl_sync(0xffffffffu, w, owner);
     const bool valid = k < total;
     int tile = 0;
     if (valid) {
-      const int local = k - o_excl;
+      const int local = static_cast<int>(k - o_excl);
       const int r = local / o_w;
       tile = (o_ty0 + r) * tiles_x + o_tx0 + (local - r * o_w);
     }
@@ -431,35 +432,33 @@ template <class Put, class Get, class Fn>
 __device__ __forceinline__ void warp_tiles_staged(int tx0, int ty0, int tx1, int ty1, int tiles_x, Put&& put, Get&& get, Fn&& fn) {
   const int lane = threadIdx.x & 31;
   const int w = tx1 - tx0 + 1;
-  const int n = (tx0 <= tx1 && ty0 <= ty1) ? w * (ty1 - ty0 + 1) : 0;
-  int incl = n;
+  const unsigned n = (tx0 <= tx1 && ty0 <= ty1) ? static_cast<unsigned>(w * (ty1 - ty0 + 1)) : 0u;
+  unsigned incl = n;  // of 32 rectangles of up to 2^26 tiles
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, d);
+    const unsigned v = __shfl_up_sync(0xffffffffu, incl, d);
     if (lane >= d) incl += v;
   }
-  const int excl = incl - n;
-  const int total = __shfl_sync(0xffffffffu, incl, 31);
-  const unsigned have = __ballot_sync(0xffffffffu, n > 0);
+  const unsigned excl = incl - n;
+  const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
+  const unsigned have = __ballot_sync(0xffffffffu, n > 0u);
   // pair -> row of its rectangle by the reciprocal width: the quotient (k +
   // 1/2) / w is at least 1/(2w) from an integer and its error below 2^-21 n / w
-  if (n > 0)
+  if (n > 0u)
     put(__popc(have & lanemask_lt()),
-        make_int4(excl, tx0 | (ty0 << 16), w, n < (1 << 20) ? __float_as_int(__frcp_rn(static_cast<float>(w))) : 0));
-  int first = n > 0 ? excl : 0x40000000;  // this lane's first pair, from the round's first
-  int before = -1;                        // last slot begun before the round
+        make_int4(static_cast<int>(excl), tx0 | (ty0 << 16), w, n < (1u << 20) ? __float_as_int(__frcp_rn(static_cast<float>(w))) : 0));
+  int before = -1;  // last slot begun before the round
   __syncwarp();
-  for (int base = 0; base < total; base += 32) {
-    const unsigned begun = __reduce_or_sync(0xffffffffu, static_cast<unsigned>(first) < 32u ? 1u << first : 0u);
+  for (unsigned base = 0; base < total; base += 32u) {
+    const unsigned begun = __reduce_or_sync(0xffffffffu, pair_begin_bit(excl, n, base));
     const int slot = before + __popc(begun & (lanemask_lt() << 1 | 1u));
     before += __popc(begun);
-    first -= 32;
-    const int k = base + lane;
+    const unsigned k = base + static_cast<unsigned>(lane);
     const bool valid = k < total;
     int tile = 0;
     if (valid) {
       const int4 o = get(slot);
-      const int local = k - o.x;
+      const int local = static_cast<int>(k - static_cast<unsigned>(o.x));
       const int r = o.w ? __float2int_rz((static_cast<float>(local) + 0.5f) * __int_as_float(o.w)) : local / o.z;
       tile = ((o.y >> 16) + r) * tiles_x + (o.y & 0xffff) + (local - r * o.z);
     }
