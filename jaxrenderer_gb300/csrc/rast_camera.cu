@@ -56,7 +56,7 @@ __device__ __forceinline__ float sum3(const float* a, const float* b) {
 struct Rows {  // (n, 3) rows; stride 0: one row for every camera
   const float* p;
   int64_t stride;
-  __device__ __forceinline__ void load(int i, float* out) const {
+  __device__ __forceinline__ void load(int64_t i, float* out) const {
 #pragma unroll
     for (int k = 0; k < 3; ++k) out[k] = __ldg(p + i * stride + k);
   }
@@ -65,7 +65,7 @@ struct Rows {  // (n, 3) rows; stride 0: one row for every camera
 __global__ void __launch_bounds__(kThreads)
 forward_kernel(int n, Rows eye, Rows centre, Rows up, const float* __restrict__ projection, float* __restrict__ w2c,
                float* __restrict__ w2e, float* __restrict__ view) {
-  const int i = blockIdx.x * kThreads + threadIdx.x;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;  // 16 i passes 2^31 at 2^27 cameras
   if (i >= n) return;
   float e[3], c[3], w[3];
   eye.load(i, e);
@@ -104,13 +104,13 @@ __device__ __forceinline__ void unit_bwd(const float* y, float n, const float* d
 struct Mats {
   const float* p;
   int64_t stride;
-  __device__ __forceinline__ float at(int i, int k) const { return p ? __ldg(p + i * stride + k) : 0.0f; }
+  __device__ __forceinline__ float at(int64_t i, int k) const { return p ? __ldg(p + i * stride + k) : 0.0f; }
 };
 
 __global__ void __launch_bounds__(kThreads)
 backward_kernel(int n, Rows eye, Rows centre, Rows up, const float* __restrict__ projection, Mats gw2c, Mats gw2e, Mats gview,
                 float* __restrict__ geye, float* __restrict__ gcentre, float* __restrict__ gup) {
-  const int i = blockIdx.x * kThreads + threadIdx.x;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * kThreads + threadIdx.x;  // 16 i passes 2^31 at 2^27 cameras
   if (i >= n) return;
   float e[3], c[3], w[3];
   eye.load(i, e);
