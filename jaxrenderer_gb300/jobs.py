@@ -196,8 +196,10 @@ class _Pool:
     def fresh(self, device) -> Optional[torch.Tensor]:
         """tensor(), never sharing memory with a part."""
         t = self.tensor(device)
-        shared = len(self.parts) == 1 and isinstance(self.parts[0], torch.Tensor) and t.device == self.parts[0].device
-        return t.clone() if shared else t
+        if len(self.parts) != 1:  # concatenated
+            return t
+        p = self.parts[0]
+        return t.clone() if t.device == (p.device if isinstance(p, torch.Tensor) else torch.device("cpu")) else t
 
     def tensor(self, device) -> Optional[torch.Tensor]:
         if not self.parts:
