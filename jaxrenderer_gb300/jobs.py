@@ -185,12 +185,16 @@ class _Pool:
         return n if self.parts else None
 
     def host_into(self, buf: np.ndarray) -> None:
-        """Write the parts into `buf` (the pool's bytes)."""
+        """Write the parts into `buf` (the pool's bytes), other types converted
+        (or refused) by torch as _to_dev does."""
         out = buf.view(np.float32 if self.dtype == torch.float32 else np.int32)
         at = 0
         for p in self.parts:
             a = np.asarray(p).reshape(-1)
-            out[at : at + a.size] = a
+            if a.dtype == out.dtype:
+                out[at : at + a.size] = a
+            else:
+                torch.from_numpy(out[at : at + a.size]).copy_(torch.from_numpy(np.ascontiguousarray(a)))
             at += a.size
 
     def fresh(self, device) -> Optional[torch.Tensor]:
