@@ -944,13 +944,13 @@ def profile_kernels(mr, steps, stream):
     launches = 0
     for it in range(steps):
         for r in mr.runners:
-            r._reset(1.0)
+            clear = r.prepare()  # as run() does: the kernels that are replayed
             prefix = f"{r.sb.width}x{r.sb.height}/" if multi else ""
             for key, _b in r.batches():
                 if it == 0:
                     passes.append((prefix + key, r, key))
                 prof = _lib.RastProfile()
-                r.launch(key, stream.cuda_stream, profile=prof)
+                r.launch(key, stream.cuda_stream, profile=prof, clear=clear[key])
                 for k in range(prof.n):
                     kname = prof.names[k].decode()
                     name = f"{prefix}{key}:{kname}"

@@ -284,9 +284,12 @@ typedef struct RastClear {
 int rast_render_tiled_clear(const RastBatch* batch, const RastTiledConfig* cfg, const RastClear* clear, void* workspace,
                             size_t workspace_bytes, void* stream, int phase);
 
-/* rast_render_tiled with per-kernel timing (synchronises `stream`). */
+/* rast_render_tiled and rast_render_tiled_clear (both phases) with per-kernel
+ * timing (synchronise `stream`). */
 int rast_render_tiled_profiled(const RastBatch* batch, const RastTiledConfig* cfg, void* workspace,
                                size_t workspace_bytes, void* stream, RastProfile* profile);
+int rast_render_tiled_clear_profiled(const RastBatch* batch, const RastTiledConfig* cfg, const RastClear* clear,
+                                     void* workspace, size_t workspace_bytes, void* stream, RastProfile* profile);
 
 /* Tiled form for callers that cannot allocate device memory.
  *

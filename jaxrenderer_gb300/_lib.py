@@ -216,6 +216,8 @@ PROTOTYPES = [
                                         c_int]),
     ("rast_render_tiled_clear", c_int, [POINTER(RastBatch), POINTER(RastTiledConfig), POINTER(RastClear), c_void_p,
                                         c_size_t, c_void_p, c_int]),
+    ("rast_render_tiled_clear_profiled", c_int, [POINTER(RastBatch), POINTER(RastTiledConfig), POINTER(RastClear), c_void_p,
+                                                 c_size_t, c_void_p, POINTER(RastProfile)]),
     ("rast_tiled_stats", c_int,
      [POINTER(RastBatch), POINTER(RastTiledConfig), c_void_p, c_void_p, POINTER(RastTiledStats)]),
     ("rast_backward_workspace_bytes", c_size_t, [POINTER(RastBatch)]),

@@ -523,8 +523,13 @@ class BatchRunner:
         b = self.shadow_batch if name == "shadow" else self.main_batch
         buf, nbytes = self.ws[name]
         if clear is not None:
-            st = self.lib.rast_render_tiled_clear(ctypes.byref(b), self._cfg(name), ctypes.byref(clear), buf.data_ptr(),
-                                                  nbytes, stream_handle, int(phase))
+            args = (ctypes.byref(b), self._cfg(name), ctypes.byref(clear), buf.data_ptr(), nbytes, stream_handle)
+            if profile is None:
+                st = self.lib.rast_render_tiled_clear(*args, int(phase))
+            elif phase == 3:
+                st = self.lib.rast_render_tiled_clear_profiled(*args, ctypes.byref(profile))
+            else:
+                raise ValueError("a profile covers both phases")
             _lib.check(st, "rast_render_tiled_clear")
             return
         if self.form == "tiled" and phase != 3 and profile is None:
@@ -673,6 +678,16 @@ class BatchRunner:
         if self.shadow_map is not None:
             self.shadow_map.fill_(FLOAT32_MAX)
 
+    def prepare(self, zbuffer_default: float = 1.0) -> Dict[str, Optional["_lib.RastClear"]]:
+        """What launch(clear=...) of each pass takes so that the buffers hold
+        their defaults where nothing is drawn: the defaults for the tiled
+        kernels to store, or None after a fill of the buffers here."""
+        if self.form == "tiled" and _is_float32(zbuffer_default):
+            return {"shadow": _lib.RastClear(None, FLOAT32_MAX),
+                    "main": _lib.RastClear(self._colour.data_ptr(), zbuffer_default)}
+        self._reset(zbuffer_default)
+        return {"shadow": None, "main": None}
+
     def run(self, stream: Optional[torch.cuda.Stream] = None, zbuffer_default: float = 1.0) -> BatchOutputs:
         """Reset the buffers to their defaults and render every scene on
         `stream`: the depth pass, then the main pass.  In the tiled form with
@@ -682,12 +697,7 @@ class BatchRunner:
         capture records as two branches."""
         s = stream if stream is not None else torch.cuda.current_stream(self.sb.device)
         with torch.cuda.stream(s):
-            clear = {"shadow": None, "main": None}
-            if self.form == "tiled" and _is_float32(zbuffer_default):  # the kernels store the defaults themselves
-                clear = {"shadow": _lib.RastClear(None, FLOAT32_MAX),
-                         "main": _lib.RastClear(self._colour.data_ptr(), zbuffer_default)}
-            else:
-                self._reset(zbuffer_default)
+            clear = self.prepare(zbuffer_default)
             if self.form == "tiled" and self.shadow_batch is not None and self.overlap_passes:
                 side = self._side_stream()
                 side.wait_stream(s)

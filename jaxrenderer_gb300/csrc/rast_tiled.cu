@@ -1702,11 +1702,23 @@ extern "C" int rast_render_tiled_phase(const RastBatch* batch, const RastTiledCo
   return tiled::render(batch, cfg, workspace, workspace_bytes, stream, nullptr, phase);
 }
 
+static int render_clear(const RastBatch* batch, const RastTiledConfig* cfg, const RastClear* clear, void* workspace,
+                        size_t workspace_bytes, void* stream, RastProfile* profile, int phase) {
+  if (!batch || !clear || (batch->pools.canvas && !clear->colour)) return RAST_ERR_INVALID_ARGUMENT;
+  return tiled::render(batch, cfg, workspace, workspace_bytes, stream, profile, phase,
+                       Clear{clear->colour, clear->depth, true});
+}
+
 extern "C" int rast_render_tiled_clear(const RastBatch* batch, const RastTiledConfig* cfg, const RastClear* clear,
                                        void* workspace, size_t workspace_bytes, void* stream, int phase) {
-  if (!batch || !clear || (batch->pools.canvas && !clear->colour)) return RAST_ERR_INVALID_ARGUMENT;
-  return tiled::render(batch, cfg, workspace, workspace_bytes, stream, nullptr, phase,
-                       Clear{clear->colour, clear->depth, true});
+  return render_clear(batch, cfg, clear, workspace, workspace_bytes, stream, nullptr, phase);
+}
+
+extern "C" int rast_render_tiled_clear_profiled(const RastBatch* batch, const RastTiledConfig* cfg,
+                                                const RastClear* clear, void* workspace, size_t workspace_bytes,
+                                                void* stream, RastProfile* profile) {
+  return render_clear(batch, cfg, clear, workspace, workspace_bytes, stream, profile,
+                      RAST_PHASE_COVERAGE | RAST_PHASE_SHADE);
 }
 
 extern "C" int rast_render_tiled_profiled(const RastBatch* batch, const RastTiledConfig* cfg,
