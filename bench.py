@@ -45,6 +45,7 @@ from typing import Callable, Optional
 import numpy as np
 
 ROOT = Path(__file__).resolve().parent
+OUTPUT = Path(os.environ.get("JAXRENDERER_GB300_BENCH_OUTPUT", ROOT / "build"))  # clock samples and detail files
 sys.path.insert(0, str(ROOT))
 
 METRIC = "frames/s @84x84x4096 scenes fwd and fwd+bwd, tiled-batched vs plain GPU"
@@ -382,11 +383,11 @@ class ClockSampler:
     def __init__(self, index: int = 0):
         self.index = index
         self.proc = None
-        self.path = ROOT / "gpurun_out" / f"clocks_{os.getpid()}.csv"
+        self.path = OUTPUT / f"clocks_{os.getpid()}.csv"
 
     def __enter__(self):
         try:
-            self.path.parent.mkdir(exist_ok=True)
+            self.path.parent.mkdir(parents=True, exist_ok=True)
             q = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
                  "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
                  "clocks_event_reasons.sw_thermal_slowdown,clocks_event_reasons.sw_power_cap")
@@ -573,9 +574,9 @@ def run_ours(args, rank, world, local):
     roof, per_kernel = roofline(prof, visible, clocks)
     detail = {"kernels": prof["summary"], "per_kernel": per_kernel,
               "backward_kernels_ms": fwd_bwd.pop("backward_kernels_ms", None), "fwd_bwd_grads": fwd_bwd.pop("grads", None)}
-    detail_path = ROOT / "gpurun_out" / f"bench_{args.workload}_s{args.scenes}_n{world}_detail.json"
+    detail_path = OUTPUT / f"bench_{args.workload}_s{args.scenes}_n{world}_detail.json"
     if rank == 0:
-        detail_path.parent.mkdir(exist_ok=True)
+        detail_path.parent.mkdir(parents=True, exist_ok=True)
         detail_path.write_text(json.dumps(detail, indent=1))
     out = {
         "metric": METRIC,
@@ -613,7 +614,7 @@ def run_ours(args, rank, world, local):
         "roofline": roof,
         "gpu_launches": kernels_per_step * args.steps,
         "clocks": clocks,
-        "detail_file": str(detail_path.relative_to(ROOT)),
+        "detail_file": os.path.relpath(detail_path, ROOT),
     }
     if e2e is not None:
         out["e2e"] = e2e
