@@ -3,9 +3,10 @@
 // one thread per camera and one launch per direction.  As tensor operations
 // the same takes about 90 launches forward and 140 backward, each of a few
 // microseconds: 3.3 ms of host time around a 0.5 ms render.  Operation order
-// of the forward: the tensor operations' own (autograd.view_matrix), with the
-// contraction their kernels have (cross products and the 4 x 4 product fuse
-// one multiply into each addition), so that the matrices keep their bits.
+// of the forward: that of the tensor operations (autograd.view_matrix) with
+// the contraction of their kernels as they are today (cross products and the
+// 4 x 4 product fuse one multiply into each addition); between the two routes
+// the matrices may differ by rounding, within what test_gpu_camera.py allows.
 #include <cuda_runtime.h>
 
 #include "rast_internal.cuh"

@@ -491,15 +491,15 @@ constexpr int kTableMax = 1024;                              // pixel -> NDC tab
 // 1,536 resident threads per SM without the small path (40 registers): the
 // kernel is latency- and issue-bound (position gathers, then the inverse's
 // division chains), and more resident warps beat the spills: 4096 brax-like
-// scenes, both passes, 1,076 us at 12 blocks of 128, 1,109 at 10, 1,248 at 8,
-// 1,382 at 14.  The small path's shared arrays allow fewer.
+// scenes, both passes, 1,027 us at 12 blocks of 128, 1,080 at 10, 1,213 at 8,
+// 1,268 at 14.  The small path's shared arrays allow fewer.
 __host__ __device__ constexpr int setup_min_blocks(bool small) { return small ? 0 : 1536 / kSetupThreads; }
 // Faces per block: rounds of one face per thread.  Two rounds fill phase 2's
-// warps better and pay the job load once per 256 faces (the whole step 4,000
-// us; one round 4,106, four 4,201, whose queue costs resident blocks).  The
-// off-screen test ahead of the inverse and records for binned faces only took
-// both passes from 1,488 to 1,046 us (of 23.3 M faces each: 0.25 ms of
-// positions at the measured copy rate).
+// warps better and pay the job load once per 256 faces (1,027 us; one round
+// 1,163; four cost resident blocks by their queue).  Without the off-screen
+// test ahead of the inverse, and with a record for every face, both passes
+// took 1,488 us (23.3 M faces each: 0.25 ms of positions at the measured copy
+// rate).
 __host__ __device__ constexpr int setup_rounds(bool small) { return small ? 1 : 2; }
 __host__ __device__ constexpr int setup_rows(bool small) { return setup_rounds(small) * kSetupThreads; }
 
