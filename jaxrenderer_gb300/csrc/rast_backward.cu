@@ -1334,7 +1334,7 @@ static int run(const RastBatch* batch, const CanvasGrad& grad_canvas, const floa
          L.vacc_stride,
          reinterpret_cast<int2*>(ws + L.fmap_off), reinterpret_cast<int2*>(ws + L.vmap_off),
          // four warps an entry while all are resident at once (post_kernel at 256 scenes: 38 us; 51 with four at any number)
-         L.fblocks, L.vblocks, warps_per_entry(L.fblocks, sms, 48, 1), warps_per_entry(L.vblocks, sms, 48, 1),
+         L.fblocks, L.vblocks, warps_per_entry(L.fblocks, sms, 48), warps_per_entry(L.vblocks, sms, 48),
          reinterpret_cast<LightUnit*>(ws + L.light_off)};
   Profiler prof(profile, s, "rast_backward");
   const int mask = b.shader_mask;

@@ -142,9 +142,9 @@ __device__ __forceinline__ int list_marked(const uint32_t* __restrict__ marks, i
 // Warps per map entry of the kernels that work through list_marked: up to
 // four while there are fewer than `per_sm` of them per SM, so that a warp's
 // rounds, 2-3 us of latency each, do not follow one another while SMs idle.
-inline unsigned warps_per_entry(unsigned entries, int sms, unsigned per_sm, unsigned least) {
+inline unsigned warps_per_entry(unsigned entries, int sms, unsigned per_sm) {
   const unsigned k = static_cast<unsigned>(sms) * per_sm / (entries > 0 ? entries : 1u);
-  return k < least ? least : k > 4u ? 4u : k;
+  return k < 1u ? 1u : k > 4u ? 4u : k;
 }
 
 // Sets `bytes` bytes at p (16-byte aligned; the last 16-byte word may run

@@ -1225,7 +1225,7 @@ raster_kernel(RastBatch B, Geometry G, const float4* __restrict__ setup, const u
 // whole float4s.  Gathers and normalisation chains bound it, at 4096
 // brax-like scenes the sectors that 3.8 M faces' corners and rows touch
 // (1.2 GB).  Warps independent of one another (no block barrier, no shared
-// job copy) and 32 registers: 230 us there, from 294 with blocks that queued
+// job copy) and 32 registers: 239 us there, from 294 with blocks that queued
 // 4,096 faces and 270 with every corner's floats stored by its own lane.  A
 // list that the raster kernel appended to balanced small batches as well but
 // lost the memory order (336 us).
@@ -1622,11 +1622,12 @@ static int render(const RastBatch* batch, const RastTiledConfig* cfg, void* work
       }
       prof.mark("raster_kernel");
       if (pre) {
-        // Four warps an entry up to some 25,000 entries, two beyond 40,000: an entry whose 256 faces are all marked
-        // is 26 rounds, and one warp that works through them alone outlasts the kernel's other work (256 brax-like
-        // scenes, 5,900 entries: 50 us at one warp, 26 at four; 1,024 scenes 87 and 72; 2,048 scenes 133 and 132, 124
-        // at two; 4,096 scenes 234 and 249, 230 at two).
-        const unsigned split = warps_per_entry(L.fmap_blocks, sms, 800, 2);
+        // Four warps an entry up to some 8,700 entries, one beyond 17,500: an entry whose 256 faces are all marked is 26
+        // rounds, and one warp that works through them alone outlasts a small batch's other work (256 brax-like scenes,
+        // 5,900 entries: 50 us at one warp, 26 at four; 512 scenes 62 and 45 at three; 768 scenes 76 and 62 at two).
+        // More warps also list an entry more often: 1,024 mixed scenes (classes of 19,000 entries, few faces marked in
+        // each) lost 1.5 % of the pass with four.
+        const unsigned split = warps_per_entry(L.fmap_blocks, sms, 230);
         const unsigned vgrid = (L.fmap_blocks * split + kFaceThreads / 32 - 1) / (kFaceThreads / 32);
         with_shader(b.shader_mask, [&](auto sh) {
           constexpr int SH = decltype(sh)::value;
